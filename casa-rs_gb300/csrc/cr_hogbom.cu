@@ -9,7 +9,9 @@
 // PSF over the overlap (subtract_shifted_kernel_in_window, lib.rs:74805-
 // 74870) as a float32 multiply then subtract.
 //
-// Each block owns a contiguous range of pixels.  One pass per iteration
+// Images that fit the registers of one block per SM run hogbom_reg_kernel
+// below.  For the others (and several planes at once) each block owns a
+// contiguous range of pixels.  One pass per iteration
 // subtracts the previous component and finds the block's next candidate with
 // a warp-shuffle argmax; one grid barrier publishes the candidates, and every
 // block reduces all candidates to the same global peak.  The kernel is
@@ -193,6 +195,265 @@ __global__ void __launch_bounds__(kHogThreads) hogbom_kernel(HogArgs a) {
     hogbom_body(a, (int)gridDim.x, (int)blockIdx.x);
 }
 
+// ---- one image with its residual in registers ---------------------------------------
+// The loop above reads and writes the residual (and reads the PSF) through
+// L2 in every iteration and spends two dependent round trips on the barrier
+// and the candidates.  Here the residual stays in registers for the whole
+// minor cycle: a warp owns 32 columns (lanes, so rows load as 128-byte
+// segments) by K rows of the image, so an iteration reads only the PSF, with
+// one column test per lane and one row test per register row, and all K PSF
+// loads of a thread in flight together.  Instead of a barrier, every block
+// sends its candidate as one 64-bit word to every block, which polls only
+// the words sent to it (all blocks polling one set of words took 3 us more at
+// 128 blocks: the polls queue before the stores at the words' L2 lines).
+//
+// The word is |value|, key << 1 | sign, and a parity bit that flips every
+// time its slot is reused; slots are double buffered by iteration.  A block
+// sends iteration i + 1's word only after it has read every word of i, so no
+// slot is overwritten before its block has read it.  Only block 0 writes
+// anything else that is shared (model and component list).
+//
+// 2048^2, 2001 components: 14.3 -> 4.4 us per component, of which about 2.5
+// is the PSF out of L2 (16.8 MB) and the rest the exchange (1.5 us at one
+// block, 2.4 at 128); 512^2: 5.8 -> 2.4 us.
+constexpr int kHogRegThreads = 512;
+constexpr int kHogRegWarps = kHogRegThreads / 32;
+
+struct HogRegArgs {
+    HogArgs a;                      // cands and bar unused
+    unsigned long long* words;      // [2][reader][writer], zeroed
+    int cols;                       // column groups of 32
+    int rows;                       // image rows per warp (<= K)
+};
+
+// All of a block's threads agree on the best candidate of the grid: false
+// when a wait gave up.  best: |value| as int bits (-1: none), key << 1 | sign.
+__device__ __forceinline__ bool hogreg_exchange(const HogRegArgs& g, long long it, int babs,
+                                                unsigned bks, int* s_abs, unsigned* s_ks,
+                                                int* oabs, unsigned* oks) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = (int)gridDim.x;
+    const unsigned long long par = ((it >> 1) & 1) ^ 1;
+    volatile unsigned long long* buf = g.words + (it & 1) * n * n;
+    // |value| in bits 63..33 (31 bits), the low half key << 1 | sign; the
+    // parity sits in bit 32.  No candidate: key 0x7fffffff (no pixel has it).
+    const unsigned long long word =
+        ((unsigned long long)(unsigned)(babs < 0 ? 0 : babs) << 33) | (par << 32) |
+        (babs < 0 ? 0xffffffffull : (unsigned long long)bks);
+    for (int i = tid; i < n; i += kHogRegThreads) buf[i * n + (int)blockIdx.x] = word;
+    volatile unsigned long long* slots = buf + (int)blockIdx.x * n;
+    int mabs = -1;
+    unsigned mks = 0xffffffffu;
+    int good = 1;
+    for (int i = tid; i < n; i += kHogRegThreads) {
+        unsigned long long w = slots[i];
+        for (long long spins = 0; ((w >> 32) & 1) != par;) {
+            if (++spins > g.a.barrier_polls) {
+                good = 0;
+                break;
+            }
+            if (spins > 256) __nanosleep(64);
+            w = slots[i];
+        }
+        const unsigned ks = (unsigned)w;
+        const int av = ks == 0xffffffffu ? -1 : (int)(w >> 33);
+        if (av > mabs || (av == mabs && ks < mks)) {
+            mabs = av;
+            mks = ks;
+        }
+    }
+    const int wa = __reduce_max_sync(0xffffffffu, mabs);
+    const unsigned wk = __reduce_min_sync(0xffffffffu, mabs == wa ? mks : 0xffffffffu);
+    if (lane == 0) {
+        s_abs[warp] = wa;
+        s_ks[warp] = wk;
+    }
+    const int ok = __syncthreads_and(good);
+    const int ra = s_abs[lane & (kHogRegWarps - 1)];
+    const unsigned rk = s_ks[lane & (kHogRegWarps - 1)];
+    *oabs = __reduce_max_sync(0xffffffffu, ra);
+    *oks = __reduce_min_sync(0xffffffffu, ra == *oabs ? rk : 0xffffffffu);
+    return ok != 0;
+}
+
+// A predicated load that stays one: as a C++ conditional the compiler turned
+// the K loads into K branches, each waiting for the one before (12.1 us per
+// component at 2048^2 instead of 4.5).
+__device__ __forceinline__ float load_if(bool take, const float* p) {
+    float v;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+        "@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(v)
+        : "l"(p), "r"((int)take));
+    return v;
+}
+constexpr int kHogRegLoads = 32;   // PSF loads in flight per thread
+
+// GENERAL: a mask or the plane rules (finite values only); otherwise every
+// pixel may win and NaN never does.
+template <int K, bool GENERAL>
+__global__ void __launch_bounds__(kHogRegThreads, 1) hogbom_reg_kernel(HogRegArgs g) {
+    __shared__ int s_abs[kHogRegWarps], s_abs2[kHogRegWarps];
+    __shared__ unsigned s_ks[kHogRegWarps];
+    __shared__ unsigned s_key;
+    const HogArgs& a = g.a;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wid = (int)blockIdx.x * kHogRegWarps + warp;
+    const int x0 = (wid / g.cols) * g.rows;
+    const int y = (wid % g.cols) * 32 + lane;
+    const int nrow = y < a.ny ? min(g.rows, a.nx - x0) : 0;   // may be <= 0
+    const float lim = a.plane_rules ? 3.402823466e38f : __int_as_float(0x7f800000);
+    const int kcx = a.nx / 2, kcy = a.ny / 2;
+    float r[K];
+    unsigned open[GENERAL ? (K + 31) / 32 : 1] = {};   // pixels that may win
+    const int64_t base = (int64_t)x0 * a.ny + y;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        // a missing pixel holds NaN, which never wins
+        r[k] = k < nrow ? a.residual[base + (int64_t)k * a.ny] : __int_as_float(0x7fc00000);
+        if (GENERAL && k < nrow && (!a.mask || a.mask[base + (int64_t)k * a.ny]))
+            open[k >> 5] |= 1u << (k & 31);
+    }
+    auto wins = [&](int k, float av) {
+        return !GENERAL || (((open[k >> 5] >> (k & 31)) & 1u) && av <= lim);
+    };
+    float m = -1.0f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const float av = fabsf(r[k]);
+        if (wins(k, av)) m = fmaxf(m, av);
+    }
+    long long it = 0;
+    int stop = CR_STOP_NONE;
+    for (;; ++it) {
+        // the block's candidate: the largest |value|, then its smallest key
+        const int wm = __reduce_max_sync(0xffffffffu, __float_as_int(m));
+        if (lane == 0) s_abs2[warp] = wm;
+        if (tid == 0) s_key = 0xffffffffu;
+        __syncthreads();
+        const int bm = __reduce_max_sync(0xffffffffu, s_abs2[lane & (kHogRegWarps - 1)]);
+        if (bm >= 0 && __float_as_int(m) == bm) {
+            const float fm = __int_as_float(bm);
+            unsigned key = 0xffffffffu;
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (fabsf(r[k]) == fm && wins(k, fm))
+                    key = min(key, ((unsigned)y * (unsigned)a.nx + (unsigned)(x0 + k)) << 1 |
+                                       (__float_as_uint(r[k]) >> 31));
+            atomicMin(&s_key, key);
+        }
+        __syncthreads();
+        if (it >= a.budget) break;
+        int babs;
+        unsigned bks;
+        if (!hogreg_exchange(g, it, bm, s_key, s_abs, s_ks, &babs, &bks)) {
+            if (tid == 0) atomicExch(a.out_status, CR_TIMEOUT);
+            return;
+        }
+        const float absval = babs < 0 ? -1.0f : __int_as_float(babs);
+        if (babs < 0)
+            stop = CR_STOP_NO_CLEANABLE_PIXELS;
+        else if (a.plane_rules)
+            stop = absval <= a.threshold         ? CR_STOP_GLOBAL_THRESHOLD
+                   : absval <= a.cycle_threshold ? CR_STOP_CYCLE_THRESHOLD
+                                                 : 0;
+        else
+            stop = stop_reason(absval, a.threshold, a.cycle_threshold, a.nsigma_threshold);
+        if (stop) break;
+        const int key = (int)(bks >> 1);
+        const float value = (bks & 1u) ? -absval : absval;
+        const int py = key / a.nx, px = key - py * a.nx;
+        const float comp = __fmul_rn(a.gain, value);
+        if (blockIdx.x == 0 && tid == 0) {
+            const int64_t p = (int64_t)px * a.ny + py;
+            a.model[p] = __fadd_rn(a.model[p], comp);
+            if (a.comp_x) {
+                a.comp_x[it] = px;
+                a.comp_y[it] = py;
+                a.comp_peak[it] = value;
+                a.comp_flux[it] = comp;
+            }
+        }
+        // subtract the shifted PSF where it overlaps, and the thread's next
+        // largest |value|
+        const int ky = y - py + kcy, kx0 = x0 - px + kcx;
+        const bool col = ky >= 0 && ky < a.ny;
+        const int lo = max(0, -kx0), hi = col ? min(nrow, a.nx - kx0) : 0;
+        const unsigned span = hi > lo ? (unsigned)(hi - lo) : 0u;
+        const float* p = a.psf + ((int64_t)kx0 * a.ny + ky);
+        m = -1.0f;
+#pragma unroll
+        for (int k0 = 0; k0 < K; k0 += kHogRegLoads) {
+            float v[kHogRegLoads];
+#pragma unroll
+            for (int j = 0; j < kHogRegLoads && k0 + j < K; ++j)
+                v[j] = load_if((unsigned)(k0 + j - lo) < span, p + (k0 + j) * a.ny);
+#pragma unroll
+            for (int j = 0; j < kHogRegLoads && k0 + j < K; ++j) {
+                const int k = k0 + j;
+                if ((unsigned)(k - lo) < span) r[k] = __fsub_rn(r[k], __fmul_rn(comp, v[j]));
+                const float av = fabsf(r[k]);
+                if (wins(k, av)) m = fmaxf(m, av);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (k < nrow) a.residual[base + (int64_t)k * a.ny] = r[k];
+    if (blockIdx.x == 0 && tid == 0) {
+        *a.out_actual = it;
+        *a.out_stop = stop;
+    }
+}
+
+// Register rows a warp may hold; an image needs the smallest K that covers
+// it with one block per SM (K = 96 reaches 2733^2 on 152 SMs).
+constexpr int kHogRegRows[] = {4, 8, 16, 32, 44, 56, 68, 80, 96};
+
+const void* hogreg_kernel(int rows, bool general) {
+    switch (rows) {
+#define CR_HOGREG_CASE(N)                                              \
+    case N:                                                            \
+        return general ? (const void*)hogbom_reg_kernel<N, true>       \
+                       : (const void*)hogbom_reg_kernel<N, false>;
+        CR_HOGREG_CASE(4)
+        CR_HOGREG_CASE(8)
+        CR_HOGREG_CASE(16)
+        CR_HOGREG_CASE(32)
+        CR_HOGREG_CASE(44)
+        CR_HOGREG_CASE(56)
+        CR_HOGREG_CASE(68)
+        CR_HOGREG_CASE(80)
+        CR_HOGREG_CASE(96)
+#undef CR_HOGREG_CASE
+    }
+    return nullptr;
+}
+
+// How an image is split for hogbom_reg_kernel: rows per warp, the template's
+// K and the blocks; K = 0 when it does not fit the registers of one block per
+// SM (hogbom_kernel takes it then).
+struct HogSplit {
+    int k = 0, rows = 0, cols = 0, blocks = 0;
+};
+
+HogSplit hogreg_split(int32_t nx, int32_t ny, int sms) {
+    HogSplit s;
+    s.cols = (ny + 31) / 32;
+    const int64_t groups = (int64_t)sms * kHogRegWarps / s.cols;   // row groups that fit
+    if (groups < 1) return s;
+    const int64_t rows = std::max<int64_t>(4, (nx + groups - 1) / groups);
+    for (int k : kHogRegRows)
+        if (rows <= k) {
+            s.k = k;
+            s.rows = (int)rows;
+            const int64_t warps = (int64_t)s.cols * ((nx + rows - 1) / rows);
+            s.blocks = (int)((warps + kHogRegWarps - 1) / kHogRegWarps);
+            break;
+        }
+    return s;
+}
+
 // Several images [P][nx][ny] at once: `per_plane` blocks for each listed
 // plane, each group with its own barrier words, candidates, component list
 // and results (slot s = the plane's position in the list).
@@ -355,33 +616,48 @@ void hogbom(cr_ctx* ctx, float* model, float* residual, const float* psf, const 
     if ((int64_t)nx * ny >= (1ll << 31)) fail(CR_INVALID, "image larger than 2^31 pixels");
     if (cycle_niter < 0) fail(CR_INVALID, "cycle_niter is negative");
     long long budget = inclusive ? cycle_niter + 1 : cycle_niter;
-    int sms = 0, per_sm = 0;
-    CR_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    CR_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hogbom_kernel,
-                                                                kHogThreads, 0));
-    if (per_sm < 1) fail(CR_CUDA, "Hogbom kernel cannot be resident");
-    int64_t npix = (int64_t)nx * ny;
-    int blocks = (int)std::min<int64_t>((int64_t)sms * std::min(per_sm, 2),
-                                        std::max<int64_t>(1, (npix + kHogThreads - 1) / kHogThreads));
-    size_t cap = (size_t)(budget > 0 ? budget : 1);
-    char* wsp = (char*)workspace(ctx, "hog_ws", 256 + (size_t)blocks * 2 * sizeof(Cand) + cap * 16);
+    const HogSplit split = hogreg_split(nx, ny, ctx->sms);
+    int blocks = split.blocks;
+    if (!split.k) {
+        int per_sm = 0;
+        CR_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hogbom_kernel,
+                                                                    kHogThreads, 0));
+        if (per_sm < 1) fail(CR_CUDA, "Hogbom kernel cannot be resident");
+        const int64_t npix = (int64_t)nx * ny;
+        blocks = (int)std::min<int64_t>((int64_t)ctx->sms * std::min(per_sm, 2),
+                                        (npix + kHogThreads - 1) / kHogThreads);
+    }
+    const size_t cap = (size_t)(budget > 0 ? budget : 1);
+    // the exchange words, or the candidates
+    const size_t cand_b = split.k ? (size_t)blocks * blocks * 16
+                                  : (size_t)blocks * 2 * sizeof(Cand);
+    char* wsp = (char*)workspace(ctx, "hog_ws", 256 + cand_b + cap * 16);
     unsigned int* bar = (unsigned int*)wsp;
     long long* out_actual = (long long*)(wsp + 16);
     int* out_stop = (int*)(wsp + 24);
     int* out_status = (int*)(wsp + 28);
     Cand* cands = (Cand*)(wsp + 256);
-    int* cx = (int*)(wsp + 256 + (size_t)blocks * 2 * sizeof(Cand));
+    int* cx = (int*)(wsp + 256 + cand_b);
     int* cy = cx + cap;
     float* cp = (float*)(cy + cap);
     float* cf = cp + cap;
-    CR_CUDA_CHECK(cudaMemsetAsync(wsp, 0, 256, ctx->stream));
+    CR_CUDA_CHECK(cudaMemsetAsync(wsp, 0, 256 + cand_b, ctx->stream));
     HogArgs a{model, residual, psf, mask, nx, ny, gain, threshold, cycle_threshold,
               nsigma_threshold, budget, cands, bar, cx, cy, cp, cf, out_actual, out_stop,
               out_status, plane_rules, ctx->barrier_polls};
-    void* args[] = {&a};
-    CR_CUDA_CHECK(cudaLaunchCooperativeKernel((void*)hogbom_kernel, dim3(blocks), dim3(kHogThreads),
-                                              args, 0, ctx->stream));
-    note_launch(ctx, "hogbom_kernel");
+    if (split.k) {
+        HogRegArgs g{a, (unsigned long long*)cands, split.cols, split.rows};
+        void* args[] = {&g};
+        CR_CUDA_CHECK(cudaLaunchCooperativeKernel(hogreg_kernel(split.k, mask || plane_rules),
+                                                  dim3(blocks), dim3(kHogRegThreads), args, 0,
+                                                  ctx->stream));
+        note_launch(ctx, "hogbom_reg_kernel");
+    } else {
+        void* args[] = {&a};
+        CR_CUDA_CHECK(cudaLaunchCooperativeKernel((void*)hogbom_kernel, dim3(blocks),
+                                                  dim3(kHogThreads), args, 0, ctx->stream));
+        note_launch(ctx, "hogbom_kernel");
+    }
     struct {
         long long actual;
         int stop, status;
