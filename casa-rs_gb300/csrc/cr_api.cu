@@ -91,9 +91,9 @@ void set_timings(cr_ctx* ctx, cr_timings t) {
 
 void bind(cr_ctx* ctx) { CR_CUDA_CHECK(cudaSetDevice(ctx->device)); }
 
-Records plan(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const DeviceBatch& b,
+Records plan(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const DeviceBatch& b, int use,
              Pool* pool = nullptr) {
-    return wp ? plan_wproj(ctx, wp, b, pool) : plan_standard(ctx, g, b, pool);
+    return wp ? plan_wproj(ctx, wp, b, use, pool) : plan_standard(ctx, g, b, use, pool);
 }
 
 void grid_records(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const Records& r, float2* psf,
@@ -580,7 +580,7 @@ int cr_grid_dirty(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* 
         float2* dirty = out_ptr<float2>(ctx, dirty_grid, out_location, gb, "dirty_grid");
         CR_CUDA_CHECK(cudaMemsetAsync(psf, 0, gb, ctx->stream));
         CR_CUDA_CHECK(cudaMemsetAsync(dirty, 0, gb, ctx->stream));
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSums);
         tm.mark();
         grid_records(ctx, g, wp, r, psf, dirty, 0);
         tm.mark();
@@ -607,7 +607,7 @@ int cr_degrid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* batc
         StagedBatch b(ctx, batch, wp != nullptr);
         const float2* grid = (const float2*)device_input(ctx, model_grid, grid_bytes(g),
                                                          grid_location, "model_grid");
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSamples);
         tm.mark();
         degrid_records(ctx, g, wp, r, grid);
         float2* out = out_ptr<float2>(ctx, pred, out_location, (size_t)b.n * 8 + 8, "pred");
@@ -615,6 +615,7 @@ int cr_degrid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* batc
         tm.mark();
         if (out_location == CR_HOST) copy_out(ctx, pred, out, (size_t)b.n * 8, CR_HOST);
         CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        check_device_status(ctx);
         set_timings(ctx, cr_timings{tm.between(0, 1), 0.f, tm.between(1, 2), 0.f, 0.f});
     });
 }
@@ -628,7 +629,7 @@ int cr_grid_residual(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batc
         bind(ctx);
         StagedBatch b(ctx, batch, wp != nullptr);
         size_t gb = grid_bytes(g);
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSums);
         if (model_grid) {
             const float2* grid = (const float2*)device_input(ctx, model_grid, gb, grid_location,
                                                              "model_grid");
@@ -742,7 +743,7 @@ int cr_dirty_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch*
         float2* dirty = (float2*)workspace(ctx, "di_dirty", gb);
         CR_CUDA_CHECK(cudaMemsetAsync(psf, 0, gb, ctx->stream));
         CR_CUDA_CHECK(cudaMemsetAsync(dirty, 0, gb, ctx->stream));
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSums);
         tm.mark();
         grid_records(ctx, g, wp, r, psf, dirty, 0);
         tm.mark();
@@ -769,7 +770,7 @@ int cr_residual_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_bat
         const float* m = (const float*)device_input(ctx, model, np * 4, model_location, "model");
         float2* mgrid = (float2*)workspace(ctx, "ri_model_grid", gb);
         image_to_grid(ctx, g, wp, m, mgrid, image_single(ctx));
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSums);
         degrid_records(ctx, g, wp, r, mgrid);
         float2* res = (float2*)workspace(ctx, "ri_residual_grid", gb);
         CR_CUDA_CHECK(cudaMemsetAsync(res, 0, gb, ctx->stream));
@@ -802,13 +803,14 @@ int cr_predict(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* bat
         float2* mgrid = (float2*)workspace(ctx, "pr_model_grid", gb);
         image_to_grid(ctx, g, wp, m, mgrid, image_single(ctx));
         fork.to_main();
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSamples);
         fork.join();
         degrid_records(ctx, g, wp, r, mgrid);
         float2* out = out_ptr<float2>(ctx, pred, out_location, (size_t)b.n * 8 + 8, "pred");
         broadcast_pred(ctx, r, out);
         if (out_location == CR_HOST) copy_out(ctx, pred, out, (size_t)b.n * 8, CR_HOST);
         CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        check_device_status(ctx);
     });
 }
 
@@ -820,7 +822,7 @@ int cr_adjoint(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* bat
         bind(ctx);
         StagedBatch b(ctx, batch, wp != nullptr);
         size_t gb = grid_bytes(g);
-        Records r = plan(ctx, g, wp, b);
+        Records r = plan(ctx, g, wp, b, kPlanSums);
         CR_CUDA_CHECK(cudaMemsetAsync(r.rec_pred, 0, (size_t)(b.n > 0 ? b.n : 1) * 8, ctx->stream));
         float2* grid = (float2*)workspace(ctx, "adj_grid", gb);
         CR_CUDA_CHECK(cudaMemsetAsync(grid, 0, gb, ctx->stream));
@@ -833,6 +835,7 @@ int cr_adjoint(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch* bat
         grid_to_image_adjoint(ctx, g, wp, grid, n2, img, image_single(ctx));
         if (out_location == CR_HOST) copy_out(ctx, image, img, np * 4, CR_HOST);
         CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        check_device_status(ctx);
     });
 }
 
@@ -851,7 +854,7 @@ int cr_plan_create(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch*
         p->g = g;
         p->wp = wp;
         try {
-            p->rec = plan(ctx, g, wp, b, &p->pool);
+            p->rec = plan(ctx, g, wp, b, kPlanAll, &p->pool);
             tm.mark();
             read_sums(ctx, p->rec, &p->sums);
         } catch (...) {
@@ -1731,7 +1734,7 @@ int cr_accumulator_add(cr_ctx* ctx, cr_accumulator* a, const cr_vis_batch* batch
         StageTimer tm(ctx);
         tm.mark();
         StagedBatch b(ctx, batch, false);
-        Records r = plan(ctx, a->g, nullptr, b);
+        Records r = plan(ctx, a->g, nullptr, b, kPlanSums);
         tm.mark();
         grid_records(ctx, a->g, nullptr, r, a->psf, a->dirty, 0);
         tm.mark();

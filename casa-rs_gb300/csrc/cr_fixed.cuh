@@ -191,6 +191,19 @@ struct PairSum {
     }
 };
 
+// float32(v - pred w) of a record's sums v = (re, im) and w, float32 pairs.
+__device__ __forceinline__ float2 residual_value(float4 v, float2 w, float2 pred) {
+    auto diff = [&](float vh, float vl, float p) {
+        const float ph = __fmul_rn(p, w.x);
+        PairSum d;
+        d.h = vh;
+        d.l = vl;
+        d.add(-ph, -__fmaf_rn(p, w.y, __fmaf_rn(p, w.x, -ph)));
+        return d.h;
+    };
+    return make_float2(diff(v.x, v.y, pred.x), diff(v.z, v.w, pred.y));
+}
+
 // The integer a nearest to x = p + e + h (h = 0 or 1/2) and dh = RN(p + h) - a
 // (exact), or false when x is within the margin of a half-integer, is
 // large, or is not finite.

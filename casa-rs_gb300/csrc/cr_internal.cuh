@@ -77,6 +77,9 @@ struct DfPlan;      // a float-pair transform plan for one line length (cr_dfft.
 // polls: milliseconds).  cr_ctx_set_wait_limits lowers them for tests.
 constexpr long long kBarrierPollsDefault = 1ll << 24;
 constexpr long long kMbarPollsDefault = 1ll << 22;
+// and of a look-back wait for an earlier tile of the same launch (polls of a
+// word in L2: a second or two)
+constexpr long long kLookbackPolls = 1ll << 21;
 // pieces of a staged host batch upload (StagedBatch)
 constexpr int kStageChunks = 4;
 
@@ -217,9 +220,32 @@ std::vector<float> sinc_axis(int64_t size, int64_t conv_sampling);
 // non-null, device pointer) receives the sum as uint64.
 void exclusive_scan_u32(cr_ctx* ctx, const uint32_t* in, uint32_t* out, int64_t n,
                         unsigned long long* total_dev);
-// Stable LSD radix sort of (key, value) pairs on the low `bits` bits.
-// Sorted output ends in keys/vals.
-void radix_sort_pairs(cr_ctx* ctx, uint64_t* keys, uint32_t* vals, int64_t n, int bits);
+// Stable LSD radix sort of 64-bit keys (on their low `bits` bits) with the
+// items' indices.  radix_sort_begin allocates and clears the sort's state; the
+// kernel that makes the keys adds their digits to `hist` (digit p of key k,
+// (k >> 8 p) & 255, counted at hist[256 p + digit], 256 * passes counters);
+// radix_sort_run then sorts.  A bounded wait that gives up sets *fail (device)
+// and the context's status word; the sorted arrays are undefined then.
+struct RadixSort {
+    int64_t n = 0;
+    int passes = 0;
+    int64_t tiles = 0;
+    uint32_t* hist = nullptr;
+    uint32_t* tickets = nullptr;          // one per pass
+    unsigned int* fail = nullptr;
+    unsigned long long* state = nullptr;  // [tiles][256]
+    uint64_t* keys = nullptr;             // unsorted keys are written here
+    const uint64_t* sorted_keys = nullptr;
+    const uint32_t* order = nullptr;      // index of each sorted item
+    // for the pass over the sorted keys that follows: one ticket and a word
+    // per kRecTile items, cleared with the rest
+    uint32_t* rec_ticket = nullptr;
+    unsigned long long* rec_state = nullptr;
+};
+constexpr int kRadixBins = 256;
+constexpr int kRecTile = 1024;
+RadixSort radix_sort_begin(cr_ctx* ctx, int64_t n, int bits);
+void radix_sort_run(cr_ctx* ctx, RadixSort& s);
 
 // ---- batch upload ------------------------------------------------------------
 struct DeviceBatch {
@@ -275,32 +301,41 @@ int64_t prepare_rows(cr_ctx* ctx, const cr_row_runs* rr, const cr_polarization* 
 
 // ---- records: the deduplicated sample plan ------------------------------------
 // Samples with identical (cell, kernel offset, w-plane, conjugation) get
-// identical taps; they are summed into one record before gridding.
+// identical taps; they are summed into one record before gridding.  Records
+// are sorted by home tile, then by plane, conjugation, offset and cell
+// (W-projection) or cell and tap rows (standard).
 struct Records {
     int64_t n_samples = 0;
-    uint64_t* keys = nullptr;        // sorted keys [n]
-    uint32_t* order = nullptr;       // sorted sample indices [n]
     int32_t* sample_rec = nullptr;   // [n] record of each sample, -1 when skipped
-    int32_t* rec_x = nullptr;        // anchor / start cell x   [n]
-    int32_t* rec_y = nullptr;        // [n]
-    int32_t* rec_a = nullptr;        // plane (wproj) or x tap row (standard)  [n]
-    int32_t* rec_b = nullptr;        // offset index (wproj) or y tap row      [n]
-    int32_t* rec_conj = nullptr;     // [n]
-    double2* rec_vsum = nullptr;     // sum vis * weight  [n]
-    double* rec_wsum = nullptr;      // sum weight        [n]
+    int2* rec_xy = nullptr;          // anchor (W-projection) or start cell [n]
+    // W-projection: plane | conj << 12 | offset index << 13; standard: x tap
+    // row | y tap row << 16
+    uint32_t* rec_meta = nullptr;
+    // sums of vis * weight and of weight, as float32 pairs (hi + lo)
+    float4* rec_vsum = nullptr;      // (re hi, re lo, im hi, im lo)  [n]
+    float2* rec_wsum = nullptr;      // [n]
     float2* rec_pred = nullptr;      // degridded value   [n]
     uint32_t* tile_start = nullptr;  // [ntiles + 1] first record of each home tile
     int64_t ntx = 0, nty = 0;        // home tiles (32 x 32 cells)
-    // device scalars: [0] gridded, [1] skipped, [2] unique records
+    // device scalars: [0] gridded, [1] skipped, [2] unique records, [3] taps
     unsigned long long* counts = nullptr;
     double* sums = nullptr;          // [0] normalisation sumwt, [1] reported sumwt
+};
+
+// What a plan's caller uses of its records.
+enum : int {
+    kPlanSums = 1,      // rec_vsum, rec_wsum (gridding)
+    kPlanSamples = 2,   // sample_rec (predictions per sample)
+    kPlanAll = 3
 };
 
 constexpr int kTile = 32;            // home/output tile edge in grid cells
 
 // The records live in `pool` (the context's workspaces when null).
-Records plan_wproj(cr_ctx* ctx, cr_wproj* wp, const DeviceBatch& b, Pool* pool = nullptr);
-Records plan_standard(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, Pool* pool = nullptr);
+Records plan_wproj(cr_ctx* ctx, cr_wproj* wp, const DeviceBatch& b, int use,
+                   Pool* pool = nullptr);
+Records plan_standard(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, int use,
+                      Pool* pool = nullptr);
 void read_sums(cr_ctx* ctx, const Records& r, cr_sums* out);
 
 // ---- gridding kernels ----------------------------------------------------------

@@ -10,12 +10,14 @@
 // the reference's FP64 operations otherwise: GB300 issues FP64 at a small
 // fraction of its float32 rate, and planning was FP64-bound.  Each valid
 // sample gets a 64-bit key
-//   home tile | (plane | conj | offset)  or  (x tap row | y tap row) | cell
+//   home tile | plane | conj | offset | cell   (W-projection)
+//   home tile | cell | x tap row | y tap row   (standard)
 // and the keys are radix-sorted.  Samples with equal keys have identical taps;
 // their weighted visibilities and weights are summed into one record, so
 // every distinct tap footprint is convolved once.  The sort is stable; the
 // sums of weights and the record sums are compensated float32-pair sums of
-// exact products, carried in FP64 across warps.
+// exact products, the sums of weights carried in FP64 across warps.
+#include <algorithm>
 #include <cmath>
 
 #include "cr_fixed.cuh"
@@ -30,6 +32,39 @@ __host__ __device__ inline int bits_for(uint64_t max_value) {
     while ((max_value >> b) != 0) ++b;
     return b;
 }
+
+// Where a plan kernel puts the keys: the key of each sample, the digit counts
+// of the sort's passes, and -1 as the record of a skipped sample.
+struct KeyOut {
+    uint64_t* keys;
+    uint32_t* hist;        // [passes][256]
+    int passes;
+    int32_t* sample_rec;   // or null
+};
+
+// The digits of a block's keys counted in shared memory, added to the global
+// counts once per block.
+struct KeyCounts {
+    uint32_t* s;           // [passes][256] in shared memory
+    __device__ void begin(const KeyOut& o) {
+        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x) s[k] = 0;
+        __syncthreads();
+    }
+    __device__ void put(const KeyOut& o, int64_t i, uint64_t key) {
+        o.keys[i] = key;
+        if (o.sample_rec && key == ~0ull) o.sample_rec[i] = -1;
+        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+            if (p < o.passes)
+                atomicAdd(&s[p * kRadixBins + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
+    }
+    __device__ void end(const KeyOut& o) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x)
+            if (s[k]) atomicAdd(&o.hist[k], s[k]);
+    }
+};
 
 struct WpPlanArgs {
     int64_t first, n;   // samples [first, n)
@@ -46,8 +81,7 @@ struct WpPlanArgs {
     int plane_bits, off_bits;
     DfScale kx, ky;            // 1 / du, 1 / dv as float32 pairs
     DfScale kw;                // w_scale as a float32 pair
-    uint64_t* keys;
-    uint32_t* vals;
+    KeyOut out;
     double* sums;
     unsigned long long* counts;
 };
@@ -62,39 +96,6 @@ __device__ __forceinline__ unsigned long long warp_sum_u(unsigned long long x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     return x;
-}
-
-// Block-wide accumulation of two FP64 sums and two counters, from values
-// already summed over each warp (held by lane 0).
-__device__ void block_finish(double s0, double s1, unsigned long long c0, unsigned long long c1,
-                             double* sums, unsigned long long* counts) {
-    __shared__ double sh_s[2][32];
-    __shared__ unsigned long long sh_c[2][32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) {
-        sh_s[0][warp] = s0;
-        sh_s[1][warp] = s1;
-        sh_c[0][warp] = c0;
-        sh_c[1][warp] = c1;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        s0 = lane < nw ? sh_s[0][lane] : 0.0;
-        s1 = lane < nw ? sh_s[1][lane] : 0.0;
-        c0 = lane < nw ? sh_c[0][lane] : 0ull;
-        c1 = lane < nw ? sh_c[1][lane] : 0ull;
-        s0 = warp_sum_d(s0);
-        s1 = warp_sum_d(s1);
-        c0 = warp_sum_u(c0);
-        c1 = warp_sum_u(c1);
-        if (lane == 0) {
-            if (s0 != 0.0) atomicAdd(&sums[0], s0);
-            if (s1 != 0.0) atomicAdd(&sums[1], s1);
-            if (c0) atomicAdd(&counts[0], c0);
-            if (c1) atomicAdd(&counts[1], c1);
-        }
-    }
-    __syncthreads();
 }
 
 // The FP64 operations kept out of line, so that the compiler branches around
@@ -317,6 +318,9 @@ __device__ __noinline__ WpDecision wp_decide_fp64(double u, double v, double w, 
 // The anchors, offsets and plane come from the float32-pair path above when
 // it decides them, else from the reference's FP64 operations.
 __global__ void __launch_bounds__(256) wp_plan_kernel(WpPlanArgs a) {
+    __shared__ uint32_t s_hist[8 * kRadixBins];
+    KeyCounts counts{s_hist};
+    counts.begin(a.out);
     PairSum s_norm, s_rep;
     double f_norm = 0.0, f_rep = 0.0;
     bool fb_used = false;
@@ -389,9 +393,9 @@ __global__ void __launch_bounds__(256) wp_plan_kernel(WpPlanArgs a) {
             c_ok++;
         else
             c_skip++;
-        a.keys[i] = key;
-        a.vals[i] = (uint32_t)i;
+        counts.put(a.out, i, key);
     }
+    counts.end(a.out);
     block_accumulate(s_norm, s_rep, f_norm, f_rep, fb_used, c_ok, c_skip, a.sums, a.counts);
 }
 
@@ -405,8 +409,7 @@ struct StdPlanArgs {
     int32_t os, tap_rows;
     int64_t nty;
     DfScale kx, ky;            // 1 / du, 1 / dv as float32 pairs
-    uint64_t* keys;
-    uint32_t* vals;
+    KeyOut out;
     double* sums;
     unsigned long long* counts;
 };
@@ -452,6 +455,9 @@ __device__ __noinline__ StdSpans std_spans_fp64(double u, double v, double du, d
 // accumulate_dirty_psf_and_residual_standard_streaming_grid_serial
 // (lib.rs:68433-68500): validity, taps, sum of weights grid_weight = w*f.
 __global__ void __launch_bounds__(256) std_plan_kernel(StdPlanArgs a) {
+    __shared__ uint32_t s_hist[8 * kRadixBins];
+    KeyCounts counts{s_hist};
+    counts.begin(a.out);
     PairSum s_norm;
     double f_norm = 0.0;
     unsigned long long c_ok = 0, c_skip = 0;
@@ -493,162 +499,325 @@ __global__ void __launch_bounds__(256) std_plan_kernel(StdPlanArgs a) {
                 s_norm.add(__fmul_rn(wt, f), 0.0f);
                 uint64_t tile = (uint64_t)(x0 >> 5) * (uint64_t)a.nty + (uint64_t)(y0 >> 5);
                 uint64_t cell = (uint64_t)(((x0 & 31) << 5) | (y0 & 31));
-                key = (((tile << 8 | (uint64_t)rx) << 8 | (uint64_t)ry) << 10) | cell;
+                key = ((tile << 10 | cell) << 8 | (uint64_t)rx) << 8 | (uint64_t)ry;
             }
         }
         if (ok)
             c_ok++;
         else
             c_skip++;
-        a.keys[i] = key;
-        a.vals[i] = (uint32_t)i;
+        counts.put(a.out, i, key);
     }
+    counts.end(a.out);
     block_accumulate(s_norm, s_norm, f_norm, f_norm, false, c_ok, c_skip, a.sums, a.counts);
 }
 
-__global__ void head_flags(const uint64_t* keys, const unsigned long long* counts, int64_t n,
-                           uint32_t* flags) {
-    int64_t nv = (int64_t)counts[0];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        flags[i] = (i < nv && (i == 0 || keys[i] != keys[i - 1])) ? 1u : 0u;
-}
-
 struct RecArgs {
-    const uint64_t* keys;
-    const uint32_t* vals;
-    const uint32_t* flags;
-    const uint32_t* excl;
-    const unsigned long long* counts;
+    const uint64_t* keys;      // sorted
+    const uint32_t* order;     // the sample of each sorted key
+    unsigned long long* counts;
     int64_t n;
-    int mode;  // 0 wproj, 1 standard
+    int mode;                  // 0 wproj, 1 standard
     int plane_bits, off_bits;
-    int64_t nty;
-    int32_t *rx, *ry, *ra, *rb, *rconj;
-    double2* vsum;
-    double* wsum;
-    int32_t* sample_rec;
+    int64_t nty, ntiles;
+    int2* xy;
+    uint32_t* meta;
+    float4* vsum;              // or null: the records' sums are not used
+    float2* wsum;
+    int32_t* sample_rec;       // or null
     const float* weight;
     const float* sumwt;
     const float2* vis;
-    uint32_t* tile_of;
-    const int32_t* support;   // per plane (W-projection); null: 7 x 7 standard taps
+    const int32_t* support;    // per plane (W-projection); null: 7 x 7 standard taps
+    uint32_t* tile_start;      // [ntiles + 1]
+    // per warp range: the sums of its leading items that belong to a record
+    // begun in an earlier range, that record (~0: none), and bit 0: a record
+    // begins in the range
+    float4* lead_v;
+    float2* lead_w;
+    uint32_t* lead_rec;
+    uint32_t* lead_flags;
+    uint32_t* ticket;
+    unsigned long long* state; // [tiles] as the sort's state words, tag 0
+    unsigned int* fail;
+    int* status;
 };
 
-// Record fields decoded from the head key of each run.
-// Also counts the taps one grid pass applies (counts[3]).
-__global__ void records_init(RecArgs a) {
-    int64_t nv = (int64_t)a.counts[0];
+constexpr int kRecThreads = 256;
+constexpr int kRecRounds = kRecTile / kRecThreads;   // rounds of 32 items per warp
+constexpr int kRecRange = 32 * kRecRounds;           // a warp's items
+constexpr uint32_t kNoRecord = 0xffffffffu;
+
+struct RecSum {
+    PairSum r, i, w;
+    __device__ __forceinline__ void add(const RecSum& o) {
+        r.add(o.r.h, o.r.l);
+        i.add(o.i.h, o.i.l);
+        w.add(o.w.h, o.w.l);
+    }
+};
+
+__device__ __forceinline__ RecSum shfl_rec(const RecSum& s, int src) {
+    RecSum o;
+    o.r.h = __shfl_sync(0xffffffffu, s.r.h, src);
+    o.r.l = __shfl_sync(0xffffffffu, s.r.l, src);
+    o.i.h = __shfl_sync(0xffffffffu, s.i.h, src);
+    o.i.l = __shfl_sync(0xffffffffu, s.i.l, src);
+    o.w.h = __shfl_sync(0xffffffffu, s.w.h, src);
+    o.w.l = __shfl_sync(0xffffffffu, s.w.l, src);
+    return o;
+}
+
+// The sorted keys to records in one pass: heads of equal-key runs counted per
+// tile, the records before a tile by look-back, each run's sums by a
+// segmented scan carried from round to round.  A run's sums are stored by the
+// warp that holds its head; a later warp range that continues the run leaves
+// its part in lead_*, which records_finish adds.  One launch instead of five
+// (head flags, scan, record fields, memset and FP64 atomics of the sums):
+// 5.05 M samples 215 -> 150 us with records_finish, 4,001 samples 22 -> 17 us.
+// Bound by the gathers of weight and visibility (two 32-byte sectors per
+// sample).
+__global__ void __launch_bounds__(kRecThreads) records_kernel(RecArgs a) {
+    __shared__ uint32_t s_heads[kRecThreads / 32];
+    __shared__ uint32_t s_base, s_tile;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // a sort that failed leaves no records
+    const int64_t nv = *(volatile unsigned int*)a.fail ? 0 : (int64_t)a.counts[0];
+    if (tid == 0) s_tile = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile;
+    if (tile * kRecTile >= nv) return;
+    const int64_t range0 = tile * kRecTile + warp * kRecRange;
+    uint64_t key[kRecRounds];
+    uint32_t sample[kRecRounds], heads[kRecRounds], total = 0;
+#pragma unroll
+    for (int j = 0; j < kRecRounds; ++j) {
+        const int64_t i = range0 + 32 * j + lane;
+        key[j] = i < nv ? a.keys[i] : 0ull;
+        sample[j] = i < nv ? a.order[i] : kNoRecord;
+    }
+    // the samples' gathers are in flight while the look-back runs
+    float gw[kRecRounds];
+    float2 z[kRecRounds];
+    if (a.vsum) {
+#pragma unroll
+        for (int j = 0; j < kRecRounds; ++j) {
+            const uint32_t s = sample[j];
+            const bool ok = s != kNoRecord;
+            gw[j] = ok ? a.weight[s] : 0.0f;
+            z[j] = ok ? a.vis[s] : make_float2(0.0f, 0.0f);
+            if (ok && a.mode != 0 && a.sumwt) gw[j] = gw[j] * a.sumwt[s];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kRecRounds; ++j) {
+        const int64_t i = range0 + 32 * j + lane;
+        uint64_t prev = __shfl_up_sync(0xffffffffu, key[j], 1);
+        const uint64_t last = j ? __shfl_sync(0xffffffffu, key[j > 0 ? j - 1 : 0], 31) : 0ull;
+        if (lane == 0) prev = j ? last : (i > 0 && i < nv) ? a.keys[i - 1] : ~key[0];
+        heads[j] = __ballot_sync(0xffffffffu, i < nv && key[j] != prev);
+        total += __popc(heads[j]);
+    }
+    if (lane == 0) s_heads[warp] = total;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t h = lane < kRecThreads / 32 ? s_heads[lane] : 0u;
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, h);
+        volatile unsigned long long* st = a.state;
+        if (lane == 0 && tile > 0) st[tile] = 1ull << 32 | sum;
+        uint32_t before = 0;
+        bool good = true;
+        for (int64_t p = tile - 1 - lane; ; p -= 32) {
+            // 32 predecessors at a time, lane 0 the nearest; tile -1 holds 0
+            unsigned long long w = p >= 0 ? st[p] : 2ull << 32;
+            for (long long polls = 0; (w >> 32) == 0;) {
+                if (++polls > kLookbackPolls) {
+                    good = false;
+                    break;
+                }
+                w = st[p];
+            }
+            const unsigned full = __ballot_sync(0xffffffffu, (w >> 32) == 2);
+            const int stop = full ? __ffs(full) - 1 : 31;
+            before += __reduce_add_sync(0xffffffffu, lane <= stop ? (uint32_t)w : 0u);
+            good = __all_sync(0xffffffffu, good);
+            if (full || !good) break;
+        }
+        if (lane == 0) {
+            st[tile] = 2ull << 32 | (before + sum);
+            s_base = good ? before : kNoRecord;
+            if (!good) {
+                atomicExch(a.fail, 1u);
+                atomicExch(a.status, CR_TIMEOUT);
+            } else if ((tile + 1) * kRecTile >= nv) {
+                a.counts[2] = before + sum;
+            }
+        }
+    }
+    __syncthreads();
+    if (s_base == kNoRecord) return;
+    uint32_t rec = s_base;   // records begun before this round
+    for (int w = 0; w < warp; ++w) rec += s_heads[w];
+    const int64_t range = tile * (kRecThreads / 32) + warp;
+    const bool lead = range0 < nv && !(heads[0] & 1u);
+    if (lane == 0 && range0 < nv) {
+        a.lead_rec[range] = lead ? rec - 1 : kNoRecord;
+        a.lead_flags[range] = total ? 1u : 0u;
+    }
     unsigned long long taps = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (!a.flags[i]) continue;
-        uint32_t r = a.excl[i];
-        uint64_t k = a.keys[i];
-        int cx = (int)((k >> 5) & 31), cy = (int)(k & 31);
-        k >>= 10;
-        uint64_t tile;
-        if (a.mode == 0) {
-            a.rb[r] = (int32_t)(k & ((1ull << a.off_bits) - 1));
-            k >>= a.off_bits;
-            a.rconj[r] = (int32_t)(k & 1);
-            k >>= 1;
-            a.ra[r] = (int32_t)(k & ((1ull << a.plane_bits) - 1));
-            k >>= a.plane_bits;
-            tile = k;
-        } else {
-            a.rb[r] = (int32_t)(k & 255);
-            a.ra[r] = (int32_t)((k >> 8) & 255);
-            a.rconj[r] = 0;
-            tile = k >> 16;
-        }
-        a.tile_of[r] = (uint32_t)tile;
-        a.rx[r] = (int32_t)((tile / (uint64_t)a.nty) * 32 + cx);
-        a.ry[r] = (int32_t)((tile % (uint64_t)a.nty) * 32 + cy);
-        a.vsum[r] = make_double2(0.0, 0.0);
-        a.wsum[r] = 0.0;
-        const unsigned long long side =
-            a.support ? 2ull * (unsigned long long)a.support[a.ra[r]] + 1ull : 7ull;
-        taps += side * side;
-    }
+    bool begun = false;      // a record of this range has begun
+    RecSum carry;            // the open run's sum over the earlier rounds
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) taps += __shfl_xor_sync(0xffffffffu, taps, o);
-    if ((threadIdx.x & 31) == 0 && taps)
-        atomicAdd(const_cast<unsigned long long*>(&a.counts[3]), taps);
+    for (int j = 0; j < kRecRounds; ++j) {
+        const int64_t i = range0 + 32 * j + lane;
+        const unsigned hb = heads[j];
+        if (range0 + 32 * j >= nv) break;
+        const uint32_t le = 0xffffffffu >> (31 - lane);
+        const uint32_t seen = __popc(hb & le);
+        const uint32_t r = rec + seen - 1;
+        const bool ok = i < nv;
+        if (ok && a.sample_rec) a.sample_rec[sample[j]] = (int32_t)r;
+        if ((hb >> lane) & 1u) {
+            uint64_t k = key[j];
+            uint64_t tile_id, cell;
+            uint32_t meta;
+            unsigned long long side = 7;
+            if (a.mode == 0) {
+                cell = k & 1023;
+                k >>= 10;
+                const uint32_t off = (uint32_t)(k & ((1ull << a.off_bits) - 1));
+                k >>= a.off_bits;
+                const uint32_t conj = (uint32_t)(k & 1);
+                k >>= 1;
+                const uint32_t plane = (uint32_t)(k & ((1ull << a.plane_bits) - 1));
+                tile_id = k >> a.plane_bits;
+                meta = plane | conj << 12 | off << 13;
+                side = 2ull * (unsigned long long)a.support[plane] + 1ull;
+            } else {
+                meta = (uint32_t)((k >> 8) & 255) | (uint32_t)(k & 255) << 16;
+                cell = (k >> 16) & 1023;
+                tile_id = k >> 26;
+            }
+            a.xy[r] = make_int2((int)((tile_id / (uint64_t)a.nty) * 32 + (cell >> 5)),
+                                (int)((tile_id % (uint64_t)a.nty) * 32 + (cell & 31)));
+            a.meta[r] = meta;
+            taps += side * side;
+        }
+        if (a.vsum) {
+            // w vis and w: the products of two floats as exact pairs
+            RecSum v;
+            v.w.h = gw[j];
+            if (isfinite(z[j].x) && isfinite(z[j].y)) {
+                v.r.h = __fmul_rn(z[j].x, gw[j]);
+                v.r.l = __fmaf_rn(z[j].x, gw[j], -v.r.h);
+                v.i.h = __fmul_rn(z[j].y, gw[j]);
+                v.i.l = __fmaf_rn(z[j].y, gw[j], -v.i.h);
+            }
+            // segmented inclusive scan: distance o only while some run has
+            // more than o items in the round
+            unsigned tail = ~hb;   // lanes with at least o earlier items in their run
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                if (!tail) break;
+                RecSum t;
+                t.r.h = __shfl_up_sync(0xffffffffu, v.r.h, o);
+                t.r.l = __shfl_up_sync(0xffffffffu, v.r.l, o);
+                t.i.h = __shfl_up_sync(0xffffffffu, v.i.h, o);
+                t.i.l = __shfl_up_sync(0xffffffffu, v.i.l, o);
+                t.w.h = __shfl_up_sync(0xffffffffu, v.w.h, o);
+                t.w.l = __shfl_up_sync(0xffffffffu, v.w.l, o);
+                if (lane >= o && ((tail >> lane) & 1u)) v.add(t);
+                tail &= tail << o;
+            }
+            if (seen == 0) v.add(carry);   // the run that reaches into this round
+            const unsigned next = (j + 1 < kRecRounds) ? heads[j + 1 < kRecRounds ? j + 1 : j] & 1u : 1u;
+            const bool last = ok && (i == nv - 1 || (lane < 31 ? (hb >> (lane + 1)) & 1u : next));
+            if (last) {
+                if (begun || seen) {
+                    a.vsum[r] = make_float4(v.r.h, v.r.l, v.i.h, v.i.l);
+                    a.wsum[r] = make_float2(v.w.h, v.w.l);
+                } else {
+                    a.lead_v[range] = make_float4(v.r.h, v.r.l, v.i.h, v.i.l);
+                    a.lead_w[range] = make_float2(v.w.h, v.w.l);
+                }
+            }
+            carry = shfl_rec(v, 31);
+            if (next) carry = RecSum();
+        }
+        rec += __popc(hb);
+        begun = begun || hb != 0u;
+    }
+    taps = warp_sum_u(taps);
+    __shared__ unsigned long long s_taps[kRecThreads / 32];
+    if (lane == 0) s_taps[warp] = taps;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kRecThreads / 32; ++w) taps += s_taps[w];
+        atomicAdd(&a.counts[3], taps);
+    }
 }
 
-// Sums of weight * vis per record: a warp-level segmented reduction over the
-// sorted run in float32 pairs, then one FP64 atomic per segment piece.
-__global__ void records_accumulate(RecArgs a) {
-    int64_t nv = (int64_t)a.counts[0];
+// A warp per range that begins a chain of leading parts: the sums of a run
+// that started in the range before and goes on through this range (and any
+// further ranges that hold nothing else) are added to its record.  The other
+// threads find the first record of every home tile.
+__global__ void __launch_bounds__(kRecThreads) records_finish(RecArgs a) {
     const int lane = threadIdx.x & 31;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t start = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t limit = ((nv + 31) / 32) * 32;
-    for (int64_t i = start; i < limit; i += stride) {
-        bool valid = i < nv;
-        int32_t r = -1;
-        // w vis and w as float32 pairs: the products of two floats exact,
-        // the segment sums compensated (FP64 only for the per-segment atomics)
-        PairSum vr, vi, ww;
-        if (valid) {
-            r = (int32_t)(a.flags[i] ? a.excl[i] : a.excl[i] - 1);
-            uint32_t s = a.vals[i];
-            a.sample_rec[s] = r;
-            float wt = a.weight[s];
-            float f = a.sumwt ? a.sumwt[s] : 1.0f;
-            float gw = a.mode == 0 ? wt : wt * f;
-            float2 v = a.vis[s];
-            ww.h = gw;
-            if (isfinite(v.x) && isfinite(v.y)) {
-                vr.h = __fmul_rn(v.x, gw);
-                vr.l = __fmaf_rn(v.x, gw, -vr.h);
-                vi.h = __fmul_rn(v.y, gw);
-                vi.l = __fmaf_rn(v.y, gw, -vi.h);
-            }
-        }
-        // segmented inclusive scan by record id
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float trh = __shfl_up_sync(0xffffffffu, vr.h, o);
-            const float trl = __shfl_up_sync(0xffffffffu, vr.l, o);
-            const float tih = __shfl_up_sync(0xffffffffu, vi.h, o);
-            const float til = __shfl_up_sync(0xffffffffu, vi.l, o);
-            const float twh = __shfl_up_sync(0xffffffffu, ww.h, o);
-            const float twl = __shfl_up_sync(0xffffffffu, ww.l, o);
-            int32_t rr = __shfl_up_sync(0xffffffffu, r, o);
-            if (lane >= o && rr == r) {
-                vr.add(trh, trl);
-                vi.add(tih, til);
-                ww.add(twh, twl);
-            }
-        }
-        int32_t next = __shfl_down_sync(0xffffffffu, r, 1);
-        bool last = (lane == 31) || (next != r);
-        if (valid && last) {
-            atomic_add_pair(&a.vsum[r].x, vr.h, vr.l);
-            atomic_add_pair(&a.vsum[r].y, vi.h, vi.l);
-            atomic_add_pair(&a.wsum[r], ww.h, ww.l);
-        }
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    const bool failed = *a.fail != 0u;   // a wait gave up: no records
+    const int64_t nrec = failed ? 0 : (int64_t)a.counts[2];
+    if (failed) {
+        if (t0 == 0) a.counts[2] = 0;
+        if (a.sample_rec)
+            for (int64_t i = t0; i < a.n; i += step) a.sample_rec[i] = -1;
     }
-}
-
-__global__ void fill_u32(uint32_t* p, int64_t n, const unsigned long long* value) {
-    uint32_t v = (uint32_t)*value;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
-
-// tile_start[t] = first record whose home tile is >= t.
-__global__ void tile_starts(const uint32_t* tile_of, const unsigned long long* counts,
-                            uint32_t* start) {
-    int64_t nr = (int64_t)counts[2];
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nr;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        int64_t prev = r == 0 ? -1 : (int64_t)tile_of[r - 1];
-        int64_t cur = tile_of[r];
-        for (int64_t t = prev + 1; t <= cur; ++t) start[t] = (uint32_t)r;
+    const int64_t nv = nrec ? (int64_t)a.counts[0] : 0;
+    const int64_t ranges = (nv + kRecRange - 1) / kRecRange;
+    if (a.vsum)
+        for (int64_t g = t0 >> 5; g < ranges; g += step >> 5) {
+            const uint32_t r = a.lead_rec[g];
+            if (r == kNoRecord || !(a.lead_flags[g - 1] & 1u)) continue;   // g > 0 here
+            RecSum s;
+            for (int64_t h = g;; h += 32) {
+                // this lane's range belongs to the chain while every range
+                // before it in the chain begins no record
+                const int64_t k = h + lane;
+                const bool mine = k < ranges && a.lead_rec[k] == r;
+                const unsigned ends = __ballot_sync(0xffffffffu, !mine || (a.lead_flags[k] & 1u));
+                const int stop = ends ? __ffs(ends) - 1 : 31;
+                if (mine && lane <= stop) {
+                    const float4 v = a.lead_v[k];
+                    const float2 w = a.lead_w[k];
+                    s.r.add(v.x, v.y);
+                    s.i.add(v.z, v.w);
+                    s.w.add(w.x, w.y);
+                }
+                if (ends) break;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const RecSum t = shfl_rec(s, lane ^ o);
+                s.add(t);
+            }
+            if (lane == 0) {
+                const float4 v = a.vsum[r];
+                const float2 w = a.wsum[r];
+                s.r.add(v.x, v.y);
+                s.i.add(v.z, v.w);
+                s.w.add(w.x, w.y);
+                a.vsum[r] = make_float4(s.r.h, s.r.l, s.i.h, s.i.l);
+                a.wsum[r] = make_float2(s.w.h, s.w.l);
+            }
+        }
+    for (int64_t t = t0; t <= a.ntiles; t += step) {
+        int64_t lo = 0, hi = nrec;   // first record whose tile is >= t
+        while (lo < hi) {
+            const int64_t m = (lo + hi) >> 1;
+            const int2 p = a.xy[m];
+            if ((int64_t)(p.x >> 5) * a.nty + (p.y >> 5) < t) lo = m + 1; else hi = m;
+        }
+        a.tile_start[t] = (uint32_t)lo;
     }
 }
 
@@ -674,7 +843,8 @@ void for_each_piece(cr_ctx* ctx, const DeviceBatch& b, F fn) {
     }
 }
 
-Records allocate_records(cr_ctx* ctx, int64_t n, int64_t ntx, int64_t nty, Pool* pool) {
+Records allocate_records(cr_ctx* ctx, int64_t n, int64_t ntx, int64_t nty, int use,
+                         Pool* pool) {
     Records r;
     size_t nn = (size_t)(n > 0 ? n : 1);
     r.n_samples = n;
@@ -682,79 +852,63 @@ Records allocate_records(cr_ctx* ctx, int64_t n, int64_t ntx, int64_t nty, Pool*
     r.nty = nty;
     Pool& P = pool ? *pool : ctx->ws;
     auto A = [&](const char* name, size_t bytes) { return pool_alloc(ctx, P, name, bytes); };
-    // keys and order are needed only while planning: always context workspaces
-    r.keys = (uint64_t*)workspace(ctx, "rec_keys", nn * 8);
-    r.order = (uint32_t*)workspace(ctx, "rec_order", nn * 4);
-    r.sample_rec = (int32_t*)A("rec_sample", nn * 4);
-    r.rec_x = (int32_t*)A("rec_x", nn * 4);
-    r.rec_y = (int32_t*)A("rec_y", nn * 4);
-    r.rec_a = (int32_t*)A("rec_a", nn * 4);
-    r.rec_b = (int32_t*)A("rec_b", nn * 4);
-    r.rec_conj = (int32_t*)A("rec_conj", nn * 4);
-    r.rec_vsum = (double2*)A("rec_vsum", nn * 16);
-    r.rec_wsum = (double*)A("rec_wsum", nn * 8);
+    if (use & kPlanSamples) r.sample_rec = (int32_t*)A("rec_sample", nn * 4);
+    r.rec_xy = (int2*)A("rec_xy", nn * 8);
+    r.rec_meta = (uint32_t*)A("rec_meta", nn * 4);
+    if (use & kPlanSums) {
+        r.rec_vsum = (float4*)A("rec_vsum", nn * 16);
+        r.rec_wsum = (float2*)A("rec_wsum", nn * 8);
+    }
     r.rec_pred = (float2*)A("rec_pred", nn * 8);
     r.tile_start = (uint32_t*)A("rec_tile_start", (size_t)(ntx * nty + 1) * 4);
-    r.counts = (unsigned long long*)A("rec_counts", 4 * 8);
-    r.sums = (double*)A("rec_sums", 2 * 8);
-    CR_CUDA_CHECK(cudaMemsetAsync(r.counts, 0, 4 * 8, ctx->stream));
-    CR_CUDA_CHECK(cudaMemsetAsync(r.sums, 0, 2 * 8, ctx->stream));
-    CR_CUDA_CHECK(cudaMemsetAsync(r.sample_rec, 0xFF, nn * 4, ctx->stream));
+    r.counts = (unsigned long long*)A("rec_counts", 4 * 8 + 2 * 8);
+    r.sums = (double*)(r.counts + 4);
+    CR_CUDA_CHECK(cudaMemsetAsync(r.counts, 0, 4 * 8 + 2 * 8, ctx->stream));
     return r;
 }
 
-void finish_records(cr_ctx* ctx, Records& r, int mode, int key_bits, int plane_bits,
+void finish_records(cr_ctx* ctx, Records& r, RadixSort& sort, int mode, int plane_bits,
                     int off_bits, const DeviceBatch& b, const int32_t* support) {
-    const int64_t n = r.n_samples;
-    const unsigned T = 256;
-    radix_sort_pairs(ctx, r.keys, r.order, n, key_bits);
-    size_t nn = (size_t)(n > 0 ? n : 1);
-    uint32_t* flags = (uint32_t*)workspace(ctx, "rec_flags", nn * 4);
-    uint32_t* excl = (uint32_t*)workspace(ctx, "rec_excl", nn * 4);
-    uint32_t* tile_of = (uint32_t*)workspace(ctx, "rec_tile_of", nn * 4);
+    const int64_t n = r.n_samples, ntiles = r.ntx * r.nty;
+    radix_sort_run(ctx, sort);
+    const size_t ranges = (size_t)((n + kRecRange - 1) / kRecRange + 1);
+    char* lead = (char*)workspace(ctx, "rec_lead", ranges * 32);
+    RecArgs a{sort.sorted_keys, sort.order, r.counts, n, mode, plane_bits, off_bits, r.nty,
+              ntiles, r.rec_xy, r.rec_meta, r.rec_vsum, r.rec_wsum, r.sample_rec, b.weight,
+              b.sumwt_factor, b.vis, support, r.tile_start, (float4*)lead,
+              (float2*)(lead + ranges * 16), (uint32_t*)(lead + ranges * 24),
+              (uint32_t*)(lead + ranges * 28), sort.rec_ticket, sort.rec_state, sort.fail,
+              ctx->status_d};
     if (n > 0) {
-        head_flags<<<grid_blocks(n, T), T, 0, ctx->stream>>>(r.keys, r.counts, n, flags);
-        note_launch(ctx, "head_flags");
+        records_kernel<<<(unsigned)((n + kRecTile - 1) / kRecTile), kRecThreads, 0,
+                         ctx->stream>>>(a);
+        note_launch(ctx, "records_kernel");
     }
-    exclusive_scan_u32(ctx, flags, excl, n, r.counts + 2);
-    RecArgs a{r.keys, r.order, flags, excl, r.counts, n, mode, plane_bits, off_bits, r.nty,
-              r.rec_x, r.rec_y, r.rec_a, r.rec_b, r.rec_conj, r.rec_vsum, r.rec_wsum,
-              r.sample_rec, b.weight, b.sumwt_factor, b.vis, tile_of, support};
-    if (n > 0) {
-        records_init<<<grid_blocks(n, T), T, 0, ctx->stream>>>(a);
-        note_launch(ctx, "records_init");
-        records_accumulate<<<grid_blocks(n, T), T, 0, ctx->stream>>>(a);
-        note_launch(ctx, "records_accumulate");
-    }
-    int64_t ntiles = r.ntx * r.nty;
-    fill_u32<<<grid_blocks(ntiles + 1, T), T, 0, ctx->stream>>>(r.tile_start, ntiles + 1,
-                                                                 r.counts + 2);
-    note_launch(ctx, "fill_u32");
-    if (n > 0) {
-        tile_starts<<<grid_blocks(n, T), T, 0, ctx->stream>>>(tile_of, r.counts, r.tile_start);
-        note_launch(ctx, "tile_starts");
-    }
+    const int64_t work = std::max<int64_t>((int64_t)ranges * 32, ntiles + 1);
+    records_finish<<<grid_blocks(work, kRecThreads), kRecThreads, 0, ctx->stream>>>(a);
+    note_launch(ctx, "records_finish");
 }
 
 }  // namespace
 
-Records plan_wproj(cr_ctx* ctx, cr_wproj* wp, const DeviceBatch& b, Pool* pool) {
+Records plan_wproj(cr_ctx* ctx, cr_wproj* wp, const DeviceBatch& b, int use, Pool* pool) {
     const cr_grid_info& gi = wp->g->info;
     int64_t ntx = (gi.grid_nx + kTile - 1) / kTile, nty = (gi.grid_ny + kTile - 1) / kTile;
-    Records r = allocate_records(ctx, b.n, ntx, nty, pool);
+    Records r = allocate_records(ctx, b.n, ntx, nty, use, pool);
     int tile_bits = bits_for((uint64_t)(ntx * nty));
     int plane_bits = bits_for((uint64_t)(wp->info.planes > 1 ? wp->info.planes - 1 : 1));
     int off_bits = bits_for((uint64_t)(wp->axis * wp->axis - 1));
     int key_bits = tile_bits + plane_bits + 1 + off_bits + 10;
     if (key_bits > 64) fail(CR_INVALID, "grid too large for the 64-bit sample key");
+    RadixSort sort = radix_sort_begin(ctx, b.n, key_bits);
+    const KeyOut out{sort.keys, sort.hist, sort.passes, r.sample_rec};
     if (b.n > 0) {
         WpPlanArgs a{0, b.n, b.u, b.v, b.w, b.weight, b.sumwt_factor, b.gridable, b.vis,
                      gi.grid_nx, gi.grid_ny, gi.du, gi.dv, wp->info.w_scale,
                      wp->info.sampling, wp->info.planes, wp->radius, wp->axis,
                      wp->support_d, wp->norm_d, nty, plane_bits, off_bits,
                      df_scale_of(1.0, gi.du, false), df_scale_of(1.0, gi.dv, false),
-                     df_scale_of(wp->info.w_scale, 1.0, true), r.keys,
-                     r.order, r.sums, r.counts};
+                     df_scale_of(wp->info.w_scale, 1.0, true), out, r.sums, r.counts};
         for_each_piece(ctx, b, [&](int64_t lo, int64_t hi) {
             a.first = lo;
             a.n = hi;
@@ -762,22 +916,24 @@ Records plan_wproj(cr_ctx* ctx, cr_wproj* wp, const DeviceBatch& b, Pool* pool) 
             note_launch(ctx, "wp_plan_kernel");
         });
     }
-    finish_records(ctx, r, 0, key_bits, plane_bits, off_bits, b, wp->support_d);
+    finish_records(ctx, r, sort, 0, plane_bits, off_bits, b, wp->support_d);
     return r;
 }
 
-Records plan_standard(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, Pool* pool) {
+Records plan_standard(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, int use, Pool* pool) {
     const cr_grid_info& gi = g->info;
     int64_t ntx = (gi.grid_nx + kTile - 1) / kTile, nty = (gi.grid_ny + kTile - 1) / kTile;
-    Records r = allocate_records(ctx, b.n, ntx, nty, pool);
+    Records r = allocate_records(ctx, b.n, ntx, nty, use, pool);
     int tile_bits = bits_for((uint64_t)(ntx * nty));
     int key_bits = tile_bits + 16 + 10;
     if (key_bits > 64) fail(CR_INVALID, "grid too large for the 64-bit sample key");
+    RadixSort sort = radix_sort_begin(ctx, b.n, key_bits);
+    const KeyOut out{sort.keys, sort.hist, sort.passes, r.sample_rec};
     if (b.n > 0) {
         StdPlanArgs a{0, b.n, b.u, b.v, b.weight, b.sumwt_factor, b.gridable, gi.grid_nx,
                       gi.grid_ny, gi.du, gi.dv, gi.oversampling, g->tap_rows, nty,
-                      df_scale_of(1.0, gi.du, false), df_scale_of(1.0, gi.dv, false), r.keys,
-                      r.order, r.sums, r.counts};
+                      df_scale_of(1.0, gi.du, false), df_scale_of(1.0, gi.dv, false), out,
+                      r.sums, r.counts};
         for_each_piece(ctx, b, [&](int64_t lo, int64_t hi) {
             a.first = lo;
             a.n = hi;
@@ -785,7 +941,7 @@ Records plan_standard(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, Pool* po
             note_launch(ctx, "std_plan_kernel");
         });
     }
-    finish_records(ctx, r, 1, key_bits, 0, 0, b, nullptr);
+    finish_records(ctx, r, sort, 1, 0, 0, b, nullptr);
     return r;
 }
 
@@ -795,9 +951,10 @@ void read_sums(cr_ctx* ctx, const Records& r, cr_sums* out) {
         unsigned long long c[4];
         double s[2];
     }* host = (decltype(host))ctx->pinned;
-    CR_CUDA_CHECK(cudaMemcpyAsync(host->c, r.counts, 32, cudaMemcpyDeviceToHost, ctx->stream));
-    CR_CUDA_CHECK(cudaMemcpyAsync(host->s, r.sums, 16, cudaMemcpyDeviceToHost, ctx->stream));
+    // the sums follow the counts
+    CR_CUDA_CHECK(cudaMemcpyAsync(host->c, r.counts, 48, cudaMemcpyDeviceToHost, ctx->stream));
     CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    check_device_status(ctx);
     out->gridded = (int64_t)host->c[0];
     out->skipped = (int64_t)host->c[1];
     out->unique_records = (int64_t)host->c[2];

@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "cr_fixed.cuh"
 #include "cr_internal.cuh"
 
 namespace cr {
@@ -221,33 +222,26 @@ inline bool band_pack_fits(int64_t gn, int planes, int radius, int smax) {
 }
 
 template <bool RESIDUAL>
-__global__ void band_pack_kernel(const int32_t* rx, const int32_t* ry, const int32_t* rplane,
-                                 const int32_t* roff, const int32_t* rconj, const double2* vsum,
-                                 const double* wsum, const float2* pred, const int32_t* support,
+__global__ void band_pack_kernel(const int2* xy, const uint32_t* rmeta, const float4* vsum,
+                                 const float2* wsum, const float2* pred, const int32_t* support,
                                  int32_t axis, const unsigned long long* counts, uint4* packed,
                                  float* weight) {
     const int64_t n = (int64_t)counts[2];
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
          r += (int64_t)gridDim.x * blockDim.x) {
-        const int plane = rplane[r];
-        const int off = roff[r];
-        const unsigned meta = (unsigned)plane | (unsigned)(off / axis) << 12 |
-                              (unsigned)(off % axis) << 18 | (unsigned)(rconj[r] ? 1 : 0) << 24 |
+        const int2 p = xy[r];
+        const uint32_t m = rmeta[r];
+        const unsigned plane = m & 0xfffu, conj = (m >> 12) & 1u, off = m >> 13;
+        const unsigned meta = plane | (off / (unsigned)axis) << 12 |
+                              (off % (unsigned)axis) << 18 | conj << 24 |
                               (unsigned)support[plane] << 25;
-        const double2 vs = vsum[r];
-        const double ws = wsum[r];
-        float vr, vi;
-        if (RESIDUAL) {
-            const float2 p = pred[r];
-            vr = (float)(vs.x - (double)p.x * ws);
-            vi = (float)(vs.y - (double)p.y * ws);
-        } else {
-            vr = (float)vs.x;
-            vi = (float)vs.y;
-        }
-        packed[r] = make_uint4((unsigned)rx[r] << 16 | (unsigned)ry[r], meta, __float_as_uint(vr),
-                               __float_as_uint(vi));
-        weight[r] = (float)ws;
+        const float4 vs = vsum[r];
+        const float2 ws = wsum[r];
+        float2 v = make_float2(vs.x, vs.z);
+        if (RESIDUAL) v = residual_value(vs, ws, pred[r]);
+        packed[r] = make_uint4((unsigned)p.x << 16 | (unsigned)p.y, meta, __float_as_uint(v.x),
+                               __float_as_uint(v.y));
+        weight[r] = ws.x;
     }
 }
 
@@ -439,7 +433,7 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3) wp_grid_kernel(BandArgs a)
 // reach the tile when supports grow with the plane index (records of a home
 // tile are sorted by plane); the work items are the tile's bands times the
 // chunks of kBandChunk candidates.
-__global__ void band_work_count(const uint32_t* tile_start, const int32_t* rplane,
+__global__ void band_work_count(const uint32_t* tile_start, const uint32_t* rmeta,
                                 const int32_t* first_plane, int32_t max_support, int monotone,
                                 int64_t ntx, int64_t nty, int R, int64_t gnx,
                                 uint32_t* seg_lo, uint32_t* seg_pre, uint8_t* nseg,
@@ -469,7 +463,7 @@ __global__ void band_work_count(const uint32_t* tile_start, const int32_t* rplan
                     uint32_t l = lo, u = hi;   // first record with plane >= p
                     while (l < u) {
                         const uint32_t m = l + ((u - l) >> 1);
-                        if (rplane[m] < p) l = m + 1; else u = m;
+                        if ((int)(rmeta[m] & 0xfffu) < p) l = m + 1; else u = m;
                     }
                     lo = l;
                     if (lo >= hi) continue;
@@ -510,7 +504,8 @@ __global__ void band_work_fill(const uint32_t* nitems, const uint32_t* first, in
 
 // ---- degridding --------------------------------------------------------------------
 struct DegridArgs {
-    const int32_t *rx, *ry, *rplane, *roff, *rconj;
+    const int2* xy;
+    const uint32_t* meta;
     const unsigned long long* counts;
     const int32_t* support;
     const int64_t* cube_off;
@@ -591,14 +586,16 @@ __global__ void __launch_bounds__(256, 4) wp_degrid_kernel(DegridArgs a) {
     const int gny = (int)a.gny;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrec;
          r += nwarps) {
-        const int plane = a.rplane[r];
+        const int2 p = a.xy[r];
+        const uint32_t meta = a.meta[r];
+        const int plane = (int)(meta & 0xfffu);
         const int s = a.support[plane];
         const int w = 2 * s + 1;
         const int q = a.cube_q[plane];
-        const int off = a.roff[r];
+        const int off = (int)(meta >> 13);
         const int ox = off / a.axis - a.radius, oy = off % a.axis - a.radius;
         const float2* cube = a.cube + a.cube_off[plane];
-        const float2* g = a.grid + (int64_t)(a.rx[r] - s) * a.gny + (a.ry[r] - s);
+        const float2* g = a.grid + (int64_t)(p.x - s) * a.gny + (p.y - s);
         // (A, C) = sum kx (gx, gy), (D, B) = sum ky (gx, gy)
         float2 AC = make_float2(0.f, 0.f), DB = make_float2(0.f, 0.f);
         switch ((w + 15) >> 4) {
@@ -628,7 +625,7 @@ __global__ void __launch_bounds__(256, 4) wp_degrid_kernel(DegridArgs a) {
             D += __shfl_xor_sync(0xffffffffu, D, o);
         }
         if (lane == 0)
-            a.pred[r] = a.rconj[r] ? make_float2(A - B, C + D) : make_float2(A + B, C - D);
+            a.pred[r] = (meta >> 12) & 1u ? make_float2(A - B, C + D) : make_float2(A + B, C - D);
     }
 }
 
@@ -913,7 +910,7 @@ static void wproj_grid_band(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2*
     uint32_t* first = (uint32_t*)workspace(ctx, "wb_first", (size_t)ntiles * 4);
     unsigned long long* total = (unsigned long long*)workspace(ctx, "wb_total", 16);
     band_work_count<<<grid_blocks(ntiles, 256), 256, 0, ctx->stream>>>(
-        r.tile_start, r.rec_a, wp->first_plane_d, wp->info.max_support,
+        r.tile_start, r.rec_meta, wp->first_plane_d, wp->info.max_support,
         wp->support_monotone ? 1 : 0, r.ntx, r.nty, R, gnx, seg_lo, seg_pre, nseg, nitems);
     note_launch(ctx, "band_work_count");
     exclusive_scan_u32(ctx, nitems, first, ntiles, total);
@@ -933,11 +930,11 @@ static void wproj_grid_band(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2*
     float* weight = (float*)workspace(ctx, "wb_weight", nrec * 4);
     if (mode == 0)
         band_pack_kernel<false><<<grid_blocks(r.n_samples, 256), 256, 0, ctx->stream>>>(
-            r.rec_x, r.rec_y, r.rec_a, r.rec_b, r.rec_conj, r.rec_vsum, r.rec_wsum, r.rec_pred,
+            r.rec_xy, r.rec_meta, r.rec_vsum, r.rec_wsum, r.rec_pred,
             wp->support_d, wp->axis, r.counts, packed, weight);
     else
         band_pack_kernel<true><<<grid_blocks(r.n_samples, 256), 256, 0, ctx->stream>>>(
-            r.rec_x, r.rec_y, r.rec_a, r.rec_b, r.rec_conj, r.rec_vsum, r.rec_wsum, r.rec_pred,
+            r.rec_xy, r.rec_meta, r.rec_vsum, r.rec_wsum, r.rec_pred,
             wp->support_d, wp->axis, r.counts, packed, weight);
     note_launch(ctx, "band_pack_kernel");
     BandArgs a{packed, weight, wp->cube_off_d, wp->cube_q_d, wp->cube_d, cube_geom(wp),
@@ -965,7 +962,7 @@ void wproj_grid(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2* psf, float2
 }
 
 void wproj_degrid(cr_ctx* ctx, cr_wproj* wp, const Records& r, const float2* grid) {
-    DegridArgs a{r.rec_x, r.rec_y, r.rec_a, r.rec_b, r.rec_conj, r.counts, wp->support_d,
+    DegridArgs a{r.rec_xy, r.rec_meta, r.counts, wp->support_d,
                  wp->cube_off_d, wp->cube_q_d, wp->cube_d, cube_geom(wp), wp->radius, wp->axis,
                  grid, wp->g->info.grid_ny, r.rec_pred};
     int blocks = sm_count(ctx) * 8;
