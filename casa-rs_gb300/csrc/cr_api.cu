@@ -101,7 +101,7 @@ void grid_records(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const Records& r, fl
     if (wp)
         wproj_grid(ctx, wp, r, psf, dirty, mode);
     else
-        std_grid(ctx, g, r, psf, dirty, mode);
+        std_grid(ctx, g, r, (float*)psf, 2, dirty, mode);
 }
 
 void degrid_records(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const Records& r,
@@ -691,9 +691,10 @@ int cr_image_to_grid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float* mode
 // dirty_grids_to_psf_and_residual_owned (lib.rs:48987-49130): PSF and dirty
 // grids with their sums -> normalised PSF and residual images and the PSF
 // state (synchronises).
-static void dirty_products(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* psf, float2* dirty,
-                           const cr_sums& s, float* psf_out, float* residual_out,
-                           int32_t out_location, cr_psf_state* state) {
+// The PSF grid is complex, or its real part alone (psf_real).
+static void dirty_products(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* psf,
+                           const float* psf_real, float2* dirty, const cr_sums& s, float* psf_out,
+                           float* residual_out, int32_t out_location, cr_psf_state* state) {
     if (s.normalization_sumwt <= 0.0 || s.reported_sumwt <= 0.0)
         fail(CR_NO_SAMPLES, "no usable samples");
     const float k = wp ? 2.0f : 1.0f;
@@ -702,24 +703,16 @@ static void dirty_products(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* psf
     float* psf_img = out_ptr<float>(ctx, psf_out, out_location, np * 4, "psf_image");
     float* res_img = out_ptr<float>(ctx, residual_out, out_location, np * 4, "res_image");
     unsigned int* peak_d = (unsigned int*)workspace(ctx, "di_peak", 4);
-    grid_to_image(ctx, g, wp, psf, k / sumwt_f, psf_img, image_single(ctx));
-    abs_peak(ctx, psf_img, (int64_t)np, peak_d);
+    dirty_pair_to_images(ctx, g, wp, psf, psf_real, dirty, k / sumwt_f, psf_img, res_img, peak_d,
+                         image_single(ctx));
     // the scaling reads the peak on the device; the host checks it once both
-    // images are done, so nothing waits in between
+    // images are done
     unsigned int* peak_h = (unsigned int*)((char*)ctx->pinned + 256);
     CR_CUDA_CHECK(cudaMemcpyAsync(peak_h, peak_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    scale_image(ctx, psf_img, (int64_t)np, 1.0f, peak_d);
-    AuxFork fork(ctx);
     if (out_location == CR_HOST) {
-        // the PSF image goes back while the residual is transformed
-        fork.to_aux();
         copy_out(ctx, psf_out, psf_img, np * 4, CR_HOST);
-        fork.to_main();
+        copy_out(ctx, residual_out, res_img, np * 4, CR_HOST);
     }
-    grid_to_image(ctx, g, wp, dirty, k / sumwt_f, res_img, image_single(ctx));
-    scale_image(ctx, res_img, (int64_t)np, 1.0f, peak_d);
-    if (out_location == CR_HOST) copy_out(ctx, residual_out, res_img, np * 4, CR_HOST);
-    fork.join();
     CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
     float peak;
     std::memcpy(&peak, peak_h, 4);
@@ -739,18 +732,24 @@ int cr_dirty_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_batch*
         tm.mark();
         StagedBatch b(ctx, batch, wp != nullptr);
         size_t gb = grid_bytes(g);
-        float2* psf = (float2*)workspace(ctx, "di_psf", gb);
+        // the standard gridder's PSF grid is real
+        const size_t pb = wp ? gb : gb / 2;
+        float2* psf = (float2*)workspace(ctx, "di_psf", pb);
         float2* dirty = (float2*)workspace(ctx, "di_dirty", gb);
-        CR_CUDA_CHECK(cudaMemsetAsync(psf, 0, gb, ctx->stream));
+        CR_CUDA_CHECK(cudaMemsetAsync(psf, 0, pb, ctx->stream));
         CR_CUDA_CHECK(cudaMemsetAsync(dirty, 0, gb, ctx->stream));
         Records r = plan(ctx, g, wp, b, kPlanSums);
         tm.mark();
-        grid_records(ctx, g, wp, r, psf, dirty, 0);
+        if (wp)
+            wproj_grid(ctx, wp, r, psf, dirty, 0);
+        else
+            std_grid(ctx, g, r, (float*)psf, 1, dirty, 0);
         tm.mark();
         cr_sums s{};
         read_sums(ctx, r, &s);
         if (sums) *sums = s;
-        dirty_products(ctx, g, wp, psf, dirty, s, psf_out, residual_out, out_location, state);
+        dirty_products(ctx, g, wp, wp ? psf : nullptr, wp ? nullptr : (const float*)psf, dirty, s,
+                       psf_out, residual_out, out_location, state);
         tm.mark();
         set_timings(ctx, cr_timings{tm.between(0, 1), tm.between(1, 2), 0.f, tm.between(2, 3), 0.f});
     });
@@ -777,8 +776,8 @@ int cr_residual_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const cr_vis_bat
         grid_records(ctx, g, wp, r, nullptr, res, 1);
         float* img = out_ptr<float>(ctx, residual_out, out_location, np * 4, "ri_image");
         const float k = wp ? 2.0f : 1.0f;
-        grid_to_image(ctx, g, wp, res, k / state->normalization_sumwt, img, image_single(ctx));
-        scale_image(ctx, img, (int64_t)np, 1.0f / state->psf_peak, nullptr);
+        grid_to_image(ctx, g, wp, res, k / state->normalization_sumwt, img, image_single(ctx),
+                      1.0f / state->psf_peak);
         if (out_location == CR_HOST) copy_out(ctx, residual_out, img, np * 4, CR_HOST);
         cr_sums s{};
         read_sums(ctx, r, &s);
@@ -965,8 +964,7 @@ int cr_plan_residual_image(cr_ctx* ctx, cr_plan* p, const float* model, int32_t 
         float* img = out_ptr<float>(ctx, residual_out, out_location, np * 4, "ri_image");
         const float k = p->wp ? 2.0f : 1.0f;
         grid_to_image(ctx, p->g, p->wp, res, k / state->normalization_sumwt, img,
-                      image_single(ctx));
-        scale_image(ctx, img, (int64_t)np, 1.0f / state->psf_peak, nullptr);
+                      image_single(ctx), 1.0f / state->psf_peak);
         tm.mark();
         if (out_location == CR_HOST) copy_out(ctx, residual_out, img, np * 4, CR_HOST);
         set_timings(ctx, cr_timings{0.f, tm.between(2, 3), tm.between(1, 2),
@@ -1761,7 +1759,7 @@ int cr_accumulator_finish(cr_ctx* ctx, cr_accumulator* a, float* psf, float* res
         if (total) *total = a->sums;
         StageTimer tm(ctx);
         tm.mark();
-        dirty_products(ctx, a->g, nullptr, a->psf, a->dirty, a->sums, psf, residual,
+        dirty_products(ctx, a->g, nullptr, a->psf, nullptr, a->dirty, a->sums, psf, residual,
                        out_location, state);
         tm.mark();
         set_timings(ctx, cr_timings{0.f, 0.f, 0.f, tm.between(0, 1), 0.f});

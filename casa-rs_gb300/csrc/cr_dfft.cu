@@ -12,19 +12,26 @@
 // multiply-add give each addition and multiplication with an error of about
 // 2^-44 of its operands, far below what the final float32 image keeps.
 //
-// One 2-D transform is two passes of 1-D transforms, one line per block, the
-// line held in shared memory: an in-place mixed-radix decimation-in-time
-// transform (radices 4, 2, 3, 5: the grids are even and 5-smooth, the
-// composite padding of gridder.rs:4152-4173) over an input loaded in
-// digit-reversed order, twiddles from a per-length table of
-// exp(2 pi i k / N) split into float pairs on the host.
-//   grid -> image: columns first (half of the grid's columns, only the
-//     image's rows kept), then the image's rows, two to a line, whose output
+// One 2-D transform is two passes of 1-D transforms, one line per block: a
+// mixed-radix decimation-in-time transform (radices 4, 2, 3, 5: the grids are
+// even and 5-smooth, the composite padding of gridder.rs:4152-4173) whose first
+// butterflies read global memory and whose last write it, with the line in
+// shared memory between them, and twiddles exp(2 pi i k / N) split into float
+// pairs on the host.
+//   grid -> image: half of the grid's rows (only the image's columns kept,
+//     stored transposed), then the image's columns, two to a line, whose output
 //     goes straight through the crop and correction of crop_correct_body;
-//   image -> grid: the image's rows first, two to a line (the apodised
-//     image is zero outside them), then half of the grid's columns, written
-//     with their mirror images as the float32 grid.
+//   image -> grid: the image's columns first, two to a line (the apodised
+//     image is zero outside them), then half of the grid's rows, written with
+//     their mirror images as the float32 grid.
+// So the grid, the largest array, is only read and written along its rows.
 // The centring is the checkerboard modulation of cr_fft.cu.
+//
+// 3600^2 grid, 3000^2 image: grid to image 417 -> 231 us; 2560^2 and
+// 2048^2: grid to image 219 -> 124 us, image to grid 219 -> 121 us
+// (against scalar, renormalised pair arithmetic with every stage through
+// shared memory, twiddles gathered from one table and the grid read and
+// written by columns: the load/store unit was the bound, not the arithmetic).
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -35,11 +42,13 @@ namespace cr {
 
 struct DfPlan {
     int32_t n = 0, ns = 0;
-    int32_t radix[16] = {};
-    int32_t* src = nullptr;   // [n] input index loaded at each position
-    float4* tw = nullptr;     // [n] exp(+2 pi i k / n) as (cos hi, cos lo, sin hi, sin lo)
+    int32_t radix[16] = {}, tw_at[16] = {};
+    int32_t* pos = nullptr;   // [n / radix[0]] where input p's butterfly goes
+    // per stage (from the second), [radix - 1][m]: exp(+2 pi i q j / (m radix))
+    // as (cos hi, sin hi, cos lo, sin lo), so that a warp reads rows
+    float4* tw = nullptr;
     ~DfPlan() {
-        cudaFree(src);
+        cudaFree(pos);
         cudaFree(tw);
     }
 };
@@ -53,7 +62,10 @@ constexpr int64_t kDfMaxN = 13824;
 
 struct DfStages {
     int32_t n, ns;
+    int32_t sa, sb;                 // the line's swizzle (at())
     int32_t radix[kDfMaxStages];
+    int32_t tw[kDfMaxStages];       // the stage's twiddles in the plan's table
+    uint32_t magic[kDfMaxStages];   // ceil(2^32 / m), m the stage's span: exact below 2^16
 };
 
 struct DfConsts {
@@ -62,171 +74,204 @@ struct DfConsts {
     float s3h, s3l;             // sin(2 pi / 3)
 };
 
+// A complex value as a float pair per part: h = (re, im) high parts, l the low
+// ones.  Both parts go through paired float32 instructions (FADD2, FMUL2,
+// FFMA2: two results per issue slot).  Sums are not renormalised: |l| stays
+// below a few ulps of the largest |h| that went into a value, so the pair
+// still holds about 2^-45 of it; the one rounding to float32 is at the end.
+struct cdd {
+    float2 h, l;
+};
 struct dd {
     float h, l;
 };
-struct cdd {
-    dd re, im;
-};
 
-// s + e = a + b exactly (Knuth); quick form when |a| >= |b| (Dekker)
-__device__ __forceinline__ dd two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    return {s, e};
+__device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
 }
-__device__ __forceinline__ dd quick_two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b);
-    return {s, __fsub_rn(b, __fsub_rn(s, a))};
+// s + e = a + b exactly (Knuth), the errors then summed with the low parts
+__device__ __forceinline__ cdd cadd(cdd a, cdd b) {
+    const float2 s = __fadd2_rn(a.h, b.h), v = sub2(s, a.h);
+    const float2 e = __fadd2_rn(sub2(a.h, sub2(s, v)), sub2(b.h, v));
+    return {s, __fadd2_rn(e, __fadd2_rn(a.l, b.l))};
 }
-__device__ __forceinline__ dd dadd(dd a, dd b) {
-    const dd s = two_sum(a.h, b.h);
-    return quick_two_sum(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+__device__ __forceinline__ cdd csub(cdd a, cdd b) {
+    const float2 s = sub2(a.h, b.h), v = sub2(s, a.h);
+    const float2 e = sub2(sub2(a.h, sub2(s, v)), __fadd2_rn(b.h, v));
+    return {s, __fadd2_rn(e, sub2(a.l, b.l))};
 }
-__device__ __forceinline__ dd dneg(dd a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ dd dsub(dd a, dd b) { return dadd(a, dneg(b)); }
-// the product's rounding error from one fused multiply-add (Dekker's product)
-__device__ __forceinline__ dd dmul(dd a, dd b) {
-    const float p = __fmul_rn(a.h, b.h);
-    float e = __fmaf_rn(a.h, b.h, -p);
-    e = __fmaf_rn(a.h, b.l, e);
-    e = __fmaf_rn(a.l, b.h, e);
-    return quick_two_sum(p, e);
+// times a real float pair: the high product's rounding error from one fused
+// multiply-add (Dekker's product), the cross terms added to it
+__device__ __forceinline__ cdd cscale(cdd a, dd c) {
+    const float2 ch = dup(c.h), p = __fmul2_rn(a.h, ch);
+    float2 e = __ffma2_rn(a.h, ch, make_float2(-p.x, -p.y));
+    e = __ffma2_rn(a.h, dup(c.l), e);
+    return {p, __ffma2_rn(a.l, ch, e)};
 }
-
-__device__ __forceinline__ cdd cadd(cdd a, cdd b) { return {dadd(a.re, b.re), dadd(a.im, b.im)}; }
-__device__ __forceinline__ cdd csub(cdd a, cdd b) { return {dsub(a.re, b.re), dsub(a.im, b.im)}; }
-// a b + sgn c d as one float pair: the two products' high parts are summed
-// exactly, their rounding errors and cross terms gathered by fused
-// multiply-adds into one correction
-__device__ __forceinline__ dd dot2(dd a, dd b, dd c, dd d, float sgn) {
-    const float p = __fmul_rn(a.h, b.h), q = sgn * __fmul_rn(c.h, d.h);
-    float t = __fmaf_rn(a.h, b.h, -p);
-    t = __fmaf_rn(a.h, b.l, t);
-    t = __fmaf_rn(a.l, b.h, t);
-    t = __fmaf_rn(sgn, __fmaf_rn(c.h, d.h, -sgn * q), t);
-    t = __fmaf_rn(sgn * c.h, d.l, t);
-    t = __fmaf_rn(sgn * c.l, d.h, t);
-    const dd s = two_sum(p, q);
-    return quick_two_sum(s.h, __fadd_rn(s.l, t));
+// a w with w = (wr, wi): (ar, ai) wr + (-ai, ar) wi, the two high products
+// summed exactly, their errors and cross terms gathered in the low part
+__device__ __forceinline__ cdd cmul(cdd a, float4 w) {
+    const float2 rh = dup(w.x), rl = dup(w.z), ih = make_float2(-w.y, w.y),
+                 il = make_float2(-w.w, w.w);
+    const float2 sh = make_float2(a.h.y, a.h.x), sl = make_float2(a.l.y, a.l.x);
+    const float2 p = __fmul2_rn(a.h, rh), q = __fmul2_rn(sh, ih);
+    float2 t = __ffma2_rn(a.h, rh, make_float2(-p.x, -p.y));
+    t = __ffma2_rn(a.h, rl, t);
+    t = __ffma2_rn(a.l, rh, t);
+    t = __fadd2_rn(t, __ffma2_rn(sh, ih, make_float2(-q.x, -q.y)));
+    t = __ffma2_rn(sh, il, t);
+    t = __ffma2_rn(sl, ih, t);
+    const float2 s = __fadd2_rn(p, q), v = sub2(s, p);
+    const float2 e = __fadd2_rn(sub2(p, sub2(s, v)), sub2(q, v));
+    return {s, __fadd2_rn(e, t)};
 }
-__device__ __forceinline__ cdd cmul(cdd a, cdd b) {
-    return {dot2(a.re, b.re, a.im, b.im, -1.0f), dot2(a.re, b.im, a.im, b.re, 1.0f)};
-}
-__device__ __forceinline__ cdd cscale(cdd a, dd c) { return {dmul(a.re, c), dmul(a.im, c)}; }
 // times +i for the inverse transform, -i for the forward one
 template <bool INV>
 __device__ __forceinline__ cdd mul_i(cdd a) {
-    return INV ? cdd{dneg(a.im), a.re} : cdd{a.im, dneg(a.re)};
+    return INV ? cdd{make_float2(-a.h.y, a.h.x), make_float2(-a.l.y, a.l.x)}
+               : cdd{make_float2(a.h.y, -a.h.x), make_float2(a.l.y, -a.l.x)};
 }
 
-__device__ __forceinline__ cdd ld(const float4* sm, int i) {
-    const float4 v = sm[i];
-    return {{v.x, v.y}, {v.z, v.w}};
+// in memory: (re hi, im hi, re lo, im lo)
+__device__ __forceinline__ cdd unpack(float4 v) {
+    return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
 }
-__device__ __forceinline__ void st(float4* sm, int i, cdd a) {
-    sm[i] = make_float4(a.re.h, a.re.l, a.im.h, a.im.l);
-}
+__device__ __forceinline__ float4 pack(cdd a) { return make_float4(a.h.x, a.h.y, a.l.x, a.l.y); }
+// A line in shared memory.  Position i lies at i with its low three bits (the
+// 16-byte bank group) exchanged by higher ones, so that the digit-reversed
+// stores of the first stage and the strided reads of the second spread over
+// the banks: counted over the stages, 1.9 wavefronts per ideal one without it,
+// 1.1-1.2 with the shifts of stages().
+struct Line {
+    float4* sm;
+    int sa, sb;
+    __device__ __forceinline__ int at(int i) const { return i ^ (((i >> sa) ^ (i >> sb)) & 7); }
+    __device__ __forceinline__ cdd ld(int i) const { return unpack(sm[at(i)]); }
+    __device__ __forceinline__ void st(int i, cdd a) const { sm[at(i)] = pack(a); }
+};
+// DFTs of 2 to 5 values in place, with the transform's sign.
 template <bool INV>
-__device__ __forceinline__ cdd twiddle(const float4* tw, int k) {
-    const float4 v = __ldg(tw + k);
-    return INV ? cdd{{v.x, v.y}, {v.z, v.w}} : cdd{{v.x, v.y}, {-v.z, -v.w}};
+__device__ __forceinline__ void dft(cdd (&x)[2], const DfConsts&) {
+    const cdd t = x[0];
+    x[0] = cadd(t, x[1]);
+    x[1] = csub(t, x[1]);
 }
 
-// Butterflies of stage span m at base: inputs base + q m, the q-th times
-// W^(q k) (k = j N / L), then a DFT of the radix with the transform's sign.
 template <bool INV>
-__device__ __forceinline__ void bfly2(float4* sm, int base, int m, int k, const float4* tw) {
-    const cdd x0 = ld(sm, base);
-    cdd x1 = ld(sm, base + m);
-    if (k) x1 = cmul(x1, twiddle<INV>(tw, k));
-    st(sm, base, cadd(x0, x1));
-    st(sm, base + m, csub(x0, x1));
-}
-
-template <bool INV>
-__device__ __forceinline__ void bfly3(float4* sm, int base, int m, int k, const float4* tw,
-                                      const DfConsts& c) {
-    const cdd x0 = ld(sm, base);
-    cdd x1 = ld(sm, base + m), x2 = ld(sm, base + 2 * m);
-    if (k) {
-        x1 = cmul(x1, twiddle<INV>(tw, k));
-        x2 = cmul(x2, twiddle<INV>(tw, 2 * k));
-    }
-    const cdd t1 = cadd(x1, x2), t2 = csub(x1, x2);
-    const cdd half{{0.5f * t1.re.h, 0.5f * t1.re.l}, {0.5f * t1.im.h, 0.5f * t1.im.l}};
-    const cdd a = csub(x0, half);
+__device__ __forceinline__ void dft(cdd (&x)[3], const DfConsts& c) {
+    const cdd t1 = cadd(x[1], x[2]), t2 = csub(x[1], x[2]);
+    const float2 half = make_float2(0.5f, 0.5f);
+    const cdd a = csub(x[0], cdd{__fmul2_rn(t1.h, half), __fmul2_rn(t1.l, half)});
     const cdd b = mul_i<INV>(cscale(t2, dd{c.s3h, c.s3l}));
-    st(sm, base, cadd(x0, t1));
-    st(sm, base + m, cadd(a, b));
-    st(sm, base + 2 * m, csub(a, b));
+    x[0] = cadd(x[0], t1);
+    x[1] = cadd(a, b);
+    x[2] = csub(a, b);
 }
 
 template <bool INV>
-__device__ __forceinline__ void bfly4(float4* sm, int base, int m, int k, const float4* tw) {
-    cdd x0 = ld(sm, base), x1 = ld(sm, base + m), x2 = ld(sm, base + 2 * m),
-        x3 = ld(sm, base + 3 * m);
-    if (k) {
-        x1 = cmul(x1, twiddle<INV>(tw, k));
-        x2 = cmul(x2, twiddle<INV>(tw, 2 * k));
-        x3 = cmul(x3, twiddle<INV>(tw, 3 * k));
-    }
-    const cdd t0 = cadd(x0, x2), t1 = csub(x0, x2), t2 = cadd(x1, x3);
-    const cdd t3 = mul_i<INV>(csub(x1, x3));
-    st(sm, base, cadd(t0, t2));
-    st(sm, base + m, cadd(t1, t3));
-    st(sm, base + 2 * m, csub(t0, t2));
-    st(sm, base + 3 * m, csub(t1, t3));
+__device__ __forceinline__ void dft(cdd (&x)[4], const DfConsts&) {
+    const cdd t0 = cadd(x[0], x[2]), t1 = csub(x[0], x[2]), t2 = cadd(x[1], x[3]);
+    const cdd t3 = mul_i<INV>(csub(x[1], x[3]));
+    x[0] = cadd(t0, t2);
+    x[1] = cadd(t1, t3);
+    x[2] = csub(t0, t2);
+    x[3] = csub(t1, t3);
 }
 
 template <bool INV>
-__device__ __forceinline__ void bfly5(float4* sm, int base, int m, int k, const float4* tw,
-                                      const DfConsts& c) {
-    const cdd x0 = ld(sm, base);
-    cdd x1 = ld(sm, base + m), x2 = ld(sm, base + 2 * m), x3 = ld(sm, base + 3 * m),
-        x4 = ld(sm, base + 4 * m);
-    if (k) {
-        x1 = cmul(x1, twiddle<INV>(tw, k));
-        x2 = cmul(x2, twiddle<INV>(tw, 2 * k));
-        x3 = cmul(x3, twiddle<INV>(tw, 3 * k));
-        x4 = cmul(x4, twiddle<INV>(tw, 4 * k));
-    }
+__device__ __forceinline__ void dft(cdd (&x)[5], const DfConsts& c) {
     const dd c1{c.c1h, c.c1l}, c2{c.c2h, c.c2l}, s1{c.s1h, c.s1l}, s2{c.s2h, c.s2l};
-    const cdd t1 = cadd(x1, x4), t2 = cadd(x2, x3), t3 = csub(x1, x4), t4 = csub(x2, x3);
-    const cdd a1 = cadd(x0, cadd(cscale(t1, c1), cscale(t2, c2)));
-    const cdd a2 = cadd(x0, cadd(cscale(t1, c2), cscale(t2, c1)));
+    const cdd t1 = cadd(x[1], x[4]), t2 = cadd(x[2], x[3]), t3 = csub(x[1], x[4]),
+              t4 = csub(x[2], x[3]);
+    const cdd a1 = cadd(x[0], cadd(cscale(t1, c1), cscale(t2, c2)));
+    const cdd a2 = cadd(x[0], cadd(cscale(t1, c2), cscale(t2, c1)));
     const cdd b1 = mul_i<INV>(cadd(cscale(t3, s1), cscale(t4, s2)));
     const cdd b2 = mul_i<INV>(csub(cscale(t3, s2), cscale(t4, s1)));
-    st(sm, base, cadd(x0, cadd(t1, t2)));
-    st(sm, base + m, cadd(a1, b1));
-    st(sm, base + 2 * m, cadd(a2, b2));
-    st(sm, base + 3 * m, csub(a2, b2));
-    st(sm, base + 4 * m, csub(a1, b1));
+    x[0] = cadd(x[0], cadd(t1, t2));
+    x[1] = cadd(a1, b1);
+    x[2] = cadd(a2, b2);
+    x[3] = csub(a2, b2);
+    x[4] = csub(a1, b1);
 }
 
-// The line in sm (loaded in digit-reversed order) to its transform, in place.
-template <bool INV>
-__device__ void line_transform(float4* sm, const DfStages& s, const float4* tw,
-                               const DfConsts& c) {
-    const int n = s.n;
-    int m = 1;
-    for (int k = 0; k < s.ns; ++k) {
-        const int r = s.radix[k], L = m * r, tstep = n / L, nb = n / r;
-        for (int beta = threadIdx.x; beta < nb; beta += blockDim.x) {
-            const int j = beta % m, base = (beta / m) * L + j, kk = j * tstep;
-            if (r == 4)
-                bfly4<INV>(sm, base, m, kk, tw);
-            else if (r == 5)
-                bfly5<INV>(sm, base, m, kk, tw, c);
-            else if (r == 2)
-                bfly2<INV>(sm, base, m, kk, tw);
-            else
-                bfly3<INV>(sm, base, m, kk, tw, c);
-        }
-        __syncthreads();
-        m = L;
+// The first stage: input p + q n / R for q < R, out to shared memory.
+template <bool INV, int R, typename Load>
+__device__ __forceinline__ void first_stage(const Line& line, const DfStages& s, const int32_t* pos,
+                                            const DfConsts& c, Load load) {
+    const int step = s.n / R;
+    for (int p = threadIdx.x; p < step; p += blockDim.x) {
+        cdd x[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[q] = load(p + q * step);
+        dft<INV>(x, c);
+        const int at = pos[p];
+#pragma unroll
+        for (int q = 0; q < R; ++q) line.st(at + q, x[q]);
     }
+}
+
+// A later stage of span m: values j + q m of group g, the q-th times its
+// twiddle, a DFT of the radix, then out(position, value).
+template <bool INV, int R, typename Out>
+__device__ __forceinline__ void stage(const Line& line, int n, int m, unsigned magic,
+                                      const float4* tw, const DfConsts& c, Out out) {
+    for (int b = threadIdx.x; b < n / R; b += blockDim.x) {
+        const int g = (int)__umulhi((unsigned)b, magic), j = b - g * m, at = g * (m * R) + j;
+        cdd x[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[q] = line.ld(at + q * m);
+#pragma unroll
+        for (int q = 1; q < R; ++q) {
+            const float4 w = __ldg(tw + (q - 1) * m + j);
+            x[q] = cmul(x[q], INV ? w : make_float4(w.x, -w.y, w.z, -w.w));
+        }
+        dft<INV>(x, c);
+#pragma unroll
+        for (int q = 0; q < R; ++q) out(at + q * m, x[q]);
+    }
+}
+
+template <bool INV, typename Out>
+__device__ __forceinline__ void any_stage(int r, const Line& line, int n, int m, unsigned magic,
+                                          const float4* tw, const DfConsts& c, Out out) {
+    if (r == 4)
+        stage<INV, 4>(line, n, m, magic, tw, c, out);
+    else if (r == 5)
+        stage<INV, 5>(line, n, m, magic, tw, c, out);
+    else if (r == 3)
+        stage<INV, 3>(line, n, m, magic, tw, c, out);
+    else
+        stage<INV, 2>(line, n, m, magic, tw, c, out);
+}
+
+// The transform of a line: load(index) gives its inputs, store(index, value)
+// takes its outputs.  With KEEP the outputs stay in shared memory (after a
+// barrier) and store is not called.
+template <bool INV, bool KEEP, typename Load, typename Store>
+__device__ __forceinline__ void line_transform(const Line& line, const DfStages& s, const int32_t* pos,
+                                               const float4* tw, const DfConsts& c, Load load,
+                                               Store store) {
+    if (s.radix[0] == 4)
+        first_stage<INV, 4>(line, s, pos, c, load);
+    else
+        first_stage<INV, 2>(line, s, pos, c, load);
+    __syncthreads();
+    int m = s.radix[0];
+    const int in_place = KEEP ? s.ns : s.ns - 1;
+    for (int k = 1; k < in_place; ++k) {
+        any_stage<INV>(s.radix[k], line, s.n, m, s.magic[k], tw + s.tw[k], c,
+                       [&](int i, const cdd& v) { line.st(i, v); });
+        __syncthreads();
+        m *= s.radix[k];
+    }
+    if (KEEP) return;
+    if (s.ns == 1) {
+        for (int i = threadIdx.x; i < s.n; i += blockDim.x) store(i, line.ld(i));
+        return;
+    }
+    any_stage<INV>(s.radix[s.ns - 1], line, s.n, m, s.magic[s.ns - 1], tw + s.tw[s.ns - 1], c,
+                   store);
 }
 
 // Only real images leave and enter these transforms, so each works on half
@@ -234,168 +279,202 @@ __device__ void line_transform(float4* sm, const DfStages& s, const float4* tw,
 // checkerboard's sign, and with g' the modulated grid:
 //   grid -> image: the real part of the inverse transform of g' is the
 //     inverse transform of its Hermitian part h(x, y) = (g'(x, y) +
-//     conj(g'(-x, -y))) / 2.  After the pass along x, column -y of h is the
-//     conjugate of column y, so only columns 0..gny/2 are transformed, and
-//     each image row is the real transform of a Hermitian line: two image
-//     rows r1, r2 go through one complex line as r1 + i r2.
-//   image -> grid: two real image rows go through one complex line as
-//     m1 + i m2 and are separated by the same symmetry (columns 0..gny/2
-//     kept); then columns 0..gny/2 are transformed along x and column -y
-//     written as the conjugate of column y.
+//     conj(g'(-x, -y))) / 2.  After the pass along y, row -x of h is the
+//     conjugate of row x, so only rows 0..gnx/2 are transformed, and each
+//     image column is the real transform of a Hermitian line: two image
+//     columns c1, c2 go through one complex line as c1 + i c2.
+//   image -> grid: two real image columns go through one complex line as
+//     m1 + i m2 and are separated by the same symmetry (rows 0..gnx/2
+//     kept); then rows 0..gnx/2 are transformed along y and row -x
+//     written as the conjugate of row x.
 // The halves h, (Z + conj(Z')) / 2 are float-pair operations; h itself is
 // exact (a two-sum halved).
 
-// grid -> image, pass 1: column y (0 <= y <= gny/2) of h transformed along
-// x; the image's rows [bx0, bx0 + nx) kept in t[(x - bx0) gnyh + y].
-__global__ void __launch_bounds__(kDfThreads, 2) dfft_inv_cols(
-    const float2* grid, const float* real_grid, int64_t gnx, int64_t gny, int64_t gnyh,
-    int64_t bx0, int32_t nx, const int32_t* src, const float4* tw, DfStages s, DfConsts c,
-    float4* t) {
-    extern __shared__ float4 sm[];
-    const int64_t y = blockIdx.x, ym = y ? gny - y : 0;
-    for (int i = threadIdx.x; i < s.n; i += blockDim.x) {
-        const int64_t x = src[i], xm = x ? gnx - x : 0;
-        float ar, ai = 0.0f, br, bi = 0.0f;
-        if (real_grid) {
-            ar = real_grid[x * gny + y];
-            br = real_grid[xm * gny + ym];
-        } else {
-            const float2 a = grid[x * gny + y], b = grid[xm * gny + ym];
-            ar = a.x;
-            ai = a.y;
-            br = b.x;
-            bi = b.y;
-        }
-        const dd re = two_sum(ar, br), im = two_sum(ai, -bi);
-        const float h = ((x + y) & 1) ? -0.5f : 0.5f;
-        sm[i] = make_float4(h * re.h, h * re.l, h * im.h, h * im.l);
-    }
-    __syncthreads();
-    line_transform<true>(sm, s, tw, c);
-    for (int xr = threadIdx.x; xr < nx; xr += blockDim.x) t[xr * gnyh + y] = sm[bx0 + xr];
-}
+// Up to two grids of one geometry in a launch (blockIdx.y).
+struct DfGrids {
+    const float2* grid[2];
+    const float* real_grid[2];   // real parts, where grid is null
+    float* image[2];
+    unsigned int* peak[2];       // max |image| (float bits), or null
+};
 
-// grid -> image, pass 2: image rows 2b and 2b + 1 as one Hermitian-extended
-// line r1 + i r2 transformed along y (the real part is row 2b, the imaginary
-// part row 2b + 1), then the crop and correction of crop_correct_body (the
-// same operations on the FP64 value).
+// grid -> image, pass 1: row x (0 <= x <= gnx/2) of h transformed along y; the
+// image's columns [by0, by0 + ny) kept in t[(y - by0) gnxh + x].
 __global__ void __launch_bounds__(kDfThreads, 2) dfft_inv_rows(
-    const float4* t, int64_t gny, int64_t gnyh, int32_t nx, int32_t ny, int64_t bx0,
-    int64_t by0, int parity, double scale, const float* corr_x, const float* corr_y,
-    const float* sx, const float* sy, int sinc_mode, const int32_t* src, const float4* tw,
-    DfStages s, DfConsts c, float* image) {
+    DfGrids im, int gnx, int gny, int gnxh, int by0, int ny, const int32_t* pos,
+    const float4* tw, DfStages s, DfConsts c, float4* t) {
     extern __shared__ float4 sm[];
-    const int64_t xr0 = 2 * (int64_t)blockIdx.x;
-    const bool two = xr0 + 1 < nx;
-    const float4* row1 = t + xr0 * gnyh;
-    const float4* row2 = row1 + gnyh;
-    for (int i = threadIdx.x; i < s.n; i += blockDim.x) {
-        const int64_t y = src[i];
-        const bool lower = y < gnyh;
-        const int64_t yy = lower ? y : gny - y;
-        const float4 a = row1[yy];
-        const float4 b = two ? row2[yy] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        // r1 + i r2 with r(-y) = conj(r(y)) for the upper half
-        const dd ar{a.x, a.y}, ai{a.z, a.w}, br{b.x, b.y}, bi{b.z, b.w};
-        const dd zr = lower ? dsub(ar, bi) : dadd(ar, bi);
-        const dd zi = lower ? dadd(ai, br) : dsub(br, ai);
-        sm[i] = make_float4(zr.h, zr.l, zi.h, zi.l);
-    }
-    __syncthreads();
-    line_transform<true>(sm, s, tw, c);
-    // the scale as a float pair: the product's high part is the float32
-    // value (float)(r * scale) of the FP64 path, but for ties at half an ulp
-    const float sh = (float)scale;
-    const dd sc{sh, (float)(scale - (double)sh)};
-    for (int k = threadIdx.x; k < (two ? 2 * ny : ny); k += blockDim.x) {
-        const int q = k >= ny;
-        const int64_t yr = k - q * ny, gy = by0 + yr, xr = xr0 + q, gx = bx0 + xr;
-        const float4 w = sm[gy];
-        dd r = q ? dd{w.z, w.w} : dd{w.x, w.y};
-        if ((gx + gy + parity) & 1) r = dneg(r);
-        float v = dmul(r, sc).h;
-        const float factor = __fmul_rn(corr_x[gx], corr_y[gy]);
-        if (sinc_mode == 1) {
-            const float sf = __fmul_rn(sx[gx], sy[gy]);
-            v = fabsf(sf) > 1.0e-6f ? v * (factor / sf) : 0.0f;
-        } else if (sinc_mode == 2) {
-            v = v * __fmul_rn(__fmul_rn(factor, sx[gx]), sy[gy]);
-        } else {
-            v = v * factor;
-        }
-        image[xr * ny + yr] = v;
-    }
+    const Line line{sm, s.sa, s.sb};
+    const int x = blockIdx.x, xm = x ? gnx - x : 0, k = blockIdx.y;
+    const float2* grid = k ? im.grid[1] : im.grid[0];
+    const float* real_grid = k ? im.real_grid[1] : im.real_grid[0];
+    const float2* ga = grid + (int64_t)x * gny;
+    const float2* gb = grid + (int64_t)xm * gny;
+    const float* ra = real_grid + (int64_t)x * gny;
+    const float* rb = real_grid + (int64_t)xm * gny;
+    const bool real = grid == nullptr;
+    t += (int64_t)k * ny * gnxh + x;
+    line_transform<true, false>(
+        line, s, pos, tw, c,
+        [&](int y) {
+            const int ym = y ? gny - y : 0;
+            const float2 a = real ? make_float2(ra[y], 0.0f) : ga[y];
+            const float2 b = real ? make_float2(rb[ym], 0.0f) : gb[ym];
+            const float2 half = dup(((x + y) & 1) ? -0.5f : 0.5f), zero = dup(0.0f);
+            const cdd z = cadd(cdd{a, zero}, cdd{make_float2(b.x, -b.y), zero});
+            return cdd{__fmul2_rn(z.h, half), __fmul2_rn(z.l, half)};
+        },
+        [&](int y, const cdd& v) {
+            const int yr = y - by0;
+            if (yr >= 0 && yr < ny) t[(int64_t)yr * gnxh] = pack(v);
+        });
 }
 
-// image -> grid, pass 1: rows 2b and 2b + 1 of the apodised, modulated model
-// (zero outside the image's columns) as one line m1 + i m2 transformed along
-// y, separated into each row's half spectrum t[xr gnyh + y], y <= gny/2.
-__global__ void __launch_bounds__(kDfThreads, 2) dfft_fwd_rows(
-    const float* model, int32_t nx, int32_t ny, int64_t gny, int64_t gnyh, int64_t bx0,
-    int64_t by0, const float* corr_x, const float* corr_y, const float* sinc_x,
-    const float* sinc_y, const int32_t* src, const float4* tw, DfStages s, DfConsts c,
-    float4* t) {
+// grid -> image, pass 2: image columns 2b and 2b + 1 as one
+// Hermitian-extended line c1 + i c2 transformed along x (the real part is
+// column 2b, the imaginary part column 2b + 1), then the crop and correction
+// of crop_correct_body (the same operations on the FP64 value), `post` (a
+// second float32 factor, 1 for none) and the peak.
+__global__ void __launch_bounds__(kDfThreads, 2) dfft_inv_cols(
+    DfGrids im, const float4* t, int gnx, int gnxh, int nx, int ny, int bx0, int by0, int parity,
+    float sh, float sl, float post, const float* corr_x, const float* corr_y, const float* sx,
+    const float* sy, int sinc_mode, const int32_t* pos, const float4* tw, DfStages s, DfConsts c) {
     extern __shared__ float4 sm[];
-    const int64_t xr0 = 2 * (int64_t)blockIdx.x, gx0 = bx0 + xr0;
-    const bool two = xr0 + 1 < nx;
-    for (int i = threadIdx.x; i < s.n; i += blockDim.x) {
-        const int64_t gy = src[i];
-        float v[2] = {0.0f, 0.0f};
-        if (gy >= by0 && gy < by0 + ny) {
-            for (int q = 0; q < (two ? 2 : 1); ++q) {
-                const int64_t gx = gx0 + q;
-                // apodize_body's operations
-                float f = __fmul_rn(corr_x[gx], corr_y[gy]);
-                if (sinc_x) f = __fmul_rn(__fmul_rn(f, sinc_x[gx]), sinc_y[gy]);
-                float u = model[(xr0 + q) * ny + (gy - by0)] * f;
-                if ((gx + gy) & 1) u = -u;
-                v[q] = u;
+    const Line line{sm, s.sa, s.sb};
+    const int y0 = 2 * blockIdx.x, k = blockIdx.y;
+    const bool two = y0 + 1 < ny;
+    const float4* col1 = t + ((int64_t)k * ny + y0) * gnxh;
+    const float4* col2 = col1 + gnxh;
+    float* image = (k ? im.image[1] : im.image[0]) + y0;
+    unsigned int* peak = k ? im.peak[1] : im.peak[0];
+    float cy[2], sfy[2] = {1.0f, 1.0f};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int gy = by0 + y0 + (q && two);
+        cy[q] = corr_y[gy];
+        if (sinc_mode) sfy[q] = sy[gy];
+    }
+    float top = 0.0f;
+    line_transform<true, false>(
+        line, s, pos, tw, c,
+        [&](int x) {
+            const bool lower = x < gnxh;
+            const int xx = lower ? x : gnx - x;
+            const float4 a = col1[xx];
+            const float4 b = two ? col2[xx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // c1 + i c2 with c(-x) = conj(c(x)) for the upper half
+            const float sg = lower ? 1.0f : -1.0f;
+            const cdd z1{make_float2(a.x, sg * a.y), make_float2(a.z, sg * a.w)};
+            const cdd z2{make_float2(-sg * b.y, b.x), make_float2(-sg * b.w, b.z)};
+            return cadd(z1, z2);
+        },
+        [&](int gx, const cdd& w) {
+            const int xr = gx - bx0;
+            if (xr < 0 || xr >= nx) return;
+            const float cx = corr_x[gx], sfx = sinc_mode ? sx[gx] : 1.0f;
+            float v[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float flip = ((gx + by0 + y0 + q + parity) & 1) ? -1.0f : 1.0f;
+                const float rh = flip * (q ? w.h.y : w.h.x), rl = flip * (q ? w.l.y : w.l.x);
+                const float ph = __fmul_rn(rh, sh);
+                float u = __fadd_rn(
+                    ph, __fmaf_rn(rl, sh, __fmaf_rn(rh, sl, __fmaf_rn(rh, sh, -ph))));
+                const float factor = __fmul_rn(cx, cy[q]);
+                if (sinc_mode == 1) {
+                    const float sf = __fmul_rn(sfx, sfy[q]);
+                    u = fabsf(sf) > 1.0e-6f ? u * (factor / sf) : 0.0f;
+                } else if (sinc_mode == 2) {
+                    u = u * __fmul_rn(__fmul_rn(factor, sfx), sfy[q]);
+                } else {
+                    u = u * factor;
+                }
+                v[q] = __fmul_rn(u, post);
             }
-        }
-        sm[i] = make_float4(v[0], 0.0f, v[1], 0.0f);
-    }
-    __syncthreads();
-    line_transform<false>(sm, s, tw, c);
-    float4* row1 = t + xr0 * gnyh;
-    for (int k = threadIdx.x; k < (two ? 2 * gnyh : gnyh); k += blockDim.x) {
-        const int q = k >= gnyh;
-        const int64_t y = k - q * gnyh;
-        const float4 a = sm[y], b = sm[y ? gny - y : 0];
-        const dd ar{a.x, a.y}, ai{a.z, a.w}, br{b.x, b.y}, bi{b.z, b.w};
-        // row 1: (Z(y) + conj(Z(-y))) / 2; row 2: (Z(y) - conj(Z(-y))) / 2i
-        const dd re = q ? dadd(ai, bi) : dadd(ar, br);
-        const dd im = q ? dsub(br, ar) : dsub(ai, bi);
-        row1[q * gnyh + y] = make_float4(0.5f * re.h, 0.5f * re.l, 0.5f * im.h, 0.5f * im.l);
+            image[(int64_t)xr * ny] = v[0];
+            top = fmaxf(top, fabsf(v[0]));   // NaN never raises the peak
+            if (two) {
+                image[(int64_t)xr * ny + 1] = v[1];
+                top = fmaxf(top, fabsf(v[1]));
+            }
+        });
+    if (peak) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(peak, m);
     }
 }
 
-// image -> grid, pass 2: column y (0 <= y <= gny/2) transformed along x
-// (rows outside [bx0, bx0 + nx) are zero), the output checkerboard, float32
-// grid; column -y written as the conjugate of column y at -x.
+// image -> grid, pass 1: columns 2b and 2b + 1 of the apodised, modulated
+// model (zero outside the image's rows) as one line m1 + i m2 transformed
+// along x, separated into each column's half spectrum t[x pitch + y], x <=
+// gnx/2.
 __global__ void __launch_bounds__(kDfThreads, 2) dfft_fwd_cols(
-    const float4* t, int64_t gny, int64_t gnyh, int32_t nx, int64_t bx0, int parity,
-    const int32_t* src, const float4* tw, DfStages s, DfConsts c, float2* grid) {
+    const float* model, int nx, int ny, int gnx, int gnxh, int bx0, int by0, int pitch,
+    const float* corr_x, const float* corr_y, const float* sinc_x, const float* sinc_y,
+    const int32_t* pos, const float4* tw, DfStages s, DfConsts c, float4* t) {
     extern __shared__ float4 sm[];
-    const int64_t y = blockIdx.x;
-    for (int i = threadIdx.x; i < s.n; i += blockDim.x) {
-        const int64_t x = src[i];
-        sm[i] = (x >= bx0 && x < bx0 + nx) ? t[(x - bx0) * gnyh + y]
-                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    __syncthreads();
-    line_transform<false>(sm, s, tw, c);
-    const bool mirror = y != 0 && y != gnyh - 1;
-    for (int x = threadIdx.x; x < s.n; x += blockDim.x) {
-        const float4 w = sm[x];
-        // the pairs are normalised: the high part is the float32 value
-        float re = w.x, im = w.z;
-        if ((x + y + parity) & 1) {
-            re = -re;
-            im = -im;
+    const Line line{sm, s.sa, s.sb};
+    const int y0 = 2 * blockIdx.x, gy0 = by0 + y0;
+    const bool two = y0 + 1 < ny;
+    line_transform<false, true>(
+        line, s, pos, tw, c,
+        [&](int gx) {
+            float v[2] = {0.0f, 0.0f};
+            if (gx >= bx0 && gx < bx0 + nx) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (q && !two) break;
+                    const int gy = gy0 + q;
+                    // apodize_body's operations
+                    float f = __fmul_rn(corr_x[gx], corr_y[gy]);
+                    if (sinc_x) f = __fmul_rn(__fmul_rn(f, sinc_x[gx]), sinc_y[gy]);
+                    const float u = model[(int64_t)(gx - bx0) * ny + y0 + q] * f;
+                    v[q] = ((gx + gy) & 1) ? -u : u;
+                }
+            }
+            return cdd{make_float2(v[0], v[1]), make_float2(0.0f, 0.0f)};
+        },
+        [](int, const cdd&) {});
+    for (int x = threadIdx.x; x < gnxh; x += blockDim.x) {
+        const cdd a = line.ld(x), b = line.ld(x ? gnx - x : 0);
+        const float2 half = dup(0.5f);
+        // column 1: (Z(x) + conj(Z(-x))) / 2; column 2: (Z(x) - conj(Z(-x))) / 2i
+        const cdd z1 = cadd(a, cdd{make_float2(b.h.x, -b.h.y), make_float2(b.l.x, -b.l.y)});
+        float4* out = t + (int64_t)x * pitch + y0;
+        out[0] = pack(cdd{__fmul2_rn(z1.h, half), __fmul2_rn(z1.l, half)});
+        if (two) {
+            const cdd z2 = cadd(cdd{make_float2(a.h.y, -a.h.x), make_float2(a.l.y, -a.l.x)},
+                                cdd{make_float2(b.h.y, b.h.x), make_float2(b.l.y, b.l.x)});
+            out[1] = pack(cdd{__fmul2_rn(z2.h, half), __fmul2_rn(z2.l, half)});
         }
-        grid[(int64_t)x * gny + y] = make_float2(re, im);
-        if (mirror) grid[(int64_t)(x ? s.n - x : 0) * gny + (gny - y)] = make_float2(re, -im);
     }
+}
+
+// image -> grid, pass 2: row x (0 <= x <= gnx/2) transformed along y
+// (columns outside [by0, by0 + ny) are zero), the output checkerboard, float32
+// grid; row -x written as the conjugate of row x at -y.
+__global__ void __launch_bounds__(kDfThreads, 2) dfft_fwd_rows(
+    const float4* t, int gnx, int gny, int gnxh, int ny, int by0, int pitch, int parity,
+    const int32_t* pos, const float4* tw, DfStages s, DfConsts c, float2* grid) {
+    extern __shared__ float4 sm[];
+    const Line line{sm, s.sa, s.sb};
+    const int x = blockIdx.x;
+    const float4* row = t + (int64_t)x * pitch;
+    const bool mirror = x != 0 && x != gnxh - 1;
+    float2* out = grid + (int64_t)x * gny;
+    float2* out_m = grid + (int64_t)(gnx - x) * gny;
+    line_transform<false, false>(
+        line, s, pos, tw, c,
+        [&](int y) {
+            const int yr = y - by0;
+            return unpack(yr >= 0 && yr < ny ? row[yr] : make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+        },
+        [&](int y, const cdd& w) {
+            float2 v = __fadd2_rn(w.h, w.l);
+            if ((x + y + parity) & 1) v = make_float2(-v.x, -v.y);
+            out[y] = v;
+            if (mirror) out_m[y ? gny - y : 0] = make_float2(v.x, -v.y);
+        });
 }
 
 void split(double v, float* h, float* l) {
@@ -440,8 +519,11 @@ const DfPlan& plan_for(cr_ctx* ctx, int64_t n) {
     p->ns = (int32_t)r.size();
     for (size_t k = 0; k < r.size(); ++k) p->radix[k] = r[k];
     // position i = q0 + r0 (q1 + r1 (q2 + ...)) holds input sum_s q_s n / L_s
-    std::vector<int32_t> src((size_t)n);
-    for (int64_t i = 0; i < n; ++i) {
+    // (L_s the product of the radices up to s); those with q0 = 0 are the
+    // first stage's butterflies
+    const int64_t r0 = r[0];
+    std::vector<int32_t> pos((size_t)(n / r0));
+    for (int64_t i = 0; i < n; i += r0) {
         int64_t rem = i, L = 1, v = 0;
         for (int32_t rs : r) {
             const int64_t q = rem % rs;
@@ -449,21 +531,29 @@ const DfPlan& plan_for(cr_ctx* ctx, int64_t n) {
             L *= rs;
             v += q * (n / L);
         }
-        src[(size_t)i] = (int32_t)v;
+        pos[(size_t)v] = (int32_t)i;
     }
-    std::vector<float4> tw((size_t)n);
+    std::vector<float4> tw;
     const double pi = 3.14159265358979323846;
-    for (int64_t k = 0; k < n; ++k) {
-        const double a = 2.0 * pi * (double)k / (double)n;
-        float4 w;
-        split(std::cos(a), &w.x, &w.y);
-        split(std::sin(a), &w.z, &w.w);
-        tw[(size_t)k] = w;
+    int64_t m = r0;
+    for (size_t k = 1; k < r.size(); ++k) {
+        p->tw_at[k] = (int32_t)tw.size();
+        const int64_t L = m * r[k];
+        for (int64_t q = 1; q < r[k]; ++q)
+            for (int64_t j = 0; j < m; ++j) {
+                const double a = 2.0 * pi * (double)(q * j) / (double)L;
+                float4 w;
+                split(std::cos(a), &w.x, &w.z);
+                split(std::sin(a), &w.y, &w.w);
+                tw.push_back(w);
+            }
+        m = L;
     }
-    CR_CUDA_CHECK(cudaMalloc((void**)&p->src, (size_t)n * 4));
-    CR_CUDA_CHECK(cudaMalloc((void**)&p->tw, (size_t)n * 16));
-    CR_CUDA_CHECK(cudaMemcpy(p->src, src.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
-    CR_CUDA_CHECK(cudaMemcpy(p->tw, tw.data(), (size_t)n * 16, cudaMemcpyHostToDevice));
+    if (tw.empty()) tw.push_back(make_float4(1.0f, 0.0f, 0.0f, 0.0f));
+    CR_CUDA_CHECK(cudaMalloc((void**)&p->pos, pos.size() * 4));
+    CR_CUDA_CHECK(cudaMalloc((void**)&p->tw, tw.size() * 16));
+    CR_CUDA_CHECK(cudaMemcpy(p->pos, pos.data(), pos.size() * 4, cudaMemcpyHostToDevice));
+    CR_CUDA_CHECK(cudaMemcpy(p->tw, tw.data(), tw.size() * 16, cudaMemcpyHostToDevice));
     ctx->df_plans[n] = p;
     return *p;
 }
@@ -472,7 +562,18 @@ DfStages stages(const DfPlan& p) {
     DfStages s{};
     s.n = p.n;
     s.ns = p.ns;
-    for (int k = 0; k < p.ns; ++k) s.radix[k] = p.radix[k];
+    // shifts with the fewest conflicts by the power of two in n (31: none)
+    int e2 = 0;
+    while (((p.n >> e2) & 1) == 0) ++e2;
+    s.sa = e2 >= 3 ? 2 : e2 == 2 ? 8 : 31;
+    s.sb = e2 >= 4 ? (p.n >= 1024 ? 8 : 6) : e2 == 3 ? 3 : 31;
+    int64_t m = 1;
+    for (int k = 0; k < p.ns; ++k) {
+        s.radix[k] = p.radix[k];
+        s.tw[k] = p.tw_at[k];
+        s.magic[k] = m > 1 ? (uint32_t)(((1ull << 32) + m - 1) / m) : 0u;
+        m *= p.radix[k];
+    }
     return s;
 }
 
@@ -490,47 +591,71 @@ bool dfft_supported(int64_t gnx, int64_t gny) {
     return true;
 }
 
-void dfft_grid_to_image(cr_ctx* ctx, cr_gridder* g, const float2* grid, const float* real_grid,
-                        double scale, const float* sx, const float* sy, int sinc_mode,
-                        float* image) {
-    const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny, gnyh = gny / 2 + 1;
-    const int32_t nx = g->geom.nx, ny = g->geom.ny;
+// Threads of a line's block: the radix-4 butterflies of one stage in equal
+// rounds of at most kDfThreads.
+static unsigned line_threads(int64_t n) {
+    const int64_t nb = (n + 3) / 4, rounds = (nb + kDfThreads - 1) / kDfThreads;
+    return (unsigned)(((nb + rounds - 1) / rounds + 31) / 32 * 32);
+}
+
+// whole groups of eight points, which the swizzle permutes
+static size_t line_bytes(int64_t n) { return (size_t)((n + 7) / 8 * 8) * 16; }
+
+void dfft_grids_to_images(cr_ctx* ctx, cr_gridder* g, int count, const float2* const* grids,
+                          const float* const* real_grids, double scale, float post,
+                          const float* sx, const float* sy, int sinc_mode, float* const* images,
+                          unsigned int* const* peaks) {
+    const int gnx = (int)g->info.grid_nx, gny = (int)g->info.grid_ny, gnxh = gnx / 2 + 1;
+    const int nx = g->geom.nx, ny = g->geom.ny;
     const DfPlan& px = plan_for(ctx, gnx);
     const DfPlan& py = plan_for(ctx, gny);
     const DfConsts c = consts();
-    float4* t = (float4*)workspace(ctx, "dfft_t", (size_t)nx * gnyh * 16);
-    const size_t smx = (size_t)gnx * 16, smy = (size_t)gny * 16;
-    allow_smem(dfft_inv_cols, smx);
+    float4* t = (float4*)workspace(ctx, "dfft_t", (size_t)count * ny * gnxh * 16);
+    const size_t smx = line_bytes(gnx), smy = line_bytes(gny);
     allow_smem(dfft_inv_rows, smy);
-    dfft_inv_cols<<<(unsigned)gnyh, kDfThreads, smx, ctx->stream>>>(
-        grid, real_grid, gnx, gny, gnyh, g->info.blc_x, nx, px.src, px.tw, stages(px), c, t);
-    note_launch(ctx, "dfft_inv_cols");
-    const int parity = (int)(((gnx / 2) + (gny / 2)) & 1);
-    dfft_inv_rows<<<(unsigned)((nx + 1) / 2), kDfThreads, smy, ctx->stream>>>(
-        t, gny, gnyh, nx, ny, g->info.blc_x, g->info.blc_y, parity, scale, g->corr_x_d,
-        g->corr_y_d, sx, sy, sinc_mode, py.src, py.tw, stages(py), c, image);
+    allow_smem(dfft_inv_cols, smx);
+    DfGrids im{};
+    for (int k = 0; k < count; ++k) {
+        im.grid[k] = grids[k];
+        im.real_grid[k] = real_grids[k];
+        im.image[k] = images[k];
+        im.peak[k] = peaks ? peaks[k] : nullptr;
+    }
+    dfft_inv_rows<<<dim3(gnxh, count), line_threads(gny), smy, ctx->stream>>>(
+        im, gnx, gny, gnxh, (int)g->info.blc_y, ny, py.pos, py.tw, stages(py), c, t);
     note_launch(ctx, "dfft_inv_rows");
+    const int parity = ((gnx / 2) + (gny / 2)) & 1;
+    // the scale as a float pair: the product's high part is the float32
+    // value (float)(r * scale) of the FP64 path, but for ties at half an ulp
+    float sh, sl;
+    split(scale, &sh, &sl);
+    dfft_inv_cols<<<dim3((ny + 1) / 2, count), line_threads(gnx), smx, ctx->stream>>>(
+        im, t, gnx, gnxh, nx, ny, (int)g->info.blc_x, (int)g->info.blc_y, parity, sh, sl, post,
+        g->corr_x_d, g->corr_y_d, sx, sy, sinc_mode, px.pos, px.tw, stages(px), c);
+    note_launch(ctx, "dfft_inv_cols");
 }
 
 void dfft_image_to_grid(cr_ctx* ctx, cr_gridder* g, const float* model, const float* sinc_x,
                         const float* sinc_y, float2* grid) {
-    const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny, gnyh = gny / 2 + 1;
-    const int32_t nx = g->geom.nx, ny = g->geom.ny;
+    const int gnx = (int)g->info.grid_nx, gny = (int)g->info.grid_ny, gnxh = gnx / 2 + 1;
+    const int nx = g->geom.nx, ny = g->geom.ny;
+    const int pitch = ny + (ny & 1);   // two columns in one 32-byte sector
     const DfPlan& px = plan_for(ctx, gnx);
     const DfPlan& py = plan_for(ctx, gny);
     const DfConsts c = consts();
-    float4* t = (float4*)workspace(ctx, "dfft_t", (size_t)nx * gnyh * 16);
-    const size_t smx = (size_t)gnx * 16, smy = (size_t)gny * 16;
-    allow_smem(dfft_fwd_rows, smy);
+    float4* t = (float4*)workspace(ctx, "dfft_t", (size_t)pitch * gnxh * 16);
+    const size_t smx = line_bytes(gnx), smy = line_bytes(gny);
     allow_smem(dfft_fwd_cols, smx);
-    dfft_fwd_rows<<<(unsigned)((nx + 1) / 2), kDfThreads, smy, ctx->stream>>>(
-        model, nx, ny, gny, gnyh, g->info.blc_x, g->info.blc_y, g->corr_x_d, g->corr_y_d,
-        sinc_x, sinc_y, py.src, py.tw, stages(py), c, t);
-    note_launch(ctx, "dfft_fwd_rows");
-    const int parity = (int)(((gnx / 2) + (gny / 2)) & 1);
-    dfft_fwd_cols<<<(unsigned)gnyh, kDfThreads, smx, ctx->stream>>>(
-        t, gny, gnyh, nx, g->info.blc_x, parity, px.src, px.tw, stages(px), c, grid);
+    allow_smem(dfft_fwd_rows, smy);
+    dfft_fwd_cols<<<(unsigned)((ny + 1) / 2), line_threads(gnx), smx, ctx->stream>>>(
+        model, nx, ny, gnx, gnxh, (int)g->info.blc_x, (int)g->info.blc_y, pitch, g->corr_x_d,
+        g->corr_y_d, sinc_x, sinc_y, px.pos, px.tw, stages(px), c, t);
     note_launch(ctx, "dfft_fwd_cols");
+    const int parity = ((gnx / 2) + (gny / 2)) & 1;
+    dfft_fwd_rows<<<(unsigned)gnxh, line_threads(gny), smy, ctx->stream>>>(
+        t, gnx, gny, gnxh, ny, (int)g->info.blc_y, pitch, parity, py.pos, py.tw, stages(py), c,
+        grid);
+    note_launch(ctx, "dfft_fwd_rows");
 }
 
 }  // namespace cr

@@ -195,6 +195,21 @@ __global__ void scale_image_kernel(float* img, int64_t n, float scale, const uns
     }
 }
 
+// Both images of a pair divided by the peak (scale_image_kernel with scale 1),
+// four pixels at a time where the image is 16-byte aligned.
+__global__ void divide_pair_kernel(float* a, float* b, int64_t n, const unsigned int* peak) {
+    float* img = blockIdx.y ? b : a;
+    const float p = __uint_as_float(*peak);
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t n4 = ((uintptr_t)img & 15) ? 0 : n / 4;
+    for (int64_t t = t0; t < n4; t += step) {
+        float4 v = reinterpret_cast<float4*>(img)[t];
+        reinterpret_cast<float4*>(img)[t] = make_float4(v.x / p, v.y / p, v.z / p, v.w / p);
+    }
+    for (int64_t t = 4 * n4 + t0; t < n; t += step) img[t] = img[t] / p;
+}
+
 }  // namespace
 
 // The bare transforms, out of place: C2R for images (Z2D in FP64, C2R in
@@ -223,7 +238,8 @@ static void exec_r2c(cr_ctx* ctx, int64_t gnx, int64_t gny, float* in, float2* o
 
 template <typename W>
 static void grid_to_image_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2* grid,
-                               float scale, float* image, bool adjoint, const float* real_grid) {
+                               float scale, float* image, bool adjoint, const float* real_grid,
+                               float post) {
     using S = decltype(W::x);
     const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny;
     if ((gnx & 1) || (gny & 1)) fail(CR_INVALID, "grid sizes must be even");
@@ -240,7 +256,8 @@ static void grid_to_image_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const f
         sy = adjoint ? wp->sinc_gy_d : wp->sinc_x_d;
     }
     if (f64 && ctx->image_fft_engine == 0 && dfft_supported(gnx, gny)) {
-        dfft_grid_to_image(ctx, g, grid, real_grid, inv * (double)scale, sx, sy, mode, image);
+        dfft_grids_to_images(ctx, g, 1, &grid, &real_grid, inv * (double)scale, post, sx, sy, mode,
+                             &image, nullptr);
         return;
     }
     const int64_t nh = gnx * (gny / 2 + 1);
@@ -254,6 +271,7 @@ static void grid_to_image_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const f
         raw, gny, g->geom.nx, g->geom.ny, g->info.blc_x, g->info.blc_y, parity,
         inv * (double)scale, g->corr_x_d, g->corr_y_d, sx, sy, mode, image);
     note_launch(ctx, "crop_correct_kernel");
+    if (post != 1.0f) scale_image(ctx, image, n, post, nullptr);
 }
 
 template <typename W>
@@ -493,27 +511,49 @@ void image_to_grid_planes(cr_ctx* ctx, cr_gridder* g, const float* models,
 }
 
 void grid_to_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* grid, float scale,
-                   float* image, bool single) {
+                   float* image, bool single, float post) {
     if (single)
-        grid_to_image_impl<float2>(ctx, g, wp, grid, scale, image, false, nullptr);
+        grid_to_image_impl<float2>(ctx, g, wp, grid, scale, image, false, nullptr, post);
     else
-        grid_to_image_impl<double2>(ctx, g, wp, grid, scale, image, false, nullptr);
+        grid_to_image_impl<double2>(ctx, g, wp, grid, scale, image, false, nullptr, post);
 }
 
-void grid_to_image_real(cr_ctx* ctx, cr_gridder* g, const float* grid, float scale,
-                        float* image, bool single) {
-    if (single)
-        grid_to_image_impl<float2>(ctx, g, nullptr, nullptr, scale, image, false, grid);
-    else
-        grid_to_image_impl<double2>(ctx, g, nullptr, nullptr, scale, image, false, grid);
+void dirty_pair_to_images(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2* psf,
+                          const float* psf_real, const float2* dirty, float scale,
+                          float* psf_image, float* dirty_image, unsigned int* peak_dev,
+                          bool single) {
+    const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny;
+    const int64_t n = (int64_t)g->geom.nx * g->geom.ny;
+    if (!single && ctx->image_fft_engine == 0 && dfft_supported(gnx, gny)) {
+        const float2* grids[2] = {psf, dirty};
+        const float* reals[2] = {psf_real, nullptr};
+        float* images[2] = {psf_image, dirty_image};
+        unsigned int* peaks[2] = {peak_dev, nullptr};
+        CR_CUDA_CHECK(cudaMemsetAsync(peak_dev, 0, 4, ctx->stream));
+        const double inv = 1.0 / ((double)gnx * (double)gny);
+        const float* sinc = wp ? wp->sinc_x_d : nullptr;
+        dfft_grids_to_images(ctx, g, 2, grids, reals, inv * (double)scale, 1.0f, sinc, sinc,
+                             wp ? 1 : 0, images, peaks);
+    } else if (single) {
+        grid_to_image_impl<float2>(ctx, g, wp, psf, scale, psf_image, false, psf_real, 1.0f);
+        abs_peak(ctx, psf_image, n, peak_dev);
+        grid_to_image_impl<float2>(ctx, g, wp, dirty, scale, dirty_image, false, nullptr, 1.0f);
+    } else {
+        grid_to_image_impl<double2>(ctx, g, wp, psf, scale, psf_image, false, psf_real, 1.0f);
+        abs_peak(ctx, psf_image, n, peak_dev);
+        grid_to_image_impl<double2>(ctx, g, wp, dirty, scale, dirty_image, false, nullptr, 1.0f);
+    }
+    divide_pair_kernel<<<dim3(grid_blocks(n, 1024, ctx->sms * 4), 2), 256, 0, ctx->stream>>>(
+        psf_image, dirty_image, n, peak_dev);
+    note_launch(ctx, "divide_pair_kernel");
 }
 
 void grid_to_image_adjoint(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* grid, float scale,
                            float* image, bool single) {
     if (single)
-        grid_to_image_impl<float2>(ctx, g, wp, grid, scale, image, true, nullptr);
+        grid_to_image_impl<float2>(ctx, g, wp, grid, scale, image, true, nullptr, 1.0f);
     else
-        grid_to_image_impl<double2>(ctx, g, wp, grid, scale, image, true, nullptr);
+        grid_to_image_impl<double2>(ctx, g, wp, grid, scale, image, true, nullptr, 1.0f);
 }
 
 void image_to_grid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float* model, float2* grid,

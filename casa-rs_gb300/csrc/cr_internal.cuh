@@ -344,8 +344,9 @@ void read_sums(cr_ctx* ctx, const Records& r, cr_sums* out);
 void wproj_grid(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2* psf, float2* dirty,
                 int mode);
 void wproj_degrid(cr_ctx* ctx, cr_wproj* wp, const Records& r, const float2* grid);
-void std_grid(cr_ctx* ctx, cr_gridder* g, const Records& r, float2* psf, float2* dirty,
-              int mode);
+// psf: the real part of cell c at psf[c * psf_step] (2: a complex grid)
+void std_grid(cr_ctx* ctx, cr_gridder* g, const Records& r, float* psf, int psf_step,
+              float2* dirty, int mode);
 void std_degrid(cr_ctx* ctx, cr_gridder* g, const Records& r, const float2* grid);
 void broadcast_pred(cr_ctx* ctx, const Records& r, float2* pred);
 
@@ -367,8 +368,16 @@ double chauvenet_max_zscore(uint64_t npts);
 // ---- FFT stage -------------------------------------------------------------------
 // grid (device, modified in place) -> image * scale (device)
 // single: float32 C2C transforms instead of FP64 Z2Z (the cube image stage)
+// post: a second float32 factor applied after the correction (1: none)
 void grid_to_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* grid, float scale,
-                   float* image, bool single = false);
+                   float* image, bool single = false, float post = 1.0f);
+// The PSF (complex, or its real part) and the dirty grid of one gridding, both
+// -> images: grid_to_image of each, the PSF image's peak into *peak_dev (float
+// bits), and both images divided by it.
+void dirty_pair_to_images(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2* psf,
+                          const float* psf_real, const float2* dirty, float scale,
+                          float* psf_image, float* dirty_image, unsigned int* peak_dev,
+                          bool single);
 // the exact adjoint of image_to_grid's image-side factor (no sinc division)
 // The image stage over planes of a cube, batched: grids (complex, or the
 // PSF's real parts) [C][gnx][gny] -> images [C][nx][ny] for the listed
@@ -391,17 +400,18 @@ void grid_to_image_adjoint(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* gri
 // model image (device) -> centred model grid (device)
 void image_to_grid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float* model, float2* grid,
                    bool single = false);
-// grid_to_image of a real grid (the real part of a PSF grid), standard gridder
-void grid_to_image_real(cr_ctx* ctx, cr_gridder* g, const float* grid, float scale,
-                        float* image, bool single = false);
 // The FP64-grade image transforms in float-pair arithmetic (cr_dfft.cu):
 // whether both grid sizes are served; grid (or the PSF's real parts) ->
 // image, with crop_correct_body's scale, sinc factors and mode; image ->
 // model grid (apodize_body's factors, then the float32 grid).
 bool dfft_supported(int64_t gnx, int64_t gny);
-void dfft_grid_to_image(cr_ctx* ctx, cr_gridder* g, const float2* grid, const float* real_grid,
-                        double scale, const float* sx, const float* sy, int sinc_mode,
-                        float* image);
+// One or two grids of the same geometry in the same launches; `post` is a
+// second float32 factor; peaks (or null, or null entries) receive max |image|
+// as float bits (the caller clears them).
+void dfft_grids_to_images(cr_ctx* ctx, cr_gridder* g, int count, const float2* const* grids,
+                          const float* const* real_grids, double scale, float post,
+                          const float* sx, const float* sy, int sinc_mode, float* const* images,
+                          unsigned int* const* peaks);
 void dfft_image_to_grid(cr_ctx* ctx, cr_gridder* g, const float* model, const float* sinc_x,
                         const float* sinc_y, float2* grid);
 // max |image| into *peak_dev (float bits as uint32)

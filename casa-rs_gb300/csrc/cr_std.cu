@@ -44,7 +44,8 @@ struct StdGridArgs {
     int64_t ntiles, nty;
     const float* taps;
     int32_t tap_floats;
-    float2* psf;
+    float* psf;
+    int psf_step;
     float2* dirty;
     int64_t gnx, gny;
 };
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kStdThreads) std_grid_kernel(StdGridArgs a) {
                 const float2 d = make_float2(s_dr[c], s_di[c]);
                 // cells past the grid's edge hold zeros
                 if (!RESIDUAL && s_psf[c] != 0.0f) {
-                    atomicAdd(&a.psf[cell].x, s_psf[c]);
+                    atomicAdd(&a.psf[cell * a.psf_step], s_psf[c]);
                     s_psf[c] = 0.0f;
                 }
                 if (d.x != 0.0f || d.y != 0.0f) {
@@ -224,10 +225,10 @@ __global__ void __launch_bounds__(256) std_degrid_kernel(StdDegridArgs a) {
 
 }  // namespace
 
-void std_grid(cr_ctx* ctx, cr_gridder* g, const Records& r, float2* psf, float2* dirty,
-              int mode) {
+void std_grid(cr_ctx* ctx, cr_gridder* g, const Records& r, float* psf, int psf_step,
+              float2* dirty, int mode) {
     StdGridArgs a{r.rec_xy, r.rec_meta, r.rec_vsum, r.rec_wsum, r.rec_pred, r.tile_start,
-                  r.counts, r.ntx * r.nty, r.nty, g->taps_d, g->tap_rows * 7, psf, dirty, g->info.grid_nx,
+                  r.counts, r.ntx * r.nty, r.nty, g->taps_d, g->tap_rows * 7, psf, psf_step, dirty, g->info.grid_nx,
                   g->info.grid_ny};
     const unsigned blocks = (unsigned)(ctx->sms * kStdBlocksPerSm);
     kernel_mark(ctx, 0, false);
