@@ -177,6 +177,42 @@ __device__ __forceinline__ bool df_split(double x, float* hi, float* lo) {
     return true;
 }
 
+// The hardware conversions, out of line so that the compiler branches around
+// them instead of predicating them on the common path.
+__device__ __noinline__ static double fp64_of(float f) { return (double)f; }
+__device__ __noinline__ static float fp32_of(double x) { return __double2float_rn(x); }
+
+// float -> double from the bits (exact, no FP64 instruction); zeros keep
+// their sign, subnormal, infinite and NaN values take the conversion.
+__device__ __forceinline__ double f2d(float f) {
+    const unsigned u = __float_as_uint(f);
+    const unsigned e = (u >> 23) & 0xffu;
+    const unsigned long long sign = (unsigned long long)(u >> 31) << 63;
+    if (e == 0u || e == 0xffu) {
+        if ((u << 1) == 0u) return __longlong_as_double((long long)sign);
+        return fp64_of(f);
+    }
+    return __longlong_as_double((long long)(sign | (unsigned long long)(e + 896u) << 52 |
+                                            (unsigned long long)(u & 0x7fffffu) << 29));
+}
+
+// RN32(x) from the bits (no FP64 instruction): the significand's low 29 bits
+// rounded to nearest even; zeros keep their sign, and values that are not
+// finite or not normal in float32 take the conversion.
+__device__ __forceinline__ float d2f(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    if (e < -126 || e > 126) {
+        if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);
+        return fp32_of(x);
+    }
+    // exponent and top 23 significand bits, plus the carry of the rounding
+    const unsigned top = (unsigned)(e + 127) << 23 | (hi & 0xfffffu) << 3 | lo >> 29;
+    const unsigned low = lo & 0x1fffffffu;
+    const unsigned up = low > 0x10000000u || (low == 0x10000000u && (top & 1u)) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | (top + up));
+}
+
 // A sum held as an unevaluated float32 pair h + l (Knuth's two-sum; about
 // 2^-47 relative per addition): sums of weights without FP64 instructions.
 struct PairSum {

@@ -22,6 +22,7 @@
 
 #include "cr_fixed.cuh"
 #include "cr_internal.cuh"
+#include "cr_lookback.cuh"
 
 namespace cr {
 
@@ -103,7 +104,6 @@ __device__ __forceinline__ unsigned long long warp_sum_u(unsigned long long x) {
 __device__ __noinline__ double fp64_product(float a, float b, float m) {
     return (double)m * ((double)a * (double)b);
 }
-__device__ __noinline__ double fp64_of(float f) { return (double)f; }
 
 // m a b (m a power of two) into s exactly, as the pair (p, fma(a, b, -p));
 // a product outside the range where that pair is exact goes to the FP64
@@ -118,20 +118,6 @@ __device__ __forceinline__ void add_product(PairSum& s, double& fb, bool& used, 
         fb += fp64_product(a, b, m);
         used = true;
     }
-}
-
-// float -> double from the bits (exact, no FP64 instruction); zeros keep
-// their sign, subnormal, infinite and NaN values take the conversion.
-__device__ __forceinline__ double f2d(float f) {
-    const unsigned u = __float_as_uint(f);
-    const unsigned e = (u >> 23) & 0xffu;
-    const unsigned long long sign = (unsigned long long)(u >> 31) << 63;
-    if (e == 0u || e == 0xffu) {
-        if ((u << 1) == 0u) return __longlong_as_double((long long)sign);
-        return fp64_of(f);
-    }
-    return __longlong_as_double((long long)(sign | (unsigned long long)(e + 896u) << 52 |
-                                            (unsigned long long)(u & 0x7fffffu) << 29));
 }
 
 // *p += h + l, one FP64 atomic per nonzero part
@@ -623,28 +609,9 @@ __global__ void __launch_bounds__(kRecThreads) records_kernel(RecArgs a) {
     if (warp == 0) {
         uint32_t h = lane < kRecThreads / 32 ? s_heads[lane] : 0u;
         const uint32_t sum = __reduce_add_sync(0xffffffffu, h);
-        volatile unsigned long long* st = a.state;
-        if (lane == 0 && tile > 0) st[tile] = 1ull << 32 | sum;
-        uint32_t before = 0;
-        bool good = true;
-        for (int64_t p = tile - 1 - lane; ; p -= 32) {
-            // 32 predecessors at a time, lane 0 the nearest; tile -1 holds 0
-            unsigned long long w = p >= 0 ? st[p] : 2ull << 32;
-            for (long long polls = 0; (w >> 32) == 0;) {
-                if (++polls > kLookbackPolls) {
-                    good = false;
-                    break;
-                }
-                w = st[p];
-            }
-            const unsigned full = __ballot_sync(0xffffffffu, (w >> 32) == 2);
-            const int stop = full ? __ffs(full) - 1 : 31;
-            before += __reduce_add_sync(0xffffffffu, lane <= stop ? (uint32_t)w : 0u);
-            good = __all_sync(0xffffffffu, good);
-            if (full || !good) break;
-        }
+        bool good;
+        const uint32_t before = tile_lookback(a.state, tile, sum, &good);
         if (lane == 0) {
-            st[tile] = 2ull << 32 | (before + sum);
             s_base = good ? before : kNoRecord;
             if (!good) {
                 atomicExch(a.fail, 1u);

@@ -15,10 +15,18 @@
 // ones of casa_vis_imaging_weight_uv_lambda (weighting.rs:748-756): the
 // float32 scale f/c, the FP64 product, rounded to float32.
 //
-// Two launches and a scan: the first marks the kept samples, an exclusive
-// scan gives each its slot, the second writes the compacted batch in
-// (row, channel) order.
-#include "cr_internal.cuh"
+// One launch: a tile of samples is loaded and judged, its kept samples are
+// counted, the kept samples before it come by look-back over the earlier tiles'
+// counts, and the tile writes its part of the compacted batch in (row, channel)
+// order.  Each input is read once; the only FP64 instructions are the five
+// products (conversions between float and double go by the bits).  1,263,600
+// rows x 64 channels x 4 correlations: 2.9 -> 1.9 ms (a marking pass, a
+// scan and a writing pass that read everything again, bound by the FP64
+// pipe's conversions as much as by memory).
+#include <algorithm>
+
+#include "cr_fixed.cuh"
+#include "cr_lookback.cuh"
 
 namespace cr {
 
@@ -28,7 +36,7 @@ struct RowArgs {
     int64_t R;
     int32_t C, ncorr;
     const double* uvw;
-    const double* ls;          // [C] f / c, device copy
+    const double* ls;          // [C] f / c, then [C] float32(f / c), device copy
     const float2* data;        // [R][C][ncorr]
     const uint8_t* flag;       // [R][C][ncorr]
     const float* weight;       // [R][ncorr]
@@ -53,44 +61,6 @@ __device__ __forceinline__ float2 collapse(float2 a, float2 b, int transform) {
 
 __device__ __forceinline__ bool pos_finite(float w) { return isfinite(w) && w > 0.0f; }
 
-// The sample of (row r, channel c): false when it is dropped.
-__device__ __forceinline__ bool row_sample(const RowArgs& a, int64_t r, int c, float2* vis,
-                                           float* natural) {
-    if (!pos_finite(a.sumwt_factor)) return false;
-    const int64_t base = (r * a.C + c) * a.ncorr;
-    if (a.mode == 0) {
-        if (a.flag && a.flag[base + a.corr0]) return false;
-        const float2 v = a.data[base + a.corr0];
-        if (!(isfinite(v.x) && isfinite(v.y))) return false;
-        const float w = a.spectrum ? a.spectrum[base + a.corr0] : a.weight[r * a.ncorr + a.corr0];
-        if (!pos_finite(w)) return false;
-        *vis = v;
-        *natural = w;
-        return true;
-    }
-    if (a.flag && (a.flag[base + a.corr0] || a.flag[base + a.corr1])) return false;
-    const float2 v = collapse(a.data[base + a.corr0], a.data[base + a.corr1], a.transform);
-    if (!(isfinite(v.x) && isfinite(v.y))) return false;
-    const float w0 = a.spectrum ? a.spectrum[base + a.corr0] : a.weight[r * a.ncorr + a.corr0];
-    const float w1 = a.spectrum ? a.spectrum[base + a.corr1] : a.weight[r * a.ncorr + a.corr1];
-    if (!(pos_finite(w0) && pos_finite(w1))) return false;
-    const float w = __fmul_rn(0.5f, __fadd_rn(w0, w1));
-    if (!pos_finite(w)) return false;
-    *vis = v;
-    *natural = w;
-    return true;
-}
-
-__global__ void rows_mark_kernel(RowArgs a, uint32_t* keep) {
-    const int64_t n = a.R * a.C;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        float2 v;
-        float w;
-        keep[i] = row_sample(a, i / a.C, (int)(i % a.C), &v, &w) ? 1u : 0u;
-    }
-}
-
 struct RowOut {
     double *u, *v, *w, *du, *dv;
     float* weight;
@@ -99,30 +69,106 @@ struct RowOut {
     float2* vis;
 };
 
-__global__ void rows_write_kernel(RowArgs a, const uint32_t* keep, const uint32_t* slot,
-                                  RowOut o) {
-    const int64_t n = a.R * a.C;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (!keep[i]) continue;
-        const int64_t r = i / a.C;
-        const int c = (int)(i % a.C);
-        float2 vis;
-        float w;
-        row_sample(a, r, c, &vis, &w);
-        const uint32_t k = slot[i];
-        const double ls = a.ls[c];
-        const double um = a.uvw[3 * r], vm = a.uvw[3 * r + 1], wm = a.uvw[3 * r + 2];
+constexpr int kRowThreads = 256;
+constexpr int kRowItems = 8;
+constexpr int kRowTile = kRowThreads * kRowItems;
+
+__global__ void __launch_bounds__(kRowThreads, 4) rows_kernel(RowArgs a, RowOut o,
+                                                              uint32_t* ticket,
+                                                              unsigned long long* state,
+                                                              unsigned long long* total,
+                                                              int* status) {
+    constexpr int kWarps = kRowThreads / 32;
+    __shared__ uint32_t s_count[kRowItems * kWarps];
+    __shared__ uint32_t s_base, s_tile;
+    __shared__ int s_good;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const uint32_t n = (uint32_t)(a.R * a.C);   // below 2^31
+    const uint32_t tile = s_tile, first = tile * (uint32_t)kRowTile + (uint32_t)tid;
+    // item j of a thread is sample first + j * kRowThreads; every load of the
+    // tile is issued before any is judged
+    float2 va[kRowItems], vb[kRowItems];
+    float wa[kRowItems], wb[kRowItems];
+    uint32_t flagged = 0;
+    const bool pair = a.mode != 0;
+#pragma unroll
+    for (int j = 0; j < kRowItems; ++j) {
+        const uint32_t i = first + j * kRowThreads;
+        va[j] = vb[j] = make_float2(0.0f, 0.0f);
+        wa[j] = wb[j] = 0.0f;
+        if (i < n) {
+            const int64_t base = (int64_t)i * a.ncorr;
+            va[j] = a.data[base + a.corr0];
+            if (pair) vb[j] = a.data[base + a.corr1];
+            if (a.flag) {
+                if (a.flag[base + a.corr0]) flagged |= 1u << j;
+                if (pair && a.flag[base + a.corr1]) flagged |= 1u << j;
+            }
+            const float* w = a.spectrum ? a.spectrum + base
+                                        : a.weight + (int64_t)(i / (uint32_t)a.C) * a.ncorr;
+            wa[j] = w[a.corr0];
+            if (pair) wb[j] = w[a.corr1];
+        }
+    }
+    uint32_t keep[kRowItems];   // the warp's kept lanes of item j
+#pragma unroll
+    for (int j = 0; j < kRowItems; ++j) {
+        bool ok = pos_finite(a.sumwt_factor) && !((flagged >> j) & 1u) && pos_finite(wa[j]);
+        if (pair) {
+            ok = ok && pos_finite(wb[j]);
+            va[j] = collapse(va[j], vb[j], a.transform);
+            wa[j] = __fmul_rn(0.5f, __fadd_rn(wa[j], wb[j]));
+            ok = ok && pos_finite(wa[j]);
+        }
+        // a sample past the end has weight zero
+        keep[j] = __ballot_sync(0xffffffffu, ok && isfinite(va[j].x) && isfinite(va[j].y));
+        if (lane == 0) s_count[j * kWarps + warp] = __popc(keep[j]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // 64 counts in sample order: two per lane
+        const uint32_t c0 = s_count[2 * lane], c1 = s_count[2 * lane + 1];
+        uint32_t x = c0 + c1;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, k);
+            if (lane >= k) x += y;
+        }
+        s_count[2 * lane] = x - c0 - c1;
+        s_count[2 * lane + 1] = x - c1;
+        const uint32_t sum = __shfl_sync(0xffffffffu, x, 31);
+        bool good;
+        const uint32_t before = tile_lookback(state, tile, sum, &good);
+        if (lane == 0) {
+            s_base = before;
+            s_good = good;
+            if (!good) atomicExch(status, CR_TIMEOUT);
+            if ((tile + 1) * (uint64_t)kRowTile >= n) *total = (uint64_t)before + sum;
+        }
+    }
+    __syncthreads();
+    if (!s_good) return;
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int j = 0; j < kRowItems; ++j) {
+        if (!((keep[j] >> lane) & 1u)) continue;
+        const uint32_t i = first + j * kRowThreads;
+        const uint32_t r = i / (uint32_t)a.C, c = i - r * (uint32_t)a.C;
+        const uint32_t k = s_base + s_count[j * kWarps + warp] + __popc(keep[j] & lt);
+        const double ls = a.ls[c], ls32 = a.ls[a.C + c];
+        const double um = a.uvw[3 * (int64_t)r], vm = a.uvw[3 * (int64_t)r + 1],
+                     wm = a.uvw[3 * (int64_t)r + 2];
         o.u[k] = __dmul_rn(um, ls);
         o.v[k] = __dmul_rn(vm, ls);
         o.w[k] = __dmul_rn(wm, ls);
-        const double ls32 = (double)__double2float_rn(ls);
-        o.du[k] = (double)__double2float_rn(__dmul_rn(um, ls32));
-        o.dv[k] = (double)__double2float_rn(__dmul_rn(vm, ls32));
-        o.weight[k] = w;
+        o.du[k] = f2d(d2f(__dmul_rn(um, ls32)));
+        o.dv[k] = f2d(d2f(__dmul_rn(vm, ls32)));
+        o.weight[k] = wa[j];
         o.sumwt_factor[k] = a.sumwt_factor;
         o.gridable[k] = a.gridable ? (a.gridable[r] ? 1 : 0) : 1;
-        o.vis[k] = vis;
+        o.vis[k] = va[j];
     }
 }
 
@@ -158,8 +204,14 @@ int64_t prepare_rows(cr_ctx* ctx, const cr_row_runs* rr, const cr_polarization* 
                                             rr->location, "rr_spectrum");
     a.gridable = (const uint8_t*)device_input(ctx, rr->gridable, (size_t)R, rr->location,
                                               "rr_gridable");
-    double* ls = (double*)workspace(ctx, "rr_ls", (size_t)C * 8);
-    CR_CUDA_CHECK(cudaMemcpyAsync(ls, rr->lambda_scale, (size_t)C * 8, cudaMemcpyHostToDevice,
+    // f / c and its float32 value, widened (casa_vis_imaging_weight_uv_lambda)
+    std::vector<double> scales((size_t)C * 2);
+    for (int64_t c = 0; c < C; ++c) {
+        scales[(size_t)c] = rr->lambda_scale[c];
+        scales[(size_t)(C + c)] = (double)(float)rr->lambda_scale[c];
+    }
+    double* ls = (double*)workspace(ctx, "rr_ls", (size_t)C * 16);
+    CR_CUDA_CHECK(cudaMemcpyAsync(ls, scales.data(), (size_t)C * 16, cudaMemcpyHostToDevice,
                                   ctx->stream));
     a.ls = ls;
     a.mode = pol->mode;
@@ -167,24 +219,23 @@ int64_t prepare_rows(cr_ctx* ctx, const cr_row_runs* rr, const cr_polarization* 
     a.corr1 = pol->corr1;
     a.transform = pol->transform;
     a.sumwt_factor = pol->sumwt_factor;
-    const size_t nn = (size_t)std::max<int64_t>(n, 1);
-    uint32_t* keep = (uint32_t*)workspace(ctx, "rr_keep", nn * 4);
-    uint32_t* slot = (uint32_t*)workspace(ctx, "rr_slot", nn * 4);
-    unsigned long long* total = (unsigned long long*)workspace(ctx, "rr_total", 8);
-    if (n > 0) {
-        rows_mark_kernel<<<grid_blocks(n, 256), 256, 0, ctx->stream>>>(a, keep);
-        note_launch(ctx, "rows_mark_kernel");
-    }
-    exclusive_scan_u32(ctx, keep, slot, n, total);
+    const size_t tiles = (size_t)((n + kRowTile - 1) / kRowTile);
+    // the total, the ticket, and a look-back word per tile
+    unsigned long long* work =
+        (unsigned long long*)workspace(ctx, "rr_work", 16 + tiles * 8);
+    unsigned long long* total = work;
+    CR_CUDA_CHECK(cudaMemsetAsync(work, 0, 16 + tiles * 8, ctx->stream));
     if (n > 0) {
         RowOut o{out.u, out.v, out.w, out.du, out.dv, out.weight, out.sumwt_factor, out.gridable,
                  out.vis};
-        rows_write_kernel<<<grid_blocks(n, 256), 256, 0, ctx->stream>>>(a, keep, slot, o);
-        note_launch(ctx, "rows_write_kernel");
+        rows_kernel<<<(unsigned)tiles, kRowThreads, 0, ctx->stream>>>(
+            a, o, (uint32_t*)(work + 1), work + 2, total, ctx->status_d);
+        note_launch(ctx, "rows_kernel");
     }
     unsigned long long h = 0;
     CR_CUDA_CHECK(cudaMemcpyAsync(&h, total, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    check_device_status(ctx);
     return (int64_t)h;
 }
 
