@@ -1546,10 +1546,9 @@ int cr_cube_plan_dirty_images(cr_ctx* ctx, cr_cube_plan* p, float* psf_images,
         }
         // the normalisation of dirty_grids_to_psf_and_residual_owned, as the
         // single-plane cr_dirty_image, with the transforms batched over planes
-        grid_to_image_planes(ctx, g, nullptr, psf, live, scales, pi, single);
-        grid_to_image_planes(ctx, g, dirty, nullptr, live, scales, ri, single);
         const std::vector<float> ones(live.size(), 1.0f);
-        abs_peak_planes(ctx, pi, (int64_t)np, live, peaks);
+        grid_to_image_planes(ctx, g, nullptr, psf, live, scales, ones, pi, peaks, single);
+        grid_to_image_planes(ctx, g, dirty, nullptr, live, scales, ones, ri, nullptr, single);
         scale_image_planes(ctx, pi, (int64_t)np, live, ones, peaks);
         scale_image_planes(ctx, ri, (int64_t)np, live, ones, peaks);
         tm.mark();
@@ -1613,10 +1612,10 @@ int cr_cube_plan_residual_images(cr_ctx* ctx, cr_cube_plan* p, const float* mode
         float* img = out_ptr<float>(ctx, residual_images, out_location, C * np * 4, "cpr_image");
         std::vector<float> scales;
         for (int c : chosen) scales.push_back(1.0f / states[c].normalization_sumwt);
-        grid_to_image_planes(ctx, g, res, nullptr, chosen, scales, img, single);
         std::vector<float> inv_peaks;
         for (int c : chosen) inv_peaks.push_back(1.0f / states[c].psf_peak);
-        scale_image_planes(ctx, img, (int64_t)np, chosen, inv_peaks, nullptr);
+        grid_to_image_planes(ctx, g, res, nullptr, chosen, scales, inv_peaks, img, nullptr,
+                             single);
         for (int c : chosen) {
             if (out_location == CR_HOST)
                 copy_out(ctx, residual_images + (size_t)c * np, img + (size_t)c * np, np * 4,

@@ -236,6 +236,13 @@ static void exec_r2c(cr_ctx* ctx, int64_t gnx, int64_t gny, float* in, float2* o
                 "cufftExecR2C");
 }
 
+// Whether the line kernels run these transforms: in float32 wherever the grid
+// allows, in FP64 grade unless the context asks for cuFFT.
+static bool line_engine(const cr_ctx* ctx, const cr_gridder* g, bool single) {
+    return (single || ctx->image_fft_engine == 0) &&
+           dfft_supported(g->info.grid_nx, g->info.grid_ny);
+}
+
 template <typename W>
 static void grid_to_image_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2* grid,
                                float scale, float* image, bool adjoint, const float* real_grid,
@@ -255,9 +262,9 @@ static void grid_to_image_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const f
         sx = adjoint ? wp->sinc_gx_d : wp->sinc_x_d;
         sy = adjoint ? wp->sinc_gy_d : wp->sinc_x_d;
     }
-    if (f64 && ctx->image_fft_engine == 0 && dfft_supported(gnx, gny)) {
-        dfft_grids_to_images(ctx, g, 1, &grid, &real_grid, inv * (double)scale, post, sx, sy, mode,
-                             &image, nullptr);
+    if (line_engine(ctx, g, !f64)) {
+        dfft_grids_to_images(ctx, g, {{grid, real_grid, image, inv * (double)scale, post, nullptr}},
+                             sx, sy, mode, !f64);
         return;
     }
     const int64_t nh = gnx * (gny / 2 + 1);
@@ -281,9 +288,9 @@ static void image_to_grid_impl(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const f
     const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny;
     if ((gnx & 1) || (gny & 1)) fail(CR_INVALID, "grid sizes must be even");
     const bool f64 = sizeof(S) == 8;
-    if (f64 && ctx->image_fft_engine == 0 && dfft_supported(gnx, gny)) {
-        dfft_image_to_grid(ctx, g, model, wp ? wp->sinc_gx_d : nullptr,
-                           wp ? wp->sinc_gy_d : nullptr, grid);
+    if (line_engine(ctx, g, !f64)) {
+        dfft_images_to_grids(ctx, g, {{model, grid}}, wp ? wp->sinc_gx_d : nullptr,
+                             wp ? wp->sinc_gy_d : nullptr, !f64);
         return;
     }
     const int64_t nh = gnx * (gny / 2 + 1);
@@ -495,15 +502,41 @@ void scale_image_planes(cr_ctx* ctx, float* images, int64_t n, const std::vector
 
 void grid_to_image_planes(cr_ctx* ctx, cr_gridder* g, const float2* grids,
                           const float* real_grids, const std::vector<int>& planes,
-                          const std::vector<float>& scales, float* images, bool single) {
+                          const std::vector<float>& scales, const std::vector<float>& posts,
+                          float* images, unsigned int* peaks, bool single) {
+    const int64_t cells = g->info.grid_nx * g->info.grid_ny;
+    const int64_t n = (int64_t)g->geom.nx * g->geom.ny;
+    if (line_engine(ctx, g, single)) {
+        const double inv = 1.0 / (double)cells;
+        std::vector<DfImage> list;
+        for (size_t k = 0; k < planes.size(); ++k) {
+            const int64_t p = planes[k];
+            list.push_back({grids ? grids + p * cells : nullptr,
+                            real_grids ? real_grids + p * cells : nullptr, images + p * n,
+                            inv * (double)scales[k], posts[k], peaks ? peaks + p : nullptr});
+        }
+        dfft_grids_to_images(ctx, g, list, nullptr, nullptr, 0, single);
+        return;
+    }
     if (single)
         grid_to_image_planes_impl<float2>(ctx, g, grids, real_grids, planes, scales, images);
     else
         grid_to_image_planes_impl<double2>(ctx, g, grids, real_grids, planes, scales, images);
+    if (std::any_of(posts.begin(), posts.end(), [](float f) { return f != 1.0f; }))
+        scale_image_planes(ctx, images, n, planes, posts, nullptr);
+    if (peaks) abs_peak_planes(ctx, images, n, planes, peaks);
 }
 
 void image_to_grid_planes(cr_ctx* ctx, cr_gridder* g, const float* models,
                           const std::vector<int>& planes, float2* grids, bool single) {
+    if (line_engine(ctx, g, single)) {
+        const int64_t cells = g->info.grid_nx * g->info.grid_ny;
+        const int64_t n = (int64_t)g->geom.nx * g->geom.ny;
+        std::vector<DfModel> list;
+        for (int p : planes) list.push_back({models + p * n, grids + p * cells});
+        dfft_images_to_grids(ctx, g, list, nullptr, nullptr, single);
+        return;
+    }
     if (single)
         image_to_grid_planes_impl<float2>(ctx, g, models, planes, grids);
     else
@@ -524,16 +557,14 @@ void dirty_pair_to_images(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2
                           bool single) {
     const int64_t gnx = g->info.grid_nx, gny = g->info.grid_ny;
     const int64_t n = (int64_t)g->geom.nx * g->geom.ny;
-    if (!single && ctx->image_fft_engine == 0 && dfft_supported(gnx, gny)) {
-        const float2* grids[2] = {psf, dirty};
-        const float* reals[2] = {psf_real, nullptr};
-        float* images[2] = {psf_image, dirty_image};
-        unsigned int* peaks[2] = {peak_dev, nullptr};
+    if (line_engine(ctx, g, single)) {
         CR_CUDA_CHECK(cudaMemsetAsync(peak_dev, 0, 4, ctx->stream));
-        const double inv = 1.0 / ((double)gnx * (double)gny);
+        const double k = 1.0 / ((double)gnx * (double)gny) * (double)scale;
         const float* sinc = wp ? wp->sinc_x_d : nullptr;
-        dfft_grids_to_images(ctx, g, 2, grids, reals, inv * (double)scale, 1.0f, sinc, sinc,
-                             wp ? 1 : 0, images, peaks);
+        dfft_grids_to_images(ctx, g,
+                             {{psf, psf_real, psf_image, k, 1.0f, peak_dev},
+                              {dirty, nullptr, dirty_image, k, 1.0f, nullptr}},
+                             sinc, sinc, wp ? 1 : 0, single);
     } else if (single) {
         grid_to_image_impl<float2>(ctx, g, wp, psf, scale, psf_image, false, psf_real, 1.0f);
         abs_peak(ctx, psf_image, n, peak_dev);

@@ -381,11 +381,13 @@ void dirty_pair_to_images(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float2
 // the exact adjoint of image_to_grid's image-side factor (no sinc division)
 // The image stage over planes of a cube, batched: grids (complex, or the
 // PSF's real parts) [C][gnx][gny] -> images [C][nx][ny] for the listed
-// planes, plane k scaled by scales[k] as grid_to_image scales; and models
+// planes, plane k scaled by scales[k] as grid_to_image scales and then by
+// posts[k], its peak into peaks[plane] (or null) as abs_peak; and models
 // [C][nx][ny] -> model grids for the listed planes.
 void grid_to_image_planes(cr_ctx* ctx, cr_gridder* g, const float2* grids,
                           const float* real_grids, const std::vector<int>& planes,
-                          const std::vector<float>& scales, float* images, bool single);
+                          const std::vector<float>& scales, const std::vector<float>& posts,
+                          float* images, unsigned int* peaks, bool single);
 void image_to_grid_planes(cr_ctx* ctx, cr_gridder* g, const float* models,
                           const std::vector<int>& planes, float2* grids, bool single);
 // abs_peak and scale_image over the listed planes of images [C][n]: peaks
@@ -400,20 +402,29 @@ void grid_to_image_adjoint(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, float2* gri
 // model image (device) -> centred model grid (device)
 void image_to_grid(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float* model, float2* grid,
                    bool single = false);
-// The FP64-grade image transforms in float-pair arithmetic (cr_dfft.cu):
-// whether both grid sizes are served; grid (or the PSF's real parts) ->
-// image, with crop_correct_body's scale, sinc factors and mode; image ->
-// model grid (apodize_body's factors, then the float32 grid).
+// The image transforms as line kernels (cr_dfft.cu), FP64-grade in float-pair
+// arithmetic or in float32 (single): whether both grid sizes are served; grids
+// (or their real parts) -> images, each with crop_correct_body's scale, the sinc
+// factors and mode, a second float32 factor `post` (1: none) and the peak
+// (max |image| as float bits, cleared by the caller; or null); and models ->
+// model grids (apodize_body's factors, then the float32 grid).
+struct DfImage {
+    const float2* grid;
+    const float* real_grid;   // where grid is null
+    float* image;
+    double scale;
+    float post;
+    unsigned int* peak;
+};
+struct DfModel {
+    const float* model;
+    float2* grid;
+};
 bool dfft_supported(int64_t gnx, int64_t gny);
-// One or two grids of the same geometry in the same launches; `post` is a
-// second float32 factor; peaks (or null, or null entries) receive max |image|
-// as float bits (the caller clears them).
-void dfft_grids_to_images(cr_ctx* ctx, cr_gridder* g, int count, const float2* const* grids,
-                          const float* const* real_grids, double scale, float post,
-                          const float* sx, const float* sy, int sinc_mode, float* const* images,
-                          unsigned int* const* peaks);
-void dfft_image_to_grid(cr_ctx* ctx, cr_gridder* g, const float* model, const float* sinc_x,
-                        const float* sinc_y, float2* grid);
+void dfft_grids_to_images(cr_ctx* ctx, cr_gridder* g, const std::vector<DfImage>& list,
+                          const float* sx, const float* sy, int sinc_mode, bool single);
+void dfft_images_to_grids(cr_ctx* ctx, cr_gridder* g, const std::vector<DfModel>& list,
+                          const float* sinc_x, const float* sinc_y, bool single);
 // max |image| into *peak_dev (float bits as uint32)
 void abs_peak(cr_ctx* ctx, const float* image, int64_t n, unsigned int* peak_dev);
 // image *= scale, then / *peak_dev when peak_dev != null
