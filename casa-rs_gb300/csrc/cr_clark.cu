@@ -378,6 +378,7 @@ void clark_minor_cycle(cr_ctx* ctx, float* model, float* residual, const float* 
         unsigned long long n_active = 0;
         CR_CUDA_CHECK(cudaMemcpyAsync(&n_active, total, 8, cudaMemcpyDeviceToHost, ctx->stream));
         CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        check_device_status(ctx);
         if (n_active == 0) {
             if (warn) {
                 stop = CR_STOP_NO_CLEANABLE_PIXELS;

@@ -590,7 +590,7 @@ constexpr uint32_t kDegridChunk = 4096; // records per degridding work item
 // (tx, ty), (tx-1, ty), (tx, ty-1), (tx-1, ty-1); their records, taken in
 // that order, are cut into chunks (of the tuned size).  A tile with one chunk is
 // written with plain stores; the chunks of a heavier tile add into the grid
-// with atomics after cube_work_fill zeroed it.  Degridding: each bin's
+// with atomics after cube_zero_heavy zeroed it.  Degridding: each bin's
 // records in chunks of kDegridChunk.
 __device__ __forceinline__ uint32_t bin_count(const uint32_t* bin_start, int64_t bin) {
     return bin_start[bin + 1] - bin_start[bin];
@@ -645,25 +645,31 @@ __global__ void cube_work_count(const uint32_t* bin_start, const uint32_t* cell_
 
 __global__ void cube_work_fill(const uint32_t* grid_chunks, const uint32_t* grid_first,
                                const uint32_t* degrid_chunks, const uint32_t* degrid_first,
-                               int64_t nbins, int64_t ntiles, int64_t nty, int64_t gnx,
-                               int64_t gny, uint2* grid_items, uint2* degrid_items, float* psf,
-                               float2* dirty) {
+                               int64_t nbins, uint2* grid_items, uint2* degrid_items) {
     for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbins;
          b += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t n = grid_chunks[b], f = grid_first[b];
         for (uint32_t k = 0; k < n; ++k) grid_items[f + k] = make_uint2((uint32_t)b, k);
         const uint32_t nd = degrid_chunks[b], fd = degrid_first[b];
         for (uint32_t k = 0; k < nd; ++k) degrid_items[fd + k] = make_uint2((uint32_t)b, k);
-        if (n > 1 && dirty) {
-            const int64_t c = b / ntiles, T = b % ntiles;
-            const int64_t x0 = (T / nty) * kTile, y0 = (T % nty) * kTile;
-            float* pc = psf ? psf + c * gnx * gny : nullptr;
-            float2* dc = dirty + c * gnx * gny;
-            for (int64_t x = x0; x < min(x0 + kTile, gnx); ++x)
-                for (int64_t y = y0; y < min(y0 + kTile, gny); ++y) {
-                    if (pc) pc[x * gny + y] = 0.0f;
-                    dc[x * gny + y] = make_float2(0.0f, 0.0f);
-                }
+    }
+}
+
+// The output tiles of several chunks zeroed, a warp per tile and row by row.
+__global__ void cube_zero_heavy(const uint32_t* grid_chunks, int64_t nbins, int64_t ntiles,
+                                int64_t nty, int64_t gnx, int64_t gny, float* psf,
+                                float2* dirty) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nbins;
+         b += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        if (grid_chunks[b] <= 1) continue;
+        const int64_t c = b / ntiles, T = b % ntiles;
+        const int64_t x0 = (T / nty) * kTile, y = (T % nty) * kTile + lane;
+        if (y >= gny) continue;
+        for (int64_t x = x0; x < min(x0 + kTile, gnx); ++x) {
+            const int64_t cell = (c * gnx + x) * gny + y;
+            if (psf) psf[cell] = 0.0f;
+            dirty[cell] = make_float2(0.0f, 0.0f);
         }
     }
 }
@@ -1308,9 +1314,14 @@ static void make_work_lists(cr_ctx* ctx, cr_gridder* g, CubeRecords& cr, uint32_
     exclusive_scan_u32(ctx, cr.grid_chunks, cr.grid_first, nbins, cr.n_items);
     exclusive_scan_u32(ctx, cr.degrid_chunks, cr.degrid_first, nbins, cr.n_items + 1);
     cube_work_fill<<<grid_blocks(nbins, 256), 256, 0, ctx->stream>>>(
-        cr.grid_chunks, cr.grid_first, cr.degrid_chunks, cr.degrid_first, nbins, cr.ntiles,
-        cr.nty, gi.grid_nx, gi.grid_ny, cr.grid_items, cr.degrid_items, psf, dirty);
+        cr.grid_chunks, cr.grid_first, cr.degrid_chunks, cr.degrid_first, nbins, cr.grid_items,
+        cr.degrid_items);
     note_launch(ctx, "cube_work_fill");
+    if (dirty) {
+        cube_zero_heavy<<<grid_blocks(nbins * 32, 256), 256, 0, ctx->stream>>>(
+            cr.grid_chunks, nbins, cr.ntiles, cr.nty, gi.grid_nx, gi.grid_ny, psf, dirty);
+        note_launch(ctx, "cube_zero_heavy");
+    }
     cr.grid_chunk = chunk;
     cr.fill_done = true;
     cr.lists_masked = plane_mask != nullptr;

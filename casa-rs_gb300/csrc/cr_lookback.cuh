@@ -36,7 +36,8 @@ __device__ __forceinline__ uint32_t tile_lookback(unsigned long long* state, int
         ok = __all_sync(0xffffffffu, ok);
         if (full || !ok) break;
     }
-    if (lane == 0) st[tile] = 2ull << 32 | (before + count);
+    // a tile whose wait gave up publishes no total, so every later tile gives up too
+    if (lane == 0 && ok) st[tile] = 2ull << 32 | (before + count);
     *good = ok;
     return before;
 }
