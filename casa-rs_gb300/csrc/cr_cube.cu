@@ -26,9 +26,9 @@
 // and scatters 16-byte records {cell | tap rows, sample, w vis} plus the
 // weight into bin order.  The index selection runs on the integer fixed-point path of
 // cr_fixed.cuh with the FP64 operations as the fallback.  Gridding gives
-// every (channel, output tile) to one block, which gathers the records of
-// the four home tiles whose 7 x 7 footprints reach it, accumulates the tile
-// in shared memory and writes it once with coalesced stores -- no memset and
+// every (channel, output tile) to one block, which takes the records of
+// the four home tiles whose 7 x 7 footprints reach it (contiguous ranges, by
+// the order of the cells), accumulates the tile in shared memory and writes it once with coalesced stores -- no memset and
 // no global atomics on the output grids.
 #include <algorithm>
 #include <cmath>
@@ -45,13 +45,12 @@ namespace {
 
 constexpr int kCubeThreads = 256;
 constexpr int kRowsPerBlock = 4096;   // rows of one channel per planning block
-// Shared-memory tile rows are 39 floats apart (39 = 7 mod 32): the 49 taps
-// t = 7 ix + iy of one record then fall in 49 consecutive banks mod 32, so
-// each warp-wide atomic touches 32 distinct banks.
+// Shared-memory tile rows are 39 floats apart (39 = 7 mod 32), so that the
+// seven rows of a footprint fall in different banks.
 constexpr int kRow = 39;
-constexpr int kMaxTapRows = 513;      // oversampling up to 512
-// the tap table in floats, rounded up to whole 16-byte bulk-copy units
-constexpr int kTapFloats = (kMaxTapRows * 7 + 3) / 4 * 4;
+constexpr int kMaxTapRows = 255;      // oversampling up to 254, as the gridder's
+// the tap table in floats, rows padded to 8
+constexpr int kTapFloats = kMaxTapRows * 8;
 
 struct CubeChan {
     double lscale;       // f / c
@@ -304,10 +303,21 @@ __device__ __forceinline__ void eval_samples(const CubeArgs& a, const CubeChan& 
 
 // Records are binned by (channel, home tile, start cell in the tile), so that
 // within a home tile they follow the cell order and records with one start
-// cell are adjacent.
+// cell are adjacent.  The order puts the cells in four groups: those whose
+// footprint stays in the tile; those that reach the next tile in y only
+// (y >= 26), in both directions, in x only.  The records that reach any one
+// neighbour are then contiguous.
+constexpr uint32_t kReachY = 26 * 26;                // first cell that reaches tile y + 1
+constexpr uint32_t kReachXY = kReachY + 26 * 6;      // ... both x + 1 and y + 1
+constexpr uint32_t kReachYEnd = kReachXY + 6 * 6;    // end of those reaching y + 1
+__device__ __forceinline__ uint32_t cell_order(uint32_t x, uint32_t y) {
+    return y >= 26 ? 6 * x + y + (kReachY - 26)
+                   : 26 * x + y + (x >= 26 ? kReachYEnd - kReachY : 0u);
+}
+
 __device__ __forceinline__ int64_t cell_bin(int c, int64_t ntiles, uint32_t tile,
                                             uint32_t meta) {
-    return (((int64_t)c * ntiles + tile) << 10) | (int64_t)(meta >> 22);
+    return (((int64_t)c * ntiles + tile) << 10) | cell_order(meta >> 27, (meta >> 22) & 31u);
 }
 
 // Pass 1 over every sample: with DENSITY the weight density of both cells
@@ -602,25 +612,21 @@ __device__ __forceinline__ uint32_t cell_start(const uint32_t* cell_end, int64_t
     return cb == 0 ? 0u : cell_end[cb - 1];
 }
 
-// The records of output tile (c, tx, ty)'s four sources that can reach it:
-// all of the home tile; of (tx-1, ty) and (tx-1, ty-1) only start cells with
-// x >= 26 (a contiguous suffix, records being in cell order); all of
-// (tx, ty-1) (its reaching cells, y >= 26, are not contiguous).
-__device__ __forceinline__ void source_ranges(const uint32_t* bin_start,
-                                              const uint32_t* cell_end, int64_t c,
-                                              int64_t ntiles, int64_t nty, int64_t tx,
-                                              int64_t ty, uint32_t (&lo)[4],
-                                              uint32_t (&hi)[4]) {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int64_t sx = tx - (s & 1), sy = ty - (s >> 1);
-        lo[s] = hi[s] = 0u;
-        if (sx < 0 || sy < 0) continue;
-        const int64_t sb = c * ntiles + sx * nty + sy;
-        hi[s] = bin_start[sb + 1];
-        lo[s] = (s & 1) ? cell_start(cell_end, (sb << 10) + (kTile - 6) * kTile)
-                        : bin_start[sb];
-    }
+// The records of one source of output tile (tx, ty) of channel c that reach
+// it: source s is home tile (tx - (s & 1), ty - (s >> 1)); all of the tile's
+// own, of the others the group of cells that reaches across.
+__device__ __forceinline__ uint2 source_range(const uint32_t* bin_start,
+                                              const uint32_t* cell_end, uint32_t c,
+                                              uint32_t ntiles, uint32_t nty, uint32_t tx,
+                                              uint32_t ty, int s) {
+    const uint32_t dx = s & 1, dy = s >> 1;
+    if (tx < dx || ty < dy) return make_uint2(0u, 0u);
+    const int64_t sb = (int64_t)c * ntiles + (tx - dx) * nty + (ty - dy);
+    const int64_t cb = sb << 10;
+    return make_uint2(s == 0   ? bin_start[sb]
+                      : s == 2 ? cell_start(cell_end, cb + kReachY)
+                               : cell_start(cell_end, cb + kReachXY),
+                      s < 2 ? bin_start[sb + 1] : cell_start(cell_end, cb + kReachYEnd));
 }
 
 // Channels whose plane_mask entry is 0 get no work items.
@@ -630,14 +636,18 @@ __global__ void cube_work_count(const uint32_t* bin_start, const uint32_t* cell_
                                 uint32_t* degrid_chunks) {
     for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbins;
          b += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = b / ntiles, T = b % ntiles;
+        const uint32_t c = (uint32_t)b / (uint32_t)ntiles, T = (uint32_t)b % (uint32_t)ntiles;
         if (plane_mask && !plane_mask[c]) {
             grid_chunks[b] = degrid_chunks[b] = 0u;
             continue;
         }
-        uint32_t lo[4], hi[4];
-        source_ranges(bin_start, cell_end, c, ntiles, nty, T / nty, T % nty, lo, hi);
-        const uint32_t n = (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]) + (hi[3] - lo[3]);
+        const uint32_t tx = T / (uint32_t)nty, ty = T % (uint32_t)nty;
+        uint32_t n = 0;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint2 r = source_range(bin_start, cell_end, c, ntiles, nty, tx, ty, s);
+            n += r.y - r.x;
+        }
         grid_chunks[b] = n == 0 ? 1u : (n + grid_chunk - 1) / grid_chunk;
         degrid_chunks[b] = (bin_count(bin_start, b) + kDegridChunk - 1) / kDegridChunk;
     }
@@ -679,7 +689,7 @@ struct CubeGridArgs {
     const float* rec_w;
     const uint32_t* bin_start;   // [C * ntiles + 1]
     const uint32_t* cell_end;    // [C * ntiles * 1024] end of each cell bin
-    const float* taps;           // [tap_rows][7], zero-padded to taps_bytes
+    const float* taps;           // [tap_rows][8], rows padded with a zero
     int32_t tap_rows;
     uint32_t taps_bytes;
     int* status;                 // set to CR_TIMEOUT when a bounded wait gives up
@@ -697,31 +707,108 @@ struct CubeGridArgs {
 
 // A block per work item: the chunk's records (from the four source bins)
 // accumulate into a shared-memory copy of the output tile, which is then
-// stored (single-chunk tile) or added (heavier tile) to the grid.  A warp
-// loads 32 records, keeps those whose footprint reaches the tile and runs
-// them in turn, one lane per tap; tile rows are kRow floats apart so that a
-// record's 49 taps hit distinct banks.  (A variant with a private tile per
-// warp and plain read-modify-writes ran 1.5x slower: 8 warps per SM could
-// not hide the dependent shared-memory chain of consecutive records.)
-constexpr int kGridThreads = kCubeThreads;
+// stored (single-chunk tile) or added (heavier tile) to the grid.
+//
+// The kernel is bound by instruction issue (some 18 M records of 49 taps on a
+// 16-channel batch of 1.26 M rows), so records are summed by runs of one start
+// cell.  A warp's four groups of eight lanes take a record each: lane ix of a
+// group holds row ix of the 7 x 7 footprint, its columns as four pairs per
+// component, and a record costs the group one x tap, two 16-byte loads of y
+// taps and twelve paired FMAs.  A vote over the records' cells ends a run:
+// the groups' sums are then exchanged so that each lane holds two columns,
+// and added to the tile.  A float32 add to shared memory is a
+// compare-and-swap loop that the hardware serialises by lane, so re and im
+// share one 64-bit swap.  Records are decoded by a lane each, 32 ahead of
+// their use; warp 0 fetches the next item's ranges before the tile is
+// written; the tile is zeroed as it is read out.
+//
+// Four warps per block: an item has some 600 records, and every warp more
+// cuts its runs once more (256 threads: 6 % slower; 96 and 64 lose occupancy
+// to the tile's shared memory, 13 and 44 %).  16 channels of 1.26 M rows:
+// 0.57 ms against 0.78 with a lane per tap (411 M instructions against 742 M).
+constexpr int kGridThreads = 128, kGridBlocks = 8;
 
 // With RESIDUAL the records carry w (vis - pred) from `res` and no PSF is
 // formed.
+// A work item as the block reads it.  The tile's sources one after the other
+// give its records positions: source s holds [off[s], off[s + 1]) and
+// position p is record p + rec[s].
+struct GridItem {
+    int32_t count;       // records of the chunk, from position `first`; -1: no more items
+    uint32_t first;
+    uint32_t off[5];
+    uint32_t rec[4];
+    int32_t x0, y0, rows, cols;   // the tile and its extent inside the grid
+    int64_t plane;
+    bool shared;         // the tile has several chunks
+};
+
+// The next work item into `out`, by one warp.
+__device__ __forceinline__ void next_item(const CubeGridArgs& a, int lane, GridItem& out) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(a.item_counter, 1u);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= *a.n_items) {
+        if (lane == 0) out.count = -1;
+        return;
+    }
+    const uint2 it = a.items[item];
+    const uint32_t nty = (uint32_t)a.nty, ntiles = (uint32_t)a.ntx * nty;
+    const uint32_t c = it.x / ntiles, T = it.x % ntiles, tx = T / nty, ty = T % nty;
+    const uint2 r = lane < 4 ? source_range(a.bin_start, a.cell_end, c, ntiles, nty, tx, ty, lane)
+                             : make_uint2(0u, 0u);
+    uint32_t end = r.y - r.x;   // inclusive sum over lanes 0-3
+#pragma unroll
+    for (int o = 1; o < 4; o *= 2) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += up;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, end, 3);
+    if (lane < 4) {
+        out.off[lane + 1] = end;
+        out.rec[lane] = r.y - end;
+    }
+    if (lane == 0) {
+        const uint32_t lo = it.y * a.grid_chunk;
+        out.off[0] = 0;
+        out.first = lo;
+        out.count = (int32_t)(min(total, lo + a.grid_chunk) - min(total, lo));
+        out.x0 = (int32_t)(tx * kTile);
+        out.y0 = (int32_t)(ty * kTile);
+        out.rows = (int32_t)min((int64_t)kTile, a.gnx - tx * kTile);
+        out.cols = (int32_t)min((int64_t)kTile, a.gny - ty * kTile);
+        out.plane = c;
+        out.shared = a.grid_chunks[it.x] > 1;
+    }
+}
+
+// (re, im) += (x, y) in shared memory, one 64-bit compare-and-swap per try
+__device__ __forceinline__ void shared_add2(float2* p, float x, float y) {
+    unsigned long long* q = reinterpret_cast<unsigned long long*>(p);
+    unsigned long long old = *q, seen;
+    do {
+        seen = old;
+        const float re = __uint_as_float((uint32_t)seen) + x;
+        const float im = __uint_as_float((uint32_t)(seen >> 32)) + y;
+        old = atomicCAS(q, seen,
+                        (unsigned long long)__float_as_uint(im) << 32 | __float_as_uint(re));
+    } while (old != seen);
+}
+
 template <bool RESIDUAL>
-__global__ void __launch_bounds__(kGridThreads, 6) cube_grid_kernel(CubeGridArgs a) {
-    __shared__ float s_psf[kTile * kRow];
-    __shared__ float s_re[kTile * kRow];
-    __shared__ float s_im[kTile * kRow];
+__global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(CubeGridArgs a) {
+    constexpr int kPlane = kTile * kRow, kComps = RESIDUAL ? 2 : 3;
+    constexpr int kWarps = kGridThreads / 32;
+    constexpr int kAcc = 4 * kComps;   // a lane's sums in pairs: component x 8 columns
+    constexpr uint32_t kDone = ~0u;
     __shared__ __align__(16) float s_taps[kTapFloats];
+    __shared__ float s_psf[RESIDUAL ? 1 : kPlane];
+    __shared__ __align__(8) float2 s_ri[kPlane];
+    __shared__ __align__(16) int4 s_ra[kGridThreads];
+    __shared__ __align__(8) float2 s_rb[kGridThreads];
     __shared__ __align__(8) uint64_t s_bar;
-    // per warp, the decoded records of its current batch of 32:
-    // {run key, x tap row * 7, y tap row * 7, weight} and {w vis}
-    __shared__ int4 s_ra[kGridThreads];
-    __shared__ float2 s_rb[kGridThreads];
-    __shared__ int s_item;
+    __shared__ GridItem s_items[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t ntiles = a.ntx * a.nty;
-    const unsigned long long n_items = *a.n_items;
     // the tap table by one bulk copy
     if (tid == 0) {
         mbar_init(&s_bar, 1);
@@ -737,186 +824,176 @@ __global__ void __launch_bounds__(kGridThreads, 6) cube_grid_kernel(CubeGridArgs
         }
         return;
     }
+    if (warp == 0) next_item(a, lane, s_items[0]);
+    // the tile is zero between items
+    for (int k = tid; k < kPlane; k += kGridThreads) {
+        if (!RESIDUAL) s_psf[k] = 0.0f;
+        s_ri[k] = make_float2(0.0f, 0.0f);
+    }
     int4* w_ra = s_ra + warp * 32;
     float2* w_rb = s_rb + warp * 32;
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(a.item_counter, 1u);
-        __syncthreads();
-        const int64_t item = s_item;
-        if ((unsigned long long)item >= n_items) break;
-        const uint2 it = a.items[item];
-        const int64_t bin = it.x;
-        const int64_t c = bin / ntiles, T = bin % ntiles;
-        const int64_t tx = T / a.nty, ty = T % a.nty;
-        const bool shared_tile = a.grid_chunks[bin] > 1;
-        const uint32_t clo = it.y * a.grid_chunk, chi = clo + a.grid_chunk;
-        // source s = home tile (tx - (s & 1), ty - (s >> 1)); [b0, b1) its records
-        // inside this chunk (empty when none)
-        uint32_t b0[4], b1[4];
-        source_ranges(a.bin_start, a.cell_end, c, ntiles, a.nty, tx, ty, b0, b1);
-        int nsrc = 0;
-        uint32_t off = 0;   // position of this source in the concatenated order
+    const int g = lane >> 3, ix = lane & 7;
+    const float* tap_x = s_taps + ix;
+    float2 acc[kAcc];
+    auto clear = [&]() {
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const uint32_t lo = b0[s], n = b1[s] - b0[s];
-            const uint32_t a0 = max(off, clo), a1 = min(off + n, chi);
-            b0[s] = b1[s] = 0;
-            if (a0 < a1) {
-                b0[s] = lo + (a0 - off);
-                b1[s] = lo + (a1 - off);
-                ++nsrc;
-            }
-            off += n;
-        }
-        const int64_t gx0 = tx * kTile, gy0 = ty * kTile;
-        float* psf_c = RESIDUAL ? nullptr : a.psf + c * a.gnx * a.gny;
-        float2* dirty_c = a.dirty + c * a.gnx * a.gny;
-        if (nsrc == 0) {
-            if (!shared_tile)
-                for (int k = tid; k < kTile * kTile; k += kGridThreads) {
-                    const int64_t x = gx0 + k / kTile, y = gy0 + k % kTile;
-                    if (x < a.gnx && y < a.gny) {
-                        if (!RESIDUAL) psf_c[x * a.gny + y] = 0.0f;
-                        dirty_c[x * a.gny + y] = make_float2(0.0f, 0.0f);
-                    }
-                }
-            __syncthreads();
-            continue;
-        }
-        for (int k = tid; k < kTile * kRow; k += kGridThreads) {
-            s_psf[k] = 0.0f;
-            s_re[k] = 0.0f;
-            s_im[k] = 0.0f;
-        }
+        for (int q = 0; q < kAcc; ++q) acc[q] = make_float2(0.0f, 0.0f);
+    };
+    for (int buf = 0;; buf ^= 1) {
         __syncthreads();
-        // Records of a home tile arrive in start-cell order, so a warp's
-        // consecutive records often share a start cell: lane t sums tap t of
-        // such a run in registers and adds it to the tile once per run.
-        // Lane t holds taps t (slot 0) and t + 32 (slot 1, lanes 0-16; the
-        // other lanes form a dummy product that is never added).  A run is
-        // keyed by (source, start cell); a run whose footprint lies inside
-        // the tile adds at run base + a per-lane offset without bounds tests.
-        const int ix0 = lane / 7, iy0 = lane % 7;
-        const int ix1 = (lane + 32) / 7, iy1 = (lane + 32) % 7;
-        const bool has1 = lane + 32 < 49;
-        const int jx1 = has1 ? ix1 : 0, jy1 = has1 ? iy1 : 0;
-        const int off0 = ix0 * kRow + iy0, off1 = ix1 * kRow + iy1;
-        uint32_t cur_key = ~0u;
-        int cur_lx = 0, cur_ly = 0, cur_base = 0;
-        bool cur_inside = false;
-        // (psf slot 0, psf slot 1), (re, im) slot 0, (re, im) slot 1: paired
-        // float32 FMAs (FFMA2) update two sums per instruction
-        float2 pp = make_float2(0.f, 0.f), ri0 = pp, ri1 = pp;
-        auto flush = [&]() {
-            if (cur_inside) {
-                const int c0 = cur_base + off0;
-                if (!RESIDUAL) atomicAdd(&s_psf[c0], pp.x);
-                atomicAdd(&s_re[c0], ri0.x);
-                atomicAdd(&s_im[c0], ri0.y);
-                if (has1) {
-                    const int c1 = cur_base + off1;
-                    if (!RESIDUAL) atomicAdd(&s_psf[c1], pp.y);
-                    atomicAdd(&s_re[c1], ri1.x);
-                    atomicAdd(&s_im[c1], ri1.y);
+        const GridItem& it = s_items[buf];
+        if (it.count < 0) break;
+        // the groups' sums of the run at cell (x, y) of the tile, exchanged so
+        // that group q holds columns 2 q and 2 q + 1 of each row, into the tile
+        auto flush = [&](int x, int y) {
+            const bool hi = lane & 16, hi2 = lane & 8;
+            float n[kComps][2];
+#pragma unroll
+            for (int c = 0; c < kComps; ++c) {
+                float m[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const float2 p0 = acc[4 * c + (t >> 1)], p1 = acc[4 * c + 2 + (t >> 1)];
+                    const float f0 = (t & 1) ? p0.y : p0.x, f1 = (t & 1) ? p1.y : p1.x;
+                    m[t] = (hi ? f1 : f0) + __shfl_xor_sync(0xffffffffu, hi ? f0 : f1, 16);
                 }
-                return;
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+                    n[c][t] = (hi2 ? m[t + 2] : m[t]) +
+                              __shfl_xor_sync(0xffffffffu, hi2 ? m[t] : m[t + 2], 8);
             }
-            int cx = cur_lx + ix0, cy = cur_ly + iy0;
-            if (cx >= 0 && cx < kTile && cy >= 0 && cy < kTile) {
-                const int cell = cx * kRow + cy;
-                if (!RESIDUAL) atomicAdd(&s_psf[cell], pp.x);
-                atomicAdd(&s_re[cell], ri0.x);
-                atomicAdd(&s_im[cell], ri0.y);
-            }
-            cx = cur_lx + ix1;
-            cy = cur_ly + iy1;
-            if (has1 && cx >= 0 && cx < kTile && cy >= 0 && cy < kTile) {
-                const int cell = cx * kRow + cy;
-                if (!RESIDUAL) atomicAdd(&s_psf[cell], pp.y);
-                atomicAdd(&s_re[cell], ri1.x);
-                atomicAdd(&s_im[cell], ri1.y);
+            const bool row = ix < 7 && (unsigned)(x + ix) < kTile;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int iy = 2 * g + t;
+                if (row && iy < 7 && (unsigned)(y + iy) < kTile) {
+                    const int cell = (x + ix) * kRow + y + iy;
+                    if (!RESIDUAL) atomicAdd(&s_psf[cell], n[0][t]);
+                    shared_add2(&s_ri[cell], n[kComps - 2][t], n[kComps - 1][t]);
+                }
             }
         };
-#pragma unroll
+        // each warp takes a contiguous share of the item's records
+        const uint32_t n = (uint32_t)it.count;
+        const uint32_t share = max(32u, (n + 4 * kWarps - 1) / (4 * kWarps) * 4u);
+        const uint32_t w0 = it.first + min(n, warp * share);
+        const uint32_t w1 = it.first + min(n, (warp + 1) * share);
+        int open_x = 0, open_y = 0;
+        bool any = false;
+        clear();
+#pragma unroll 1
         for (int s = 0; s < 4; ++s) {
-            const int sox = -(s & 1) * kTile, soy = -(s >> 1) * kTile;
-            for (uint32_t base = b0[s] + warp * 32; base < b1[s]; base += kGridThreads) {
-                // lanes load and decode 32 records; those that reach the
-                // tile are packed into the warp's staging slots
-                const uint32_t rr = base + lane;
-                bool rel = false;
-                int4 ra = make_int4(0, 0, 0, 0);
-                float2 rb = make_float2(0.0f, 0.0f);
-                if (rr < b1[s]) {
-                    const uint4 q = a.rec[rr];
-                    float qw = 0.0f;
+            const uint32_t lo = max(w0, it.off[s]), hi = min(w1, it.off[s + 1]);
+            if (lo >= hi) continue;
+            const uint32_t end = hi + it.rec[s];
+            const int sx = (s & 1) * kTile, sy = (s >> 1) * kTile;
+            uint32_t open = kDone - 1;   // the run's cell; none yet
+            uint32_t meta = 0;
+            float w = 0.0f;
+            float2 v = make_float2(0.0f, 0.0f);
+            auto load = [&](uint32_t i) {
+                if (i < end) {
                     if (RESIDUAL) {
-                        rb = a.res[rr];
+                        meta = a.rec[i].x;
+                        v = a.res[i];
                     } else {
-                        qw = a.rec_w[rr];
-                        rb = make_float2(__uint_as_float(q.z), __uint_as_float(q.w));
+                        const uint4 q = a.rec[i];
+                        meta = q.x;
+                        w = a.rec_w[i];
+                        v = make_float2(__uint_as_float(q.z), __uint_as_float(q.w));
                     }
-                    const int lx = sox + (int)(q.x >> 27), ly = soy + (int)((q.x >> 22) & 31);
-                    rel = lx + 6 >= 0 && ly + 6 >= 0;
-                    ra = make_int4((int)((q.x >> 22) | ((uint32_t)s << 10)),
-                                   (int)((q.x >> 11) & 2047u) * 7, (int)(q.x & 2047u) * 7,
-                                   __float_as_int(qw));
                 }
-                const unsigned m = __ballot_sync(0xffffffffu, rel);
-                if (rel) {
-                    const int pos = __popc(m & ((1u << lane) - 1u));
-                    w_ra[pos] = ra;
-                    w_rb[pos] = rb;
-                }
+            };
+            uint32_t base = lo + it.rec[s];
+            load(base + lane);
+#pragma unroll 1
+            for (; base < end; base += 32) {
+                // 32 records decoded by a lane each; the next 32 on their way
                 __syncwarp();
-                const int nrel = __popc(m);
-                for (int k = 0; k < nrel; ++k) {
+                w_ra[lane] = make_int4(base + lane < end ? (int)(meta >> 22) : (int)kDone,
+                                       (int)((meta >> 11) & 2047u) * 8, (int)(meta & 2047u) * 8,
+                                       __float_as_int(w));
+                w_rb[lane] = v;
+                __syncwarp();
+                load(base + 32 + lane);
+                const int n_batch = (int)min(32u, end - base);
+#pragma unroll 1
+                for (int k = g; k - g < n_batch; k += 4) {
                     const int4 A = w_ra[k];
                     const float2 B = w_rb[k];
-                    const float pw = __int_as_float(A.w);
-                    const uint32_t key = (uint32_t)A.x;
-                    if (key != cur_key) {
-                        if (cur_key != ~0u) flush();
-                        cur_key = key;
-                        cur_lx = sox + (int)((key >> 5) & 31);
-                        cur_ly = soy + (int)(key & 31);
-                        cur_base = cur_lx * kRow + cur_ly;
-                        cur_inside = cur_lx >= 0 && cur_ly >= 0 && cur_lx <= kTile - 7 &&
-                                     cur_ly <= kTile - 7;
-                        pp = ri0 = ri1 = make_float2(0.f, 0.f);
+                    uint32_t cell = (uint32_t)A.x;
+                    const float wq = __int_as_float(A.w);
+                    const float wx = tap_x[A.y];
+                    const float4* wy = reinterpret_cast<const float4*>(s_taps + A.z);
+                    const float4 y0 = wy[0], y1 = wy[1];
+                    const float2 y[4] = {make_float2(y0.x, y0.y), make_float2(y0.z, y0.w),
+                                         make_float2(y1.x, y1.y), make_float2(y1.z, y1.w)};
+                    for (;;) {
+                        const bool mine = cell == open;
+                        const unsigned match = __ballot_sync(0xffffffffu, mine);
+                        if (match) {
+                            int c = 0;
+                            if (!RESIDUAL) {
+                                const float p = mine ? __fmul_rn(wx, wq) : 0.0f;
+#pragma unroll
+                                for (int q = 0; q < 4; ++q)
+                                    acc[q] = __ffma2_rn(make_float2(p, p), y[q], acc[q]);
+                                c = 4;
+                            }
+                            const float p = mine ? __fmul_rn(wx, B.x) : 0.0f;
+                            const float q2 = mine ? __fmul_rn(wx, B.y) : 0.0f;
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                acc[c + q] = __ffma2_rn(make_float2(p, p), y[q], acc[c + q]);
+                                acc[c + 4 + q] =
+                                    __ffma2_rn(make_float2(q2, q2), y[q], acc[c + 4 + q]);
+                            }
+                            if (match == 0xffffffffu) break;
+                            if (mine) cell = kDone;
+                        }
+                        const unsigned rest = __ballot_sync(0xffffffffu, cell != kDone);
+                        if (!rest) break;
+                        if (any) {
+                            flush(open_x, open_y);
+                            clear();
+                        }
+                        any = true;
+                        open = __shfl_sync(0xffffffffu, cell, __ffs(rest) - 1);
+                        open_x = (int)(open >> 5) - sx;
+                        open_y = (int)(open & 31u) - sy;
                     }
-                    const float* wx = s_taps + A.y;
-                    const float* wy = s_taps + A.z;
-                    // w0 = wx[ix0] wy[iy0], w1 = wx[jx1] wy[jy1] (float32
-                    // products), then one fused multiply-add per sum as before
-                    const float2 w = __fmul2_rn(make_float2(wx[ix0], wx[jx1]),
-                                                make_float2(wy[iy0], wy[jy1]));
-                    if (!RESIDUAL) pp = __ffma2_rn(make_float2(pw, pw), w, pp);
-                    ri0 = __ffma2_rn(B, make_float2(w.x, w.x), ri0);
-                    ri1 = __ffma2_rn(B, make_float2(w.y, w.y), ri1);
                 }
-                __syncwarp();   // the slots are refilled by the next batch
             }
         }
-        if (cur_key != ~0u) flush();
+        if (any) flush(open_x, open_y);
+        if (warp == 0) next_item(a, lane, s_items[buf ^ 1]);
         __syncthreads();
-        for (int k = tid; k < kTile * kTile; k += kGridThreads) {
-            const int cx = k / kTile, cy = k % kTile;
-            const int64_t x = gx0 + cx, y = gy0 + cy;
-            if (x < a.gnx && y < a.gny) {
-                const int cell = cx * kRow + cy;
+        // the tile to the grid, a warp per row
+        const int64_t x0 = it.x0, y0 = it.y0;
+        const int rows = it.rows;
+        const bool col = lane < it.cols, shared_tile = it.shared;
+        const int64_t at0 = (it.plane * a.gnx + x0 + warp) * a.gny + y0 + lane;
+        float* psf = RESIDUAL ? nullptr : a.psf + at0;
+        float2* dirty = a.dirty + at0;
+#pragma unroll 4
+        for (int j = warp; j < kTile; j += kWarps) {
+            const int cell = j * kRow + lane;
+            const float vp = RESIDUAL ? 0.0f : s_psf[cell];
+            const float2 v = s_ri[cell];
+            if (!RESIDUAL) s_psf[cell] = 0.0f;
+            s_ri[cell] = make_float2(0.0f, 0.0f);
+            if (col && j < rows) {
                 if (!shared_tile) {
-                    if (!RESIDUAL) psf_c[x * a.gny + y] = s_psf[cell];
-                    dirty_c[x * a.gny + y] = make_float2(s_re[cell], s_im[cell]);
+                    if (!RESIDUAL) *psf = vp;
+                    *dirty = v;
                 } else {
-                    if (!RESIDUAL && s_psf[cell] != 0.0f)
-                        atomicAdd(&psf_c[x * a.gny + y], s_psf[cell]);
-                    if (s_re[cell] != 0.0f || s_im[cell] != 0.0f)
-                        atomicAdd(&dirty_c[x * a.gny + y], make_float2(s_re[cell], s_im[cell]));
+                    if (!RESIDUAL && vp != 0.0f) atomicAdd(psf, vp);
+                    if (v.x != 0.0f || v.y != 0.0f) atomicAdd(dirty, v);
                 }
             }
+            if (!RESIDUAL) psf += kWarps * a.gny;
+            dirty += kWarps * a.gny;
         }
-        __syncthreads();
     }
 }
 
@@ -1171,7 +1248,7 @@ CubeRecords cube_plan(cr_ctx* ctx, cr_gridder* g, const CubeInput& in, int32_t m
     if ((uint64_t)in.C * (uint64_t)in.R >= (1ull << 32))
         fail(CR_INVALID, "cube larger than 2^32 samples");
     const cr_grid_info& gi = g->info;
-    if (gi.oversampling > kMaxTapRows - 1) fail(CR_INVALID, "cube oversampling above 512");
+    if (gi.oversampling > kMaxTapRows - 1) fail(CR_INVALID, "cube oversampling above 254");
     CubeRecords cr{};
     cr.R = in.R;
     cr.C = in.C;
@@ -1333,9 +1410,9 @@ static void launch_cube_grid(cr_ctx* ctx, cr_gridder* g, const CubeRecords& cr, 
     const cr_grid_info& gi = g->info;
     unsigned int* counter = (unsigned int*)workspace(ctx, "cube_counter", 8);
     CR_CUDA_CHECK(cudaMemsetAsync(counter, 0, 8, ctx->stream));
-    CubeGridArgs a{cr.rec, cr.rec_w, cr.bin_start, cr.cell_end, g->taps_d, g->tap_rows,
-                   g->taps_bytes, ctx->status_d, cr.ntx, cr.nty, gi.grid_nx, gi.grid_ny,
-                   cr.grid_items, cr.grid_chunk, cr.grid_chunks, cr.n_items, counter, psf,
+    CubeGridArgs a{cr.rec, cr.rec_w, cr.bin_start, cr.cell_end, g->taps8_d, g->tap_rows,
+                   (uint32_t)g->tap_rows * 32u, ctx->status_d, cr.ntx, cr.nty, gi.grid_nx,
+                   gi.grid_ny, cr.grid_items, cr.grid_chunk, cr.grid_chunks, cr.n_items, counter, psf,
                    dirty, res, ctx->mbar_polls};
     int sms = 0;
     CR_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
