@@ -113,26 +113,22 @@ __global__ void cube_rows_df_kernel(const double* u, const double* v, int64_t R,
 }
 
 // The density cell (x, y) of x = s_x p_x + e_x + nx/2 (valid when 1 <= x <
-// nx, likewise y) on the float32-pair path; false when undecided.
+// nx, likewise y) on the float32-pair path; false when undecided.  The cell
+// of (-u, -v) is then (nx - x, ny - y), and valid with it.
 __device__ __forceinline__ bool df_density_cell(float px, float ex, float py, float ey,
                                                 int32_t nx, int32_t ny, int* x, int* y,
                                                 bool* ok) {
-    float ax, ay, dh;
+    int ax, ay;
+    float dh;
     if (!df_nearest(px, ex, (nx & 1) ? 0.5f : 0.0f, &ax, &dh) ||
         !df_nearest(py, ey, (ny & 1) ? 0.5f : 0.0f, &ay, &dh))
         return false;
-    const int cx = (nx >> 1) + (int)ax, cy = (ny >> 1) + (int)ay;
+    const int cx = (nx >> 1) + ax, cy = (ny >> 1) + ay;
     *ok = !(cx <= 0 || cy <= 0 || cx >= nx || cy >= ny);
     *x = cx;
     *y = cy;
     return true;
 }
-
-// Both density cells of a sample, of (u, v) and of the mirror (-u, -v),
-// from one pair of fixed-point products (FP64 fallback per cell).
-__device__ __forceinline__ void density_cells(const CubeArgs& a, const CubeChan& ch, double um,
-                                              double vm, int* x, int* y, bool* ok, int* xm,
-                                              int* ym, bool* okm);
 
 // weight_density_cell_anchor with the cube (rounded) conventions.
 __device__ __forceinline__ bool density_cell(const CubeArgs& a, const CubeChan& ch, double um,
@@ -164,33 +160,43 @@ __device__ __forceinline__ bool density_cell(const CubeArgs& a, const CubeChan& 
     return true;
 }
 
-__device__ __forceinline__ void density_cells(const CubeArgs& a, const CubeChan& ch, double um,
-                                              double vm, int* x, int* y, bool* ok, int* xm,
-                                              int* ym, bool* okm) {
+// Both density cells of row r at channel c, of (u, v) and of the mirror
+// (-u, -v), from one pair of fixed-point products (FP64 fallback per cell):
+// what the float32-pair path leaves undecided.  Out of line, so that the
+// common path stays short in the instruction cache.
+struct DensityCells {
+    int x, y, xm, ym;
+    bool ok, okm;
+};
+__device__ __noinline__ DensityCells density_cells(const CubeArgs& a, int c, int64_t r) {
+    const CubeChan& ch = a.ch[c];
+    const double um = a.u[r], vm = a.v[r];
+    DensityCells d{0, 0, 0, 0, false, false};
     long long tx, ty;
     if (fix_mul(um, ch.kdx, &tx) && fix_mul(vm, ch.kdy, &ty)) {
         long long ax, ay;
         // (u, v): x = u s + c, y = -v s + c; mirror: x = -u s + c, y = v s + c
         if (fix_round(tx + a.dcx_fix, kFixMargin, &ax) &&
             fix_round(a.dcy_fix - ty, kFixMargin, &ay)) {
-            *ok = !(ax <= 0 || ay <= 0 || ax >= a.nx || ay >= a.ny);
-            *x = (int)ax;
-            *y = (int)ay;
+            d.ok = !(ax <= 0 || ay <= 0 || ax >= a.nx || ay >= a.ny);
+            d.x = (int)ax;
+            d.y = (int)ay;
         } else {
-            *ok = density_cell(a, ch, um, vm, false, x, y);
+            d.ok = density_cell(a, ch, um, vm, false, &d.x, &d.y);
         }
         if (fix_round(a.dcx_fix - tx, kFixMargin, &ax) &&
             fix_round(a.dcy_fix + ty, kFixMargin, &ay)) {
-            *okm = !(ax <= 0 || ay <= 0 || ax >= a.nx || ay >= a.ny);
-            *xm = (int)ax;
-            *ym = (int)ay;
+            d.okm = !(ax <= 0 || ay <= 0 || ax >= a.nx || ay >= a.ny);
+            d.xm = (int)ax;
+            d.ym = (int)ay;
         } else {
-            *okm = density_cell(a, ch, um, vm, true, xm, ym);
+            d.okm = density_cell(a, ch, um, vm, true, &d.xm, &d.ym);
         }
-        return;
+        return d;
     }
-    *ok = density_cell(a, ch, um, vm, false, x, y);
-    *okm = density_cell(a, ch, um, vm, true, xm, ym);
+    d.ok = density_cell(a, ch, um, vm, false, &d.x, &d.y);
+    d.okm = density_cell(a, ch, um, vm, true, &d.xm, &d.ym);
+    return d;
 }
 
 __device__ __forceinline__ bool finite_f(float x) { return isfinite(x); }
@@ -202,37 +208,74 @@ struct Eval {
     float w;
 };
 
-// sample_tap_span of row r at channel ch: the home tile and meta = start cell
-// in the tile | tap rows; float32 pairs first, then the integer path, then
-// the reference's FP64 operations.  False when the sample does not grid.
-__device__ __forceinline__ bool plan_sample(const CubeArgs& a, const CubeChan& ch, float4 uv,
-                                            int64_t r, uint32_t* tile, uint32_t* meta) {
+// sample_tap_span of a row of a channel: the home tile and meta = start cell
+// in the tile | tap rows.
+__device__ __forceinline__ void pack_sample(const CubeArgs& a, int32_t x0, int32_t y0, int32_t rx,
+                                            int32_t ry, uint32_t* tile, uint32_t* meta) {
+    *tile = (uint32_t)(x0 >> 5) * (uint32_t)a.nty + (uint32_t)(y0 >> 5);
+    *meta = (uint32_t)(x0 & 31) << 27 | (uint32_t)(y0 & 31) << 22 | (uint32_t)rx << 11 |
+            (uint32_t)ry;
+}
+
+// What the float32 pairs leave undecided: the integer path, then the
+// reference's FP64 operations.
+struct PlannedSample {
+    bool ok;
+    uint32_t tile, meta;
+};
+__device__ __noinline__ PlannedSample plan_sample_exact(const CubeArgs& a, int c, int64_t r) {
+    const CubeChan& ch = a.ch[c];
+    const double um = a.u[r], vm = a.v[r];
+    PlannedSample out{false, 0u, 0u};
     int64_t x0 = 0, y0 = 0;
     int32_t rx = 0, ry = 0;
-    // x = u K_x + G/2, y = -v K_y + G/2
-    float px, ex, py, ey;
-    df_product(uv.x, uv.y, ch.fx, &px, &ex);
-    df_product(-uv.z, -uv.w, ch.fy, &py, &ey);
-    int sx = df_tap_span(px, ex, a.gnx, a.os, a.tap_rows, &x0, &rx);
-    int sy = sx == 0 ? 0 : df_tap_span(py, ey, a.gny, a.os, a.tap_rows, &y0, &ry);
-    if (sx == 0 || sy == 0) return false;
+    int sx = -1, sy = -1;
     long long tx, ty;
-    if ((sx < 0 || sy < 0) && fix_mul(a.u[r], ch.kx, &tx) && fix_mul(a.v[r], ch.ky, &ty)) {
+    // x = u K_x + G/2, y = -v K_y + G/2
+    if (fix_mul(um, ch.kx, &tx) && fix_mul(vm, ch.ky, &ty)) {
         sx = fix_tap_span(tx + a.cx_fix, a.gnx, a.os, a.tap_rows, &x0, &rx);
         if (sx != 0) sy = fix_tap_span(a.cy_fix - ty, a.gny, a.os, a.tap_rows, &y0, &ry);
-        if (sx == 0 || sy == 0) return false;
+        if (sx == 0 || sy == 0) return out;
     }
     if (sx < 0 || sy < 0) {
-        const double u = __dmul_rn(a.u[r], ch.lscale), v = __dmul_rn(a.v[r], ch.lscale);
+        const double u = __dmul_rn(um, ch.lscale), v = __dmul_rn(vm, ch.lscale);
         const double x = __dadd_rn(__ddiv_rn(u, a.du), (double)a.gnx / 2.0);
         const double y = __dadd_rn(__ddiv_rn(-v, a.dv), (double)a.gny / 2.0);
         if (!f64_tap_span(x, a.gnx, a.os, a.tap_rows, &x0, &rx) ||
             !f64_tap_span(y, a.gny, a.os, a.tap_rows, &y0, &ry))
-            return false;
+            return out;
     }
-    *tile = (uint32_t)((x0 >> 5) * a.nty + (y0 >> 5));
-    *meta = ((uint32_t)(x0 & 31) << 27) | ((uint32_t)(y0 & 31) << 22) | ((uint32_t)rx << 11) |
-            (uint32_t)ry;
+    out.ok = true;
+    pack_sample(a, (int32_t)x0, (int32_t)y0, rx, ry, &out.tile, &out.meta);
+    return out;
+}
+
+// The scales of a channel's float32-pair path.
+struct DfChan {
+    DfScale fx, fy, fdx, fdy;
+};
+__device__ __forceinline__ DfChan df_chan(const CubeArgs& a, int c) {
+    const CubeChan& ch = a.ch[c];
+    return DfChan{ch.fx, ch.fy, ch.fdx, ch.fdy};
+}
+
+// False when the sample does not grid.
+__device__ __forceinline__ bool plan_sample(const CubeArgs& a, const DfChan& ch, float4 uv, int c,
+                                            int64_t r, uint32_t* tile, uint32_t* meta) {
+    int32_t x0 = 0, y0 = 0, rx = 0, ry = 0;
+    float px, ex, py, ey;
+    df_product(uv.x, uv.y, ch.fx, &px, &ex);
+    df_product(-uv.z, -uv.w, ch.fy, &py, &ey);
+    const int sx = df_tap_span(px, ex, (int32_t)a.gnx, a.os, a.tap_rows, &x0, &rx);
+    const int sy = df_tap_span(py, ey, (int32_t)a.gny, a.os, a.tap_rows, &y0, &ry);
+    if (sx == 0 || sy == 0) return false;
+    if (sx < 0 || sy < 0) {
+        const PlannedSample p = plan_sample_exact(a, c, r);
+        *tile = p.tile;
+        *meta = p.meta;
+        return p.ok;
+    }
+    pack_sample(a, x0, y0, rx, ry, tile, meta);
     return true;
 }
 
@@ -246,7 +289,7 @@ constexpr int kVec = 4;
 constexpr int kWarpRows = 32 * kVec;
 
 // kVec samples of channel c: flags, reweighting, validity and taps.
-__device__ __forceinline__ void eval_samples(const CubeArgs& a, const CubeChan& ch, float f2,
+__device__ __forceinline__ void eval_samples(const CubeArgs& a, const DfChan& ch, float f2,
                                              int c, int64_t row0, int64_t r1,
                                              Eval (&e)[kVec]) {
     float w[kVec];
@@ -278,7 +321,7 @@ __device__ __forceinline__ void eval_samples(const CubeArgs& a, const CubeChan& 
                 int x, y;
                 d[j] = 0.0f;
                 const int64_t r = row0 + 32 * j;
-                if (live[j] && density_cell(a, ch, a.u[r], a.v[r], false, &x, &y))
+                if (live[j] && density_cell(a, a.ch[c], a.u[r], a.v[r], false, &x, &y))
                     d[j] = dens[(int64_t)x * a.ny + y];
             }
         }
@@ -295,7 +338,7 @@ __device__ __forceinline__ void eval_samples(const CubeArgs& a, const CubeChan& 
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
         if (!live[j] || !(finite_f(w[j]) && w[j] > 0.0f)) continue;
-        if (!plan_sample(a, ch, uv[j], row0 + 32 * j, &e[j].tile, &e[j].meta)) continue;
+        if (!plan_sample(a, ch, uv[j], c, row0 + 32 * j, &e[j].tile, &e[j].meta)) continue;
         e[j].ok = true;
         e[j].w = w[j];
     }
@@ -329,9 +372,9 @@ __device__ __forceinline__ int64_t cell_bin(int c, int64_t ntiles, uint32_t tile
 // complete, must also come out positive; the scatter gives a sample for
 // which it does not a null record, so the counts stay exact.
 template <bool DENSITY>
-__global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(CubeArgs a) {
+__global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(const __grid_constant__ CubeArgs a) {
     const int c = blockIdx.y;
-    const CubeChan ch = a.ch[c];
+    const DfChan ch = df_chan(a, c);
     const int64_t ntiles = a.ntx * a.nty;
     const int64_t r0 = (int64_t)blockIdx.x * kRowsPerBlock;
     const int64_t r1 = min(a.R, r0 + kRowsPerBlock);
@@ -360,21 +403,30 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(CubeArgs 
             if (DENSITY) {
                 uint32_t cell = ~0u;
                 if (live[j]) {
-                    int x = 0, y = 0, xm = 0, ym = 0;
-                    bool ok = false, okm = false;
+                    int x = 0, y = 0;
+                    bool ok = false;
                     // float32 pairs first: (u, v) -> x = u s_x + nx/2,
-                    // y = -v s_y + ny/2; the mirror negates both products
+                    // y = -v s_y + ny/2
                     float px, ex, py, ey;
                     df_product(uv[j].x, uv[j].y, ch.fdx, &px, &ex);
                     df_product(-uv[j].z, -uv[j].w, ch.fdy, &py, &ey);
-                    if (!df_density_cell(px, ex, py, ey, a.nx, a.ny, &x, &y, &ok) ||
-                        !df_density_cell(-px, -ex, -py, -ey, a.nx, a.ny, &xm, &ym, &okm))
-                        density_cells(a, ch, a.u[r], a.v[r], &x, &y, &ok, &xm, &ym, &okm);
-                    if (ok) {
-                        cell = (uint32_t)x * (uint32_t)a.ny + (uint32_t)y;
-                        if (pos) atomicAdd(&dens[cell], w[j]);
+                    if (df_density_cell(px, ex, py, ey, a.nx, a.ny, &x, &y, &ok)) {
+                        if (ok) {
+                            cell = (uint32_t)x * (uint32_t)a.ny + (uint32_t)y;
+                            if (pos) {
+                                atomicAdd(&dens[cell], w[j]);
+                                atomicAdd(&dens[(uint32_t)(a.nx - x) * (uint32_t)a.ny +
+                                                (uint32_t)(a.ny - y)], w[j]);
+                            }
+                        }
+                    } else {
+                        const DensityCells d = density_cells(a, c, r);
+                        if (d.ok) {
+                            cell = (uint32_t)d.x * (uint32_t)a.ny + (uint32_t)d.y;
+                            if (pos) atomicAdd(&dens[cell], w[j]);
+                        }
+                        if (d.okm && pos) atomicAdd(&dens[(int64_t)d.xm * a.ny + d.ym], w[j]);
                     }
-                    if (okm && pos) atomicAdd(&dens[(int64_t)xm * a.ny + ym], w[j]);
                 }
                 a.dcell[i] = cell;
                 own = cell != ~0u;
@@ -382,7 +434,7 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(CubeArgs 
             uint32_t tile = kUngriddedSample, meta = 0u;
             if (!live[j]) {
                 tile = kFlaggedSample;
-            } else if (pos && own && plan_sample(a, ch, uv[j], r, &tile, &meta)) {
+            } else if (pos && own && plan_sample(a, ch, uv[j], c, r, &tile, &meta)) {
                 atomicAdd(&a.hist[cell_bin(c, ntiles, tile, meta)], 1u);
             } else {
                 tile = kUngriddedSample;
@@ -1176,9 +1228,9 @@ __global__ void __launch_bounds__(kCubeThreads) cube_degrid_kernel(
 }
 
 // Per-sample plan of every channel (start cells, tap rows, imaging weight).
-__global__ void __launch_bounds__(kCubeThreads) cube_taps_kernel(CubeArgs a, CubeTaps t) {
+__global__ void __launch_bounds__(kCubeThreads) cube_taps_kernel(const __grid_constant__ CubeArgs a, CubeTaps t) {
     const int c = blockIdx.y;
-    const CubeChan ch = a.ch[c];
+    const DfChan ch = df_chan(a, c);
     const float f2 = a.mode == CR_WEIGHT_BRIGGS ? a.f2[c] : 0.0f;
     const int64_t r0 = (int64_t)blockIdx.x * kRowsPerBlock;
     const int64_t r1 = min(a.R, r0 + kRowsPerBlock);

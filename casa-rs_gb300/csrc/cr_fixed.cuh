@@ -116,15 +116,20 @@ __device__ __forceinline__ int fix_tap_span(long long X, int64_t size, int32_t o
 // a = ah + al (ah = RN32(a), al = RN32(a - ah), or df_split's truncated ah)
 // and K = kh + kl, both to about 2^-47 relative; the product a K is then p + e with p = RN(ah kh),
 // e = fma(ah, kh, -p) + ah kl + al kh (three FMAs), about 2^-44 |a K| from
-// the exact value.  A decision is taken only when the exact value lies more
-// than kDfMargin (in the decision's own units: cells for the anchor,
-// oversampled cells for the offset) from its boundaries.  With |x| < 2^20
-// the pair's error (below 2^-14 after the offset's scaling by os <= 512)
-// and the reference's own FP64 error (below 2^-38) are far inside the
-// margin, so the decision equals the FP64 one.  Otherwise (about one
-// decision in 2^11) the caller takes the integer path.
-constexpr float kDfMargin = 1.0f / 4096.0f;
-constexpr float kDfLimit = 1048576.0f;   // |p| < 2^20
+// the exact value.  A decision is taken only when that value lies further
+// from its boundaries than the pair, the float32 sums and the reference's own
+// FP64 operations can be off:
+//   * anchor (cells), |p| < 2^20: 2^-24 + 2^-25 (the rounding of d) + 2^-32,
+//     inside the margin of 2^-20;
+//   * offset (oversampled cells), os <= 254: 2^-18 (the rounding of a value
+//     below 128) + |p| os 2^-43, inside 2^-16 + |p| os 2^-41.
+// Then the decision equals the FP64 one; otherwise (about one sample in 2^14)
+// the caller takes the integer path or FP64.  A margin of 2^-12 for both sent
+// one sample in 300 there, and with it one warp in eleven.
+constexpr float kDfAnchorMargin = 0x1p-20f;
+constexpr float kDfOffsetMargin = 0x1p-16f;
+constexpr float kDfOffsetRel = 0x1p-41f;   // of |p| os
+constexpr float kDfLimit = 1048576.0f;     // |p| < 2^20
 
 struct DfScale {
     float hi, lo;
@@ -240,41 +245,67 @@ __device__ __forceinline__ float2 residual_value(float4 v, float2 w, float2 pred
     return make_float2(diff(v.x, v.y, pred.x), diff(v.z, v.w, pred.y));
 }
 
+// rintf(x) for |x| < 2^22, as a float32 and as an integer, by a sum whose
+// last bit is 1 (the conversion instructions run at a quarter of its rate).
+__device__ __forceinline__ float df_rint(float x, int* i) {
+    const float t = __fadd_rn(x, 12582912.0f);   // 1.5 * 2^23
+    *i = __float_as_int(t) - 0x4b400000;
+    return __fsub_rn(t, 12582912.0f);
+}
+
 // The integer a nearest to x = p + e + h (h = 0 or 1/2) and dh = RN(p + h) - a
-// (exact), or false when x is within the margin of a half-integer, is
-// large, or is not finite.
-__device__ __forceinline__ bool df_nearest(float p, float e, float h, float* a, float* dh) {
+// (exact; the rounding of p + h goes to e), or false when x is within the
+// margin of a half-integer, is large, or is not finite.
+__device__ __forceinline__ bool df_nearest(float p, float& e, float h, int* a, float* dh) {
     if (!(fabsf(p) < kDfLimit)) return false;
-    const float q = __fadd_rn(p, h);
-    const float r = rintf(q);
-    const float d = __fadd_rn(__fsub_rn(q, r), e);
-    if (!(fabsf(fabsf(d) - 0.5f) > kDfMargin)) return false;
-    float n = r;
-    if (d > 0.5f) n = r + 1.0f;
-    if (d < -0.5f) n = r - 1.0f;
+    float q = p;
+    if (h != 0.0f) {
+        q = __fadd_rn(p, h);
+        const float b = __fsub_rn(q, p);
+        e = __fadd_rn(e, __fadd_rn(__fsub_rn(p, __fsub_rn(q, b)), __fsub_rn(h, b)));
+    }
+    int n;
+    const float r = df_rint(q, &n);
+    float f = __fsub_rn(q, r);
+    const float d = __fadd_rn(f, e);
+    if (!(fabsf(__fsub_rn(fabsf(d), 0.5f)) > kDfAnchorMargin)) return false;
+    if (d > 0.5f) {
+        ++n;
+        f = __fsub_rn(f, 1.0f);
+    }
+    if (d < -0.5f) {
+        --n;
+        f = __fadd_rn(f, 1.0f);
+    }
     *a = n;
-    *dh = __fsub_rn(q, n);
+    *dh = f;
     return true;
+}
+
+// round((a - x) os) of an axis with dh, e from df_nearest: -(dh + e) os.
+// False within the margin of a half-integer.
+__device__ __forceinline__ bool df_offset(float p, float e, float dh, int32_t os, int* off) {
+    const float osf = (float)os;
+    const float v = -__fmaf_rn(dh, osf, __fmul_rn(e, osf));
+    const float o = df_rint(v, off);
+    return 0.5f - fabsf(__fsub_rn(v, o)) >
+           __fmaf_rn(__fmul_rn(fabsf(p), osf), kDfOffsetRel, kDfOffsetMargin);
 }
 
 // sample_tap_span of x = p + e + size / 2 (the grid coordinate): 1 =
 // accepted, 0 = rejected, -1 = undecided (take the integer path).
-__device__ __forceinline__ int df_tap_span(float p, float e, int64_t size, int32_t os,
-                                           int32_t rows, int64_t* start, int32_t* row) {
-    float a, dh;
+__device__ __forceinline__ int df_tap_span(float p, float e, int32_t size, int32_t os,
+                                           int32_t rows, int32_t* start, int32_t* row) {
+    int a, off;
+    float dh;
     if (!df_nearest(p, e, (size & 1) ? 0.5f : 0.0f, &a, &dh)) return -1;
-    // |a| < 2^20
-    const int64_t anchor = (size >> 1) + (int)a;
+    const int32_t anchor = (size >> 1) + a;   // |a| <= 2^20
     if (anchor - 3 < 0 || anchor + 3 >= size) return 0;
-    // offset round((anchor - x) os) = round(-(dh + e) os)
-    const float osf = (float)os;
-    const float v = -__fmaf_rn(dh, osf, __fmul_rn(e, osf));
-    const float o = rintf(v);
-    if (!(0.5f - fabsf(__fsub_rn(v, o)) > kDfMargin)) return -1;
-    const int64_t idx = (int)o + os / 2;
+    if (!df_offset(p, e, dh, os, &off)) return -1;
+    const int32_t idx = off + os / 2;
     if (idx < 0 || idx >= rows) return 0;
     *start = anchor - 3;
-    *row = (int32_t)idx;
+    *row = idx;
     return 1;
 }
 

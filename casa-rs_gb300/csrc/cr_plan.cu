@@ -192,18 +192,16 @@ __device__ __forceinline__ bool finite_d(double x) {
 // The anchor loc = round(x) and offset round((loc - x) s) of the grid
 // coordinate x = u / du + G/2 in float32 pairs (x - G/2 = p + e from one
 // pair product with 1/du): the decisions of cr_fixed.cuh's fast path, taken
-// only more than kDfMargin from their rounding boundaries, where they equal
+// only further than the margins from their rounding boundaries, where they equal
 // the reference's FP64 ones.  False when undecided.
 __device__ __forceinline__ bool df_wp_axis(float p, float e, int64_t size, int32_t s,
                                            int64_t* loc, int64_t* off) {
-    float a, dh;
-    if (!df_nearest(p, e, (size & 1) ? 0.5f : 0.0f, &a, &dh)) return false;
-    const float sf = (float)s;
-    const float v = -__fmaf_rn(dh, sf, __fmul_rn(e, sf));
-    const float o = rintf(v);
-    if (!(0.5f - fabsf(__fsub_rn(v, o)) > kDfMargin)) return false;
-    *loc = (size >> 1) + (int)a;
-    *off = (int)o;
+    float dh;
+    int a, o;
+    if (!df_nearest(p, e, (size & 1) ? 0.5f : 0.0f, &a, &dh) || !df_offset(p, e, dh, s, &o))
+        return false;
+    *loc = (size >> 1) + a;
+    *off = o;
     return true;
 }
 
@@ -455,8 +453,7 @@ __global__ void __launch_bounds__(256) std_plan_kernel(StdPlanArgs a) {
         bool ok = (!a.gridable || a.gridable[i]) && finite_f(wt) && wt > 0.0f && finite_f(f) &&
                   f > 0.0f;
         if (ok) {
-            int64_t x0 = 0, y0 = 0;
-            int32_t rx = 0, ry = 0;
+            int32_t x0 = 0, y0 = 0, rx = 0, ry = 0;
             // float32 pairs first (cr_fixed.cuh's decisions, 1 / 0 / -1 =
             // accepted / rejected / undecided), the FP64 operations otherwise
             const double u = a.u[i], v = a.v[i];
@@ -466,8 +463,8 @@ __global__ void __launch_bounds__(256) std_plan_kernel(StdPlanArgs a) {
                 float px, ex, py, ey;
                 df_product(uh, ul, a.kx, &px, &ex);
                 df_product(-vh, -vl, a.ky, &py, &ey);
-                dx = df_tap_span(px, ex, a.gnx, a.os, a.tap_rows, &x0, &rx);
-                if (dx == 1) dy = df_tap_span(py, ey, a.gny, a.os, a.tap_rows, &y0, &ry);
+                dx = df_tap_span(px, ex, (int32_t)a.gnx, a.os, a.tap_rows, &x0, &rx);
+                if (dx == 1) dy = df_tap_span(py, ey, (int32_t)a.gny, a.os, a.tap_rows, &y0, &ry);
             }
             if (dx == 0 || dy == 0) {
                 ok = false;
@@ -475,17 +472,17 @@ __global__ void __launch_bounds__(256) std_plan_kernel(StdPlanArgs a) {
                 const StdSpans d = std_spans_fp64(u, v, a.du, a.dv, a.gnx, a.gny, a.os,
                                                   a.tap_rows);
                 ok = d.ok;
-                x0 = d.x0;
-                y0 = d.y0;
+                x0 = (int32_t)d.x0;
+                y0 = (int32_t)d.y0;
                 rx = d.rx;
                 ry = d.ry;
             }
             if (ok) {
                 // the float32 product w f, as the reference sums it
                 s_norm.add(__fmul_rn(wt, f), 0.0f);
-                uint64_t tile = (uint64_t)(x0 >> 5) * (uint64_t)a.nty + (uint64_t)(y0 >> 5);
-                uint64_t cell = (uint64_t)(((x0 & 31) << 5) | (y0 & 31));
-                key = ((tile << 10 | cell) << 8 | (uint64_t)rx) << 8 | (uint64_t)ry;
+                const uint64_t tile = (uint64_t)(x0 >> 5) * (uint32_t)a.nty + (uint32_t)(y0 >> 5);
+                const uint32_t cell = (uint32_t)((x0 & 31) << 5 | (y0 & 31));
+                key = tile << 26 | (uint64_t)(cell << 16 | (uint32_t)rx << 8 | (uint32_t)ry);
             }
         }
         if (ok)
