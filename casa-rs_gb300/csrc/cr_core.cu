@@ -513,37 +513,64 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_pass_kernel(RadixPass a
     }
 }
 
-RadixSort radix_sort_begin(cr_ctx* ctx, int64_t n, int bits) {
+// bytes of the keys, of the values and of the words that one memset clears:
+// state, histograms, tickets, fail
+struct RadixBytes {
+    int passes;
+    int64_t tiles;
+    size_t keys, vals, state, rec, hist;
+    size_t cleared() const { return state + rec + hist + 64; }
+};
+
+static RadixBytes radix_bytes(int64_t n, int bits) {
+    RadixBytes b;
+    b.passes = (bits + 7) / 8;
+    const int64_t tile = kSortThreads * (n < kSortSmall ? kSortItemsSmall : kSortItems);
+    b.tiles = (n + tile - 1) / tile;
+    b.keys = (size_t)(n > 0 ? n : 1) * 8;
+    b.vals = ((size_t)(n > 0 ? n : 1) * 4 + 7) & ~size_t(7);
+    b.state = (size_t)b.tiles * kRadixBins * 8;
+    b.rec = (size_t)((n + kRecTile - 1) / kRecTile) * 8;
+    b.hist = (size_t)b.passes * kRadixBins * 4;
+    return b;
+}
+
+size_t radix_sort_bytes(int64_t n, int bits) {
+    const RadixBytes b = radix_bytes(n, bits);
+    return 2 * b.keys + 2 * b.vals + b.cleared();
+}
+
+RadixSort radix_sort_begin(cr_ctx* ctx, int64_t n, int bits, void* mem) {
+    const RadixBytes b = radix_bytes(n, bits);
     RadixSort s;
     s.n = n;
-    s.passes = (bits + 7) / 8;
-    const int64_t tile = kSortThreads * (n < kSortSmall ? kSortItemsSmall : kSortItems);
-    s.tiles = (n + tile - 1) / tile;
-    const size_t nn = (size_t)(n > 0 ? n : 1);
-    s.keys = (uint64_t*)workspace(ctx, "rec_keys", nn * 8);
-    workspace(ctx, "sort_keys_alt", nn * 8);
-    workspace(ctx, "rec_order", nn * 4);
-    workspace(ctx, "sort_vals_alt", nn * 4);
-    // one buffer, cleared by one memset: state, histograms, tickets, fail
-    const size_t rec_tiles = (size_t)((n + kRecTile - 1) / kRecTile);
-    const size_t state_b = (size_t)s.tiles * kRadixBins * 8, rec_b = rec_tiles * 8,
-                 hist_b = (size_t)s.passes * kRadixBins * 4;
-    const size_t bytes = state_b + rec_b + hist_b + 64;
-    char* w = (char*)workspace(ctx, "sort_state", bytes);
+    s.passes = b.passes;
+    s.tiles = b.tiles;
+    char* m = (char*)mem;
+    auto take = [&](const char* name, size_t bytes) {
+        if (!mem) return (char*)workspace(ctx, name, bytes);
+        char* p = m;
+        m += bytes;
+        return p;
+    };
+    s.keys = (uint64_t*)take("rec_keys", b.keys);
+    s.keys_alt = (uint64_t*)take("sort_keys_alt", b.keys);
+    s.vals[0] = (uint32_t*)take("rec_order", b.vals);
+    s.vals[1] = (uint32_t*)take("sort_vals_alt", b.vals);
+    char* w = take("sort_state", b.cleared());
     s.state = (unsigned long long*)w;
-    s.rec_state = (unsigned long long*)(w + state_b);
-    s.hist = (uint32_t*)(w + state_b + rec_b);
-    s.tickets = (uint32_t*)(w + state_b + rec_b + hist_b);   // at most 8 passes
+    s.rec_state = (unsigned long long*)(w + b.state);
+    s.hist = (uint32_t*)(w + b.state + b.rec);
+    s.tickets = (uint32_t*)(w + b.state + b.rec + b.hist);   // at most 8 passes
     s.rec_ticket = s.tickets + 8;
     s.fail = s.tickets + 9;
-    CR_CUDA_CHECK(cudaMemsetAsync(w, 0, bytes, ctx->stream));
+    CR_CUDA_CHECK(cudaMemsetAsync(w, 0, b.cleared(), ctx->stream));
     return s;
 }
 
 void radix_sort_run(cr_ctx* ctx, RadixSort& s) {
-    uint64_t* kbuf[2] = {s.keys, (uint64_t*)workspace(ctx, "sort_keys_alt", 16)};
-    uint32_t* vbuf[2] = {(uint32_t*)workspace(ctx, "rec_order", 16),
-                         (uint32_t*)workspace(ctx, "sort_vals_alt", 16)};
+    uint64_t* kbuf[2] = {s.keys, s.keys_alt};
+    uint32_t* vbuf[2] = {s.vals[0], s.vals[1]};
     const bool small = s.n < kSortSmall;
     auto kern = small ? radix_pass_kernel<kSortItemsSmall> : radix_pass_kernel<kSortItems>;
     const size_t smem = (size_t)kSortThreads * (small ? kSortItemsSmall : kSortItems) * 12;

@@ -28,8 +28,9 @@
 // cr_fixed.cuh with the FP64 operations as the fallback.  Gridding gives
 // every (channel, output tile) to one block, which takes the records of
 // the four home tiles whose 7 x 7 footprints reach it (contiguous ranges, by
-// the order of the cells), accumulates the tile in shared memory and writes it once with coalesced stores -- no memset and
-// no global atomics on the output grids.
+// the order of the cells), accumulates the tile in shared memory and writes
+// it once with coalesced stores -- no memset and no global atomics on the
+// output grids.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -64,7 +65,8 @@ struct CubeArgs {
     int32_t C;
     const double* u;
     const double* v;
-    const float4* uvdf;        // per row (u_hi, u_lo, v_hi, v_lo); NaN u_hi: exact path only
+    const float4* uvdf;        // per position (u_hi, u_lo, v_hi, v_lo); NaN u_hi: exact path only
+    const uint32_t* rows;      // the row at each position, or null (in order)
     const CubeChan* ch;
     const float2* vis;
     const float* weight;
@@ -89,18 +91,26 @@ struct CubeArgs {
     unsigned long long* counts;// [C][2]: gridded, skipped
     uint4* rec;                // {meta, c R + r, w vis.re, w vis.im}
     float* rec_w;
-    // per-sample results kept between the passes ([C][R])
+    // per-sample results kept between the passes ([C][R] by position)
     uint32_t* dcell;           // density cell x ny + y of (u, v), ~0 when none
     uint32_t* ev_tile;         // home tile, or kFlaggedSample / kUngriddedSample
     uint32_t* ev_meta;         // cell in tile | tap rows
 };
 
-// Rows' u, v as float32 pairs for the fast path.  Rows whose coordinates are
-// not finite, exceed 2^60 or are below 2^-60 (but not zero) get a NaN u_hi
-// and always take the integer path.
-__global__ void cube_rows_df_kernel(const double* u, const double* v, int64_t R, float4* out) {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < R;
-         r += (int64_t)gridDim.x * blockDim.x) {
+// Rows' u, v as float32 pairs for the fast path, in the order of the
+// positions (`order`, or the rows' own).  Rows whose coordinates are not
+// finite, exceed 2^60 or are below 2^-60 (but not zero) get a NaN u_hi and
+// always take the integer path.
+__global__ void cube_rows_df_kernel(const double* u, const double* v, int64_t R,
+                                    const uint32_t* order, uint32_t* rows, float4* out) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < R;
+         p += (int64_t)gridDim.x * blockDim.x) {
+        int64_t r = p;
+        if (order) {
+            // in range also after a sort that gave up
+            r = min((int64_t)order[p], R - 1);
+            rows[p] = (uint32_t)r;
+        }
         const double um = u[r], vm = v[r];
         const bool ok = isfinite(um) && isfinite(vm) && fabs(um) < 0x1p60 &&
                         fabs(vm) < 0x1p60 && (um == 0.0 || fabs(um) > 0x1p-60) &&
@@ -108,9 +118,58 @@ __global__ void cube_rows_df_kernel(const double* u, const double* v, int64_t R,
         const float uh = __double2float_rn(um), vh = __double2float_rn(vm);
         const float ul = __double2float_rn(__dsub_rn(um, (double)uh));
         const float vl = __double2float_rn(__dsub_rn(vm, (double)vh));
-        out[r] = ok ? make_float4(uh, ul, vh, vl) : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+        out[p] = ok ? make_float4(uh, ul, vh, vl)
+                    : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
     }
 }
+
+// The key that puts rows near each other in the uv plane together: the home
+// tile and cell of the row's point on the grid of the channel with the
+// finest cells (su, sv: cells per metre there).  Any order is correct.
+constexpr int kMaxKeyPasses = 5;
+__global__ void __launch_bounds__(256) cube_row_keys_kernel(const double* u, const double* v,
+                                                            int64_t R, double su, double sv,
+                                                            int32_t gnx, int32_t gny,
+                                                            uint32_t nty, KeyOut out) {
+    __shared__ uint32_t s_counts[kMaxKeyPasses * kRadixBins];
+    KeyCounts counts{s_counts};
+    counts.begin(out);
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < R;
+         r += (int64_t)gridDim.x * blockDim.x) {
+        // (max and min drop a NaN)
+        const float fx = fmaxf((float)(u[r] * su) + 0.5f * (float)gnx, 0.0f);
+        const float fy = fmaxf((float)(-v[r] * sv) + 0.5f * (float)gny, 0.0f);
+        const uint32_t x = (uint32_t)fminf(fx, (float)gnx - 1.0f);
+        const uint32_t y = (uint32_t)fminf(fy, (float)gny - 1.0f);
+        counts.put(out, r, (uint64_t)((x >> 5) * nty + (y >> 5)) << 10 | (x & 31u) << 5 |
+                               (y & 31u));
+    }
+    counts.end(out);
+}
+
+// Lanes of a warp in runs of equal neighbouring keys.
+struct LaneRuns {
+    unsigned heads;   // lanes at which a run starts
+    int start;        // the lane's own run's
+    __device__ __forceinline__ LaneRuns(uint32_t key, int lane) {
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+        heads = __ballot_sync(0xffffffffu, lane == 0 || key != prev);
+        start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    }
+    __device__ __forceinline__ int end(int lane) const {   // one past the run's last lane
+        const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+        return after ? lane + __ffs(after) : 32;
+    }
+    // the sum of v over the run, complete in its last lane
+    __device__ __forceinline__ float sum(float v, int lane) const {
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const float t = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane - d >= start) v += t;
+        }
+        return v;
+    }
+};
 
 // The density cell (x, y) of x = s_x p_x + e_x + nx/2 (valid when 1 <= x <
 // nx, likewise y) on the float32-pair path; false when undecided.  The cell
@@ -358,10 +417,11 @@ __device__ __forceinline__ uint32_t cell_order(uint32_t x, uint32_t y) {
                    : 26 * x + y + (x >= 26 ? kReachYEnd - kReachY : 0u);
 }
 
-__device__ __forceinline__ int64_t cell_bin(int c, int64_t ntiles, uint32_t tile,
-                                            uint32_t meta) {
-    return (((int64_t)c * ntiles + tile) << 10) | cell_order(meta >> 27, (meta >> 22) & 31u);
+// the bin of a channel (all bins of a cube fit 32 bits)
+__device__ __forceinline__ uint32_t cell_bin(uint32_t tile, uint32_t meta) {
+    return tile << 10 | cell_order(meta >> 27, (meta >> 22) & 31u);
 }
+constexpr uint32_t kNoCell = ~0u;   // no bin's and no density cell's index
 
 // Pass 1 over every sample: with DENSITY the weight density of both cells
 // (u, v) and (-u, -v) and the sample's own density cell; then its grid plan
@@ -371,8 +431,15 @@ __device__ __forceinline__ int64_t cell_bin(int c, int64_t ntiles, uint32_t tile
 // imaging weight w / d or w / (d f2 + 1), known only once every density is
 // complete, must also come out positive; the scatter gives a sample for
 // which it does not a null record, so the counts stay exact.
-template <bool DENSITY>
-__global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(const __grid_constant__ CubeArgs a) {
+// With SORTED, positions are rows in uv order (a.rows): the lanes of a warp
+// then share cells, and each run of equal cells adds once.  In row order a
+// warp's samples lie in different cells, and the kernel is bound by the
+// requests of its three adds a sample: 16 channels of 1.26 M rows 491 us
+// against 347 us in uv order.
+constexpr int kDensVec = 2;   // 4: 384 us
+template <bool DENSITY, bool SORTED>
+__global__ void __launch_bounds__(kCubeThreads, 5)
+cube_density_kernel(const __grid_constant__ CubeArgs a) {
     const int c = blockIdx.y;
     const DfChan ch = df_chan(a, c);
     const int64_t ntiles = a.ntx * a.nty;
@@ -380,28 +447,33 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(const __g
     const int64_t r1 = min(a.R, r0 + kRowsPerBlock);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* dens = DENSITY ? a.density + (int64_t)c * a.nx * a.ny : nullptr;
-    for (int64_t base = r0 + warp * kWarpRows; base < r1; base += kCubeThreads * kVec) {
-        float w[kVec];
-        float4 uv[kVec];
-        bool live[kVec];
+    for (int64_t base = r0 + warp * 32 * kDensVec; base < r1; base += kCubeThreads * kDensVec) {
+        float w[kDensVec];
+        float4 uv[kDensVec];
+        uint32_t row[kDensVec];
+        bool live[kDensVec];
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int64_t r = base + lane + 32 * j;
-            live[j] = r < r1;
-            const int64_t i = (int64_t)c * a.R + (live[j] ? r : 0);
-            if (live[j] && a.flags) live[j] = a.flags[i] == 0;
-            w[j] = a.weight ? a.weight[i] : 1.0f;
-            uv[j] = a.uvdf[live[j] ? r : 0];
+        for (int j = 0; j < kDensVec; ++j) {
+            const int64_t p = base + lane + 32 * j;
+            live[j] = p < r1;
+            row[j] = SORTED ? a.rows[live[j] ? p : r0] : (uint32_t)(live[j] ? p : r0);
+            uv[j] = a.uvdf[live[j] ? p : r0];
         }
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int64_t r = base + lane + 32 * j;
-            if (r >= r1) continue;
-            const int64_t i = (int64_t)c * a.R + r;
+        for (int j = 0; j < kDensVec; ++j) {
+            const int64_t i = (int64_t)c * a.R + row[j];
+            if (a.flags) live[j] = live[j] && a.flags[i] == 0;
+            w[j] = a.weight ? a.weight[i] : 1.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < kDensVec; ++j) {
+            const int64_t p = base + lane + 32 * j;
+            const int64_t i = (int64_t)c * a.R + p;
             const bool pos = finite_f(w[j]) && w[j] > 0.0f;
             bool own = true;
             if (DENSITY) {
-                uint32_t cell = ~0u;
+                uint32_t cell = kNoCell, mirror = kNoCell;
+                bool add = false;
                 if (live[j]) {
                     int x = 0, y = 0;
                     bool ok = false;
@@ -413,14 +485,11 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(const __g
                     if (df_density_cell(px, ex, py, ey, a.nx, a.ny, &x, &y, &ok)) {
                         if (ok) {
                             cell = (uint32_t)x * (uint32_t)a.ny + (uint32_t)y;
-                            if (pos) {
-                                atomicAdd(&dens[cell], w[j]);
-                                atomicAdd(&dens[(uint32_t)(a.nx - x) * (uint32_t)a.ny +
-                                                (uint32_t)(a.ny - y)], w[j]);
-                            }
+                            mirror = (uint32_t)(a.nx - x) * (uint32_t)a.ny + (uint32_t)(a.ny - y);
+                            add = pos;
                         }
                     } else {
-                        const DensityCells d = density_cells(a, c, r);
+                        const DensityCells d = density_cells(a, c, row[j]);
                         if (d.ok) {
                             cell = (uint32_t)d.x * (uint32_t)a.ny + (uint32_t)d.y;
                             if (pos) atomicAdd(&dens[cell], w[j]);
@@ -428,19 +497,39 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_density_kernel(const __g
                         if (d.okm && pos) atomicAdd(&dens[(int64_t)d.xm * a.ny + d.ym], w[j]);
                     }
                 }
-                a.dcell[i] = cell;
-                own = cell != ~0u;
+                if (SORTED) {
+                    const LaneRuns runs(add ? cell : kNoCell, lane);
+                    const float sum = runs.sum(add ? w[j] : 0.0f, lane);
+                    if (add && runs.end(lane) == lane + 1) {
+                        atomicAdd(&dens[cell], sum);
+                        atomicAdd(&dens[mirror], sum);
+                    }
+                } else if (add) {
+                    atomicAdd(&dens[cell], w[j]);
+                    atomicAdd(&dens[mirror], w[j]);
+                }
+                if (p < r1) a.dcell[i] = cell;
+                own = cell != kNoCell;
             }
             uint32_t tile = kUngriddedSample, meta = 0u;
-            if (!live[j]) {
+            if (!live[j])
                 tile = kFlaggedSample;
-            } else if (pos && own && plan_sample(a, ch, uv[j], c, r, &tile, &meta)) {
-                atomicAdd(&a.hist[cell_bin(c, ntiles, tile, meta)], 1u);
-            } else {
+            else if (!(pos && own && plan_sample(a, ch, uv[j], c, row[j], &tile, &meta)))
                 tile = kUngriddedSample;
+            const bool bin = tile < kUngriddedSample;
+            if (SORTED) {
+                const uint32_t b = bin ? cell_bin(tile, meta) : kNoCell;
+                const LaneRuns runs(b, lane);
+                if (bin && runs.start == lane)
+                    atomicAdd(&a.hist[((int64_t)c * ntiles << 10) + b],
+                              (uint32_t)(runs.end(lane) - lane));
+            } else if (bin) {
+                atomicAdd(&a.hist[((int64_t)c * ntiles << 10) + cell_bin(tile, meta)], 1u);
             }
-            a.ev_tile[i] = tile;
-            a.ev_meta[i] = meta;
+            if (p < r1) {
+                a.ev_tile[i] = tile;
+                a.ev_meta[i] = meta;
+            }
         }
     }
 }
@@ -532,9 +621,14 @@ __global__ void tile_starts_from_cells(const uint32_t* cell_start, int64_t nbins
 // weight and value, no sample index), which grids and degrids nothing.  The
 // channel's sum of weights and its gridded and unflagged-but-not-gridded
 // counts are summed here.
-constexpr int kScatterVec = 6;
+//
+// With SORTED the lanes of a warp share cells: a run of equal cells takes its
+// slots with one atomic and writes them side by side (16 channels of 1.26 M
+// rows: 310 us against 452 us in row order).
+constexpr int kScatterVec = 3;   // 6 at 4 blocks per SM: 324 us
 constexpr uint32_t kNullSample = ~0u;   // sample index of a null record
-__global__ void __launch_bounds__(kCubeThreads, 4) cube_scatter_kernel(CubeArgs a) {
+template <bool SORTED>
+__global__ void __launch_bounds__(kCubeThreads, 6) cube_scatter_kernel(CubeArgs a) {
     __shared__ double s_sum[kCubeThreads / 32];
     __shared__ unsigned long long s_ok[kCubeThreads / 32], s_skip[kCubeThreads / 32];
     const int c = blockIdx.y;
@@ -546,6 +640,7 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_scatter_kernel(CubeArgs 
     const float f2 = a.mode == CR_WEIGHT_BRIGGS ? a.f2[c] : 0.0f;
     const float* dens = a.mode != CR_WEIGHT_NATURAL ? a.density + (int64_t)c * a.nx * a.ny
                                                     : nullptr;
+    uint32_t* cursor = a.cursor + ((int64_t)c * ntiles << 10);
     // the channel's sum of weights as a float pair (no FP64 instruction per
     // sample), in FP64 from the warp sums on
     PairSum swp;
@@ -553,19 +648,21 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_scatter_kernel(CubeArgs 
     for (int64_t base = r0 + wp * 32 * kScatterVec; base < r1;
          base += kCubeThreads * kScatterVec) {
         // loads first, then every cursor atomic, then the stores: the kScatterVec
-        // atomics of a thread are in flight together.  (The samples of a
-        // warp -- consecutive rows of one channel, different baselines --
-        // almost never share a cell bin, so the atomics are not aggregated:
-        // a warp match cost more than it saved.)
-        uint32_t tile[kScatterVec], meta[kScatterVec], pos[kScatterVec];
+        // atomics of a thread are in flight together
+        uint32_t tile[kScatterVec], meta[kScatterVec], pos[kScatterVec], row[kScatterVec];
         float w[kScatterVec];
         float2 vv[kScatterVec];
 #pragma unroll
         for (int j = 0; j < kScatterVec; ++j) {
-            const int64_t r = base + lane + 32 * j;
-            const int64_t i = (int64_t)c * a.R + (r < r1 ? r : r0);
-            tile[j] = r < r1 ? a.ev_tile[i] : kFlaggedSample;
-            meta[j] = a.ev_meta[i];
+            const int64_t p = base + lane + 32 * j;
+            const int64_t q = p < r1 ? p : r0;
+            tile[j] = p < r1 ? a.ev_tile[(int64_t)c * a.R + q] : kFlaggedSample;
+            meta[j] = a.ev_meta[(int64_t)c * a.R + q];
+            row[j] = SORTED ? a.rows[q] : (uint32_t)q;
+        }
+#pragma unroll
+        for (int j = 0; j < kScatterVec; ++j) {
+            const int64_t i = (int64_t)c * a.R + row[j];
             w[j] = a.weight ? a.weight[i] : 1.0f;
             vv[j] = a.vis[i];
         }
@@ -586,11 +683,25 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_scatter_kernel(CubeArgs 
                 w[j] = nw;
             }
         }
+        int start[kScatterVec];
 #pragma unroll
         for (int j = 0; j < kScatterVec; ++j) {
+            const bool bin = tile[j] < kUngriddedSample;
+            const uint32_t b = bin ? cell_bin(tile[j], meta[j]) : kNoCell;
             pos[j] = 0u;
-            if (tile[j] < kUngriddedSample)
-                pos[j] = atomicAdd(&a.cursor[cell_bin(c, ntiles, tile[j], meta[j])], 1u);
+            if (SORTED) {
+                const LaneRuns runs(b, lane);
+                start[j] = runs.start;
+                if (bin && runs.start == lane)
+                    pos[j] = atomicAdd(&cursor[b], (uint32_t)(runs.end(lane) - lane));
+            } else if (bin) {
+                pos[j] = atomicAdd(&cursor[b], 1u);
+            }
+        }
+        if (SORTED) {
+#pragma unroll
+            for (int j = 0; j < kScatterVec; ++j)
+                pos[j] = __shfl_sync(0xffffffffu, pos[j], start[j]) + (uint32_t)(lane - start[j]);
         }
 #pragma unroll
         for (int j = 0; j < kScatterVec; ++j) {
@@ -598,7 +709,7 @@ __global__ void __launch_bounds__(kCubeThreads, 4) cube_scatter_kernel(CubeArgs 
             const bool ok = tile[j] != kUngriddedSample && finite_f(w[j]) && w[j] > 0.0f;
             if (!ok) ++n_skip;
             if (tile[j] == kUngriddedSample) continue;
-            const int64_t i = (int64_t)c * a.R + base + lane + 32 * j;
+            const int64_t i = (int64_t)c * a.R + row[j];
             float vr = 0.0f, vi = 0.0f, wr = 0.0f;
             uint32_t sample = kNullSample;
             if (ok) {
@@ -1228,7 +1339,8 @@ __global__ void __launch_bounds__(kCubeThreads) cube_degrid_kernel(
 }
 
 // Per-sample plan of every channel (start cells, tap rows, imaging weight).
-__global__ void __launch_bounds__(kCubeThreads) cube_taps_kernel(const __grid_constant__ CubeArgs a, CubeTaps t) {
+__global__ void __launch_bounds__(kCubeThreads) cube_taps_kernel(const __grid_constant__ CubeArgs a,
+                                                                 CubeTaps t) {
     const int c = blockIdx.y;
     const DfChan ch = df_chan(a, c);
     const float f2 = a.mode == CR_WEIGHT_BRIGGS ? a.f2[c] : 0.0f;
@@ -1284,6 +1396,16 @@ void cube_upload_channels(cr_ctx* ctx, cr_gridder* g, const CubeInput& in) {
                                   cudaMemcpyHostToDevice, ctx->stream));
     // the pageable source must outlive the copy
     CR_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+}
+
+// Rows are put in uv order when that pays: the sort costs some 35 us and
+// 60 ps a row once, and saves up to 25 ps a sample in every channel where
+// many rows share a cell.  Whole calls, in row order / in uv order: 1.26 M
+// rows of 256 channels 32.3 / 26.9 ms, of 16 2.27 / 2.11 ms, of 1 414 /
+// 505 us; 270,001 rows of 101 channels 3.65 / 3.53 ms; 262,144 rows of 48
+// 1.43 / 1.47 ms; 8 M rows of 4 3.78 / 3.75 ms; 50,000 rows of 64 626 / 668 us.
+static bool cube_rows_sorted(int64_t R, int32_t C) {
+    return C >= 8 && R >= (1 << 18) && R * C >= (1 << 24);
 }
 
 CubeRecords cube_plan(cr_ctx* ctx, cr_gridder* g, const CubeInput& in, int32_t mode,
@@ -1364,16 +1486,41 @@ CubeRecords cube_plan(cr_ctx* ctx, cr_gridder* g, const CubeInput& in, int32_t m
     const dim3 grid((unsigned)std::max<int64_t>((in.R + kRowsPerBlock - 1) / kRowsPerBlock, 1),
                     (unsigned)in.C);
     float4* uvdf = (float4*)workspace(ctx, "cube_uvdf", (size_t)std::max<int64_t>(in.R, 1) * 16);
+    a.ev_tile = (uint32_t*)workspace(ctx, "cube_ev_tile", ns * 4);
+    a.ev_meta = (uint32_t*)workspace(ctx, "cube_ev_meta", ns * 4);
+    // (a context with an allocation limit keeps the smaller scratch)
+    bool sorted = !taps && ctx->alloc_limit == 0 && cube_rows_sorted(in.R, in.C);
+    int bits = 10;
+    while (((uint64_t)cr.ntiles << 10) >> bits) ++bits;
+    // the sort works in the per-sample results' memory, which is not yet in use
+    sorted = sorted && radix_sort_bytes(in.R, bits) <= ns * 4;
+    const uint32_t* order = nullptr;
+    uint32_t* rows = nullptr;
+    if (sorted) {
+        rows = (uint32_t*)workspace(ctx, "cube_rows", (size_t)in.R * 4);
+        double s_max = 0.0;
+        for (int c = 0; c < in.C; ++c) s_max = std::max(s_max, in.lambda_scale[c]);
+        RadixSort sort = radix_sort_begin(ctx, in.R, bits, a.ev_tile);
+        const KeyOut out{sort.keys, sort.hist, sort.passes, nullptr};
+        cube_row_keys_kernel<<<grid_blocks(in.R, 256 * 8), 256, 0, ctx->stream>>>(
+            in.u, in.v, in.R, s_max / gi.du, s_max / gi.dv, (int32_t)gi.grid_nx,
+            (int32_t)gi.grid_ny, (uint32_t)cr.nty, out);
+        note_launch(ctx, "cube_row_keys_kernel");
+        radix_sort_run(ctx, sort);
+        order = sort.order;
+    }
     if (in.R > 0) {
-        cube_rows_df_kernel<<<grid_blocks(in.R, 256), 256, 0, ctx->stream>>>(in.u, in.v, in.R,
-                                                                             uvdf);
+        cube_rows_df_kernel<<<grid_blocks(in.R, 256), 256, 0, ctx->stream>>>(
+            in.u, in.v, in.R, order, rows, uvdf);
         note_launch(ctx, "cube_rows_df_kernel");
     }
     a.uvdf = uvdf;
-    a.ev_tile = (uint32_t*)workspace(ctx, "cube_ev_tile", ns * 4);
-    a.ev_meta = (uint32_t*)workspace(ctx, "cube_ev_meta", ns * 4);
+    a.rows = rows;
     if (mode == CR_WEIGHT_NATURAL && in.R > 0) {
-        cube_density_kernel<false><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+        if (sorted)
+            cube_density_kernel<false, true><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+        else
+            cube_density_kernel<false, false><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
         note_launch(ctx, "cube_plan_kernel");
     }
     if (mode != CR_WEIGHT_NATURAL) {
@@ -1382,7 +1529,10 @@ CubeRecords cube_plan(cr_ctx* ctx, cr_gridder* g, const CubeInput& in, int32_t m
         a.dcell = (uint32_t*)workspace(ctx, "cube_dcell", ns * 4);
         CR_CUDA_CHECK(cudaMemsetAsync(a.density, 0, (size_t)(in.C * cells) * 4, ctx->stream));
         if (in.R > 0) {
-            cube_density_kernel<true><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+            if (sorted)
+                cube_density_kernel<true, true><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+            else
+                cube_density_kernel<true, false><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
             note_launch(ctx, "cube_density_kernel");
         }
         float* f2 = (float*)workspace(ctx, "cube_f2", (size_t)in.C * 4);
@@ -1411,7 +1561,10 @@ CubeRecords cube_plan(cr_ctx* ctx, cr_gridder* g, const CubeInput& in, int32_t m
                                                                                  cr.bin_start);
     note_launch(ctx, "tile_starts_from_cells");
     if (in.R > 0) {
-        cube_scatter_kernel<<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+        if (sorted)
+            cube_scatter_kernel<true><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
+        else
+            cube_scatter_kernel<false><<<grid, kCubeThreads, 0, ctx->stream>>>(a);
         note_launch(ctx, "cube_scatter_kernel");
     }
     // work-list buffers (the lists are made by cube_grid / cube_degrid)
@@ -1464,8 +1617,8 @@ static void launch_cube_grid(cr_ctx* ctx, cr_gridder* g, const CubeRecords& cr, 
     CR_CUDA_CHECK(cudaMemsetAsync(counter, 0, 8, ctx->stream));
     CubeGridArgs a{cr.rec, cr.rec_w, cr.bin_start, cr.cell_end, g->taps8_d, g->tap_rows,
                    (uint32_t)g->tap_rows * 32u, ctx->status_d, cr.ntx, cr.nty, gi.grid_nx,
-                   gi.grid_ny, cr.grid_items, cr.grid_chunk, cr.grid_chunks, cr.n_items, counter, psf,
-                   dirty, res, ctx->mbar_polls};
+                   gi.grid_ny, cr.grid_items, cr.grid_chunk, cr.grid_chunks, cr.n_items,
+                   counter, psf, dirty, res, ctx->mbar_polls};
     int sms = 0;
     CR_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     int per_sm = 0;

@@ -235,6 +235,8 @@ struct RadixSort {
     unsigned int* fail = nullptr;
     unsigned long long* state = nullptr;  // [tiles][256]
     uint64_t* keys = nullptr;             // unsorted keys are written here
+    uint64_t* keys_alt = nullptr;
+    uint32_t* vals[2] = {nullptr, nullptr};
     const uint64_t* sorted_keys = nullptr;
     const uint32_t* order = nullptr;      // index of each sorted item
     // for the pass over the sorted keys that follows: one ticket and a word
@@ -244,8 +246,43 @@ struct RadixSort {
 };
 constexpr int kRadixBins = 256;
 constexpr int kRecTile = 1024;
-RadixSort radix_sort_begin(cr_ctx* ctx, int64_t n, int bits);
+// `mem`: memory of radix_sort_bytes(n, bits) to work in, or null (workspaces)
+size_t radix_sort_bytes(int64_t n, int bits);
+RadixSort radix_sort_begin(cr_ctx* ctx, int64_t n, int bits, void* mem = nullptr);
 void radix_sort_run(cr_ctx* ctx, RadixSort& s);
+
+// Where a plan kernel puts the keys: the key of each sample, the digit counts
+// of the sort's passes, and -1 as the record of a skipped sample.
+struct KeyOut {
+    uint64_t* keys;
+    uint32_t* hist;        // [passes][256]
+    int passes;
+    int32_t* sample_rec;   // or null
+};
+
+// The digits of a block's keys counted in shared memory, added to the global
+// counts once per block.
+struct KeyCounts {
+    uint32_t* s;           // [passes][256] in shared memory
+    __device__ void begin(const KeyOut& o) {
+        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x) s[k] = 0;
+        __syncthreads();
+    }
+    __device__ void put(const KeyOut& o, int64_t i, uint64_t key) {
+        o.keys[i] = key;
+        if (o.sample_rec && key == ~0ull) o.sample_rec[i] = -1;
+        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+            if (p < o.passes)
+                atomicAdd(&s[p * kRadixBins + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
+    }
+    __device__ void end(const KeyOut& o) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x)
+            if (s[k]) atomicAdd(&o.hist[k], s[k]);
+    }
+};
 
 // ---- batch upload ------------------------------------------------------------
 struct DeviceBatch {

@@ -34,39 +34,6 @@ __host__ __device__ inline int bits_for(uint64_t max_value) {
     return b;
 }
 
-// Where a plan kernel puts the keys: the key of each sample, the digit counts
-// of the sort's passes, and -1 as the record of a skipped sample.
-struct KeyOut {
-    uint64_t* keys;
-    uint32_t* hist;        // [passes][256]
-    int passes;
-    int32_t* sample_rec;   // or null
-};
-
-// The digits of a block's keys counted in shared memory, added to the global
-// counts once per block.
-struct KeyCounts {
-    uint32_t* s;           // [passes][256] in shared memory
-    __device__ void begin(const KeyOut& o) {
-        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x) s[k] = 0;
-        __syncthreads();
-    }
-    __device__ void put(const KeyOut& o, int64_t i, uint64_t key) {
-        o.keys[i] = key;
-        if (o.sample_rec && key == ~0ull) o.sample_rec[i] = -1;
-        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
-#pragma unroll
-        for (int p = 0; p < 8; ++p)
-            if (p < o.passes)
-                atomicAdd(&s[p * kRadixBins + (((p < 4 ? lo : hi) >> (8 * (p & 3))) & 255u)], 1u);
-    }
-    __device__ void end(const KeyOut& o) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < o.passes * kRadixBins; k += blockDim.x)
-            if (s[k]) atomicAdd(&o.hist[k], s[k]);
-    }
-};
-
 struct WpPlanArgs {
     int64_t first, n;   // samples [first, n)
     const double *u, *v, *w;
