@@ -1179,9 +1179,15 @@ struct CubeDegridArgs {
 };
 
 // Bins in turn.  The block stages the 38 x 38 model footprint of its home
-// tile in shared memory; a warp takes 4 records at a time, 7 lanes per
-// record, lane ix forming wx[ix] * sum_iy wy[iy] g[x0 + ix][y0 + iy]
-// (float32), and the 7 lanes' sums are reduced with shuffles.
+// tile in shared memory.  Records follow the cell order, so the 7 x 7 cells
+// of a record are mostly those of the one before: a group of four lanes takes
+// a record, lane ix holding rows 2 ix and 2 ix + 1 of the cells in registers
+// until the cell changes, and a record costs it the tap rows and
+// sum_ix wx[ix] sum_iy wy[iy] g[x0 + ix][y0 + iy] in paired FMAs.  The lanes'
+// sums of four records are exchanged at once, and each lane writes its own.
+// (Seven shared-memory loads of cells a lane and record had the load/store
+// unit 91 % busy: 16 channels of 1.26 M rows 432 us, 223 us this way; eight
+// lanes a record, one row each, 235 us; four blocks per SM spill, 299 us.)
 // With RESIDUAL each record's w vis - w pred goes to res (record order)
 // instead of pred (sample order).
 // With TMA the footprints come as tensor-map boxes (float32 view
@@ -1190,10 +1196,10 @@ struct CubeDegridArgs {
 // already in flight.  Without TMA (a grid whose rows are not a multiple of
 // 16 bytes, or an unaligned base) the block loads each footprint itself.
 // The tap table arrives by one bulk copy in either case, its rows padded to
-// 8 floats so that a record's 7 y taps come in two 16-byte loads (the
-// kernel is bound by shared-memory instructions).
+// 8 floats so that a record's 7 y taps come in two 16-byte loads.
+constexpr int kDegridBlocks = 3;
 template <bool RESIDUAL, bool TMA>
-__global__ void __launch_bounds__(kCubeThreads) cube_degrid_kernel(
+__global__ void __launch_bounds__(kCubeThreads, kDegridBlocks) cube_degrid_kernel(
     const __grid_constant__ CUtensorMap gmap, CubeDegridArgs a) {
     constexpr int kFoot = kTile + 6;
     constexpr int kPitch = TMA ? kFoot : kRow;   // float2 per footprint row
@@ -1204,9 +1210,12 @@ __global__ void __launch_bounds__(kCubeThreads) cube_degrid_kernel(
     __shared__ __align__(128) float2 s_g[kBufs][kBufElems];
     __shared__ __align__(8) uint64_t s_bar[3];   // footprint buffers 0, 1; taps
     __shared__ int s_item[2];
+    // a warp's batch: cell in the footprint, x and y tap rows
+    __shared__ __align__(16) int4 s_rec[kCubeThreads];
     extern __shared__ __align__(16) float s_taps[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int sub = lane >> 3, ix = lane & 7;   // record slot, tap column (7 = idle)
+    const int sub = lane >> 2, ix = lane & 3;   // group of lanes, its pair of footprint rows
+    int4* w_rec = s_rec + warp * 32;
     const unsigned long long n_items = *a.n_items;
     // thread 0: the footprint of `item` into buffer `buf`
     auto issue = [&](int item, int buf) {
@@ -1282,54 +1291,99 @@ __global__ void __launch_bounds__(kCubeThreads) cube_degrid_kernel(
             }
             __syncthreads();
         }
-        // each record is loaded one iteration ahead of its use, so a warp
-        // keeps the next batch's loads in flight while it computes
+        // each warp takes a contiguous share of the item's records
+        const uint32_t n = hi - lo, share = (n + kCubeThreads - 1) / kCubeThreads * 32u;
+        const uint32_t w0 = lo + min(n, warp * share), w1 = lo + min(n, (warp + 1) * share);
+        // this lane's two rows of the 7 x 7 cells at `held`, two columns to a pair
+        float2 row_re[2][4], row_im[2][4];
+        int held = -1;
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            row_re[t >> 2][t & 3] = row_im[t >> 2][t & 3] = make_float2(0.0f, 0.0f);
+        // records are loaded a batch ahead of their use, one per lane
         uint4 qn = make_uint4(0u, 0u, 0u, 0u);
         float wn = 0.0f;
-        if (lo + warp * 4 + sub < hi) {
-            qn = a.rec[lo + warp * 4 + sub];
-            if (RESIDUAL) wn = a.rec_w[lo + warp * 4 + sub];
+        if (w0 + lane < w1) {
+            qn = a.rec[w0 + lane];
+            if (RESIDUAL) wn = a.rec_w[w0 + lane];
         }
-        for (uint32_t base = lo + warp * 4; base < hi; base += kCubeThreads / 8) {
-            const uint32_t k = base + sub;
+#pragma unroll 1
+        for (uint32_t base = w0; base < w1; base += 32) {
+            const uint32_t k = base + lane;
             const uint4 q = qn;
             const float w = wn;
-            if (k + kCubeThreads / 8 < hi) {
-                qn = a.rec[k + kCubeThreads / 8];
-                if (RESIDUAL) wn = a.rec_w[k + kCubeThreads / 8];
+            __syncwarp();
+            w_rec[lane] = make_int4((int)(q.x >> 27) * kPitch + (int)((q.x >> 22) & 31u),
+                                    (int)((q.x >> 11) & 2047u) * 8, (int)(q.x & 2047u) * 8, 0);
+            __syncwarp();
+            if (k + 32 < w1) {
+                qn = a.rec[k + 32];
+                if (RESIDUAL) wn = a.rec_w[k + 32];
             }
-            float2 acc = make_float2(0.0f, 0.0f);   // (re, im), paired FMAs
-            uint32_t sample = 0;
-            if (k < hi) {
-                sample = q.y;
-                if (ix < 7) {
-                    const uint32_t meta = q.x;
-                    const float wxi = s_taps[((meta >> 11) & 2047u) * 8 + ix];
-                    const float4* wy4 = reinterpret_cast<const float4*>(s_taps) +
-                                        (meta & 2047u) * 2;
-                    const float4 ya = wy4[0], yb = wy4[1];
-                    const float wy[7] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z};
-                    const int row =
-                        ((int)(meta >> 27) + ix) * kPitch + (int)((meta >> 22) & 31);
+            float re[4], im[4];
 #pragma unroll
-                    for (int iy = 0; iy < 7; ++iy) {
-                        const float wgt = __fmul_rn(wxi, wy[iy]);
-                        acc = __ffma2_rn(sg[row + iy], make_float2(wgt, wgt), acc);
+            for (int j = 0; j < 4; ++j) {
+                const int4 A = w_rec[j * 8 + sub];
+                if (A.x != held) {
+                    held = A.x;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (2 * ix + h < 7) {
+                            const float2* cell = sg + held + (2 * ix + h) * kPitch;
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+                                const float2 g0 = cell[2 * t];
+                                const float2 g1 =
+                                    t < 3 ? cell[2 * t + 1] : make_float2(0.0f, 0.0f);
+                                row_re[h][t] = make_float2(g0.x, g1.x);
+                                row_im[h][t] = make_float2(g0.y, g1.y);
+                            }
+                        }
                     }
                 }
-            }
-            float re = acc.x, im = acc.y;
+                const float2 wx = *reinterpret_cast<const float2*>(s_taps + A.y + 2 * ix);
+                const float4* wy = reinterpret_cast<const float4*>(s_taps + A.z);
+                const float4 y0 = wy[0], y1 = wy[1];
+                const float2 y[4] = {make_float2(y0.x, y0.y), make_float2(y0.z, y0.w),
+                                     make_float2(y1.x, y1.y), make_float2(y1.z, y1.w)};
+                float2 r[2], i[2];
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {
-                re += __shfl_xor_sync(0xffffffffu, re, o);
-                im += __shfl_xor_sync(0xffffffffu, im, o);
+                for (int h = 0; h < 2; ++h) {
+                    r[h] = __fmul2_rn(row_re[h][0], y[0]);
+                    i[h] = __fmul2_rn(row_im[h][0], y[0]);
+#pragma unroll
+                    for (int t = 1; t < 4; ++t) {
+                        r[h] = __ffma2_rn(row_re[h][t], y[t], r[h]);
+                        i[h] = __ffma2_rn(row_im[h][t], y[t], i[h]);
+                    }
+                }
+                re[j] = __fmaf_rn(__fadd_rn(r[1].x, r[1].y), wx.y,
+                                  __fmul_rn(__fadd_rn(r[0].x, r[0].y), wx.x));
+                im[j] = __fmaf_rn(__fadd_rn(i[1].x, i[1].y), wx.y,
+                                  __fmul_rn(__fadd_rn(i[0].x, i[0].y), wx.x));
             }
-            if (ix == 0 && k < hi) {
+            // the rows' sums: lane ix of group `sub` ends with record 8 ix + sub,
+            // which then goes to its own lane
+#pragma unroll
+            for (int o = 2; o > 0; o >>= 1) {
+                const bool up = ix & o;
+#pragma unroll
+                for (int t = 0; t < o; ++t) {
+                    re[t] = (up ? re[t + o] : re[t]) +
+                            __shfl_xor_sync(0xffffffffu, up ? re[t] : re[t + o], o);
+                    im[t] = (up ? im[t + o] : im[t]) +
+                            __shfl_xor_sync(0xffffffffu, up ? im[t] : im[t + o], o);
+                }
+            }
+            const int from = 4 * (lane & 7) + (lane >> 3);
+            re[0] = __shfl_sync(0xffffffffu, re[0], from);
+            im[0] = __shfl_sync(0xffffffffu, im[0], from);
+            if (k < w1) {
                 if (RESIDUAL) {
-                    a.res[k] = make_float2(__fsub_rn(__uint_as_float(q.z), __fmul_rn(w, re)),
-                                           __fsub_rn(__uint_as_float(q.w), __fmul_rn(w, im)));
-                } else if (sample != kNullSample) {
-                    a.pred[sample] = make_float2(re, im);
+                    a.res[k] = make_float2(__fsub_rn(__uint_as_float(q.z), __fmul_rn(w, re[0])),
+                                           __fsub_rn(__uint_as_float(q.w), __fmul_rn(w, im[0])));
+                } else if (q.y != kNullSample) {
+                    a.pred[q.y] = make_float2(re[0], im[0]);
                 }
             }
         }
@@ -1693,10 +1747,10 @@ static void launch_cube_degrid(cr_ctx* ctx, cr_gridder* g, const CubeRecords& cr
                                           row * (uint64_t)gi.grid_nx, 2 * (kTile + 6), kTile + 6);
     if (tma)
         cube_degrid_kernel<RESIDUAL, true>
-            <<<sms * 8, kCubeThreads, taps8_bytes, ctx->stream>>>(map, a);
+            <<<sms * kDegridBlocks, kCubeThreads, taps8_bytes, ctx->stream>>>(map, a);
     else
         cube_degrid_kernel<RESIDUAL, false>
-            <<<sms * 8, kCubeThreads, taps8_bytes, ctx->stream>>>(map, a);
+            <<<sms * kDegridBlocks, kCubeThreads, taps8_bytes, ctx->stream>>>(map, a);
     note_launch(ctx, RESIDUAL ? "cube_degrid_kernel_residual" : "cube_degrid_kernel");
 }
 
