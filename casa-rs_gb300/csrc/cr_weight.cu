@@ -13,6 +13,7 @@
 // weighting.rs:2440-2443).
 #include <cmath>
 
+#include "cr_fixed.cuh"
 #include "cr_internal.cuh"
 
 namespace cr {
@@ -25,6 +26,18 @@ struct DensityCellParams {
     int32_t convention;          // 0 VisImagingWeight, 1 cube PerPlane (rounded, FP64)
     double du_scale, dv_scale, dcx, dcy;
 };
+
+// the VisImagingWeight cell of (u, v) with tx = u u_scale, ty = v v_scale
+__device__ __forceinline__ bool float_cell(const DensityCellParams& p, float tx, float ty, int* ox,
+                                           int* oy) {
+    const float x = __fadd_rn(-tx, p.cx), y = __fadd_rn(ty, p.cy);
+    if (!(isfinite(x) && isfinite(y))) return false;
+    // trunc(x) in (0, nx) <=> 1 <= x < nx
+    if (!(x >= 1.0f && x < (float)p.nx && y >= 1.0f && y < (float)p.ny)) return false;
+    *ox = (int)x;
+    *oy = (int)y;
+    return true;
+}
 
 __device__ __forceinline__ bool density_cell(const DensityCellParams& p, double u, double v,
                                              int* ox, int* oy) {
@@ -39,45 +52,77 @@ __device__ __forceinline__ bool density_cell(const DensityCellParams& p, double 
         *oy = (int)ry;
         return true;
     }
-    float uf = __double2float_rn(u), vf = __double2float_rn(v);
-    float x = __fadd_rn(__fmul_rn(-uf, p.u_scale), p.cx);
-    float y = __fadd_rn(__fmul_rn(vf, p.v_scale), p.cy);
-    if (!(isfinite(x) && isfinite(y))) return false;
-    // trunc(x) in (0, nx) <=> 1 <= x < nx
-    if (!(x >= 1.0f && x < (float)p.nx && y >= 1.0f && y < (float)p.ny)) return false;
-    *ox = (int)x;
-    *oy = (int)y;
-    return true;
+    return float_cell(p, __fmul_rn(d2f(u), p.u_scale), __fmul_rn(d2f(v), p.v_scale), ox, oy);
 }
 
-__global__ void density_kernel(const double* u, const double* v, const float* weight, int64_t n,
-                               DensityCellParams p, float* density) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        float w = weight[i];
-        if (!(isfinite(w) && w > 0.0f)) continue;
-        int x, y;
-        if (density_cell(p, u[i], v[i], &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w);
-        if (density_cell(p, -u[i], -v[i], &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w);
+// Four samples a thread, so that their loads and adds are in flight together;
+// the float32 coordinates come from the bits (the FP64 pipe converted four
+// doubles a sample), and the mirror's are the negated ones.
+constexpr int kDensityVec = 4;
+__global__ void __launch_bounds__(256) density_kernel(const double* u, const double* v,
+                                                      const float* weight, int64_t n,
+                                                      DensityCellParams p, float* density) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < n;
+         base += step * kDensityVec) {
+        float w[kDensityVec];
+        double us[kDensityVec], vs[kDensityVec];
+#pragma unroll
+        for (int j = 0; j < kDensityVec; ++j) {
+            const int64_t i = base + j * step;
+            w[j] = i < n ? weight[i] : 0.0f;
+            us[j] = i < n ? u[i] : 0.0;
+            vs[j] = i < n ? v[i] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < kDensityVec; ++j) {
+            if (!(isfinite(w[j]) && w[j] > 0.0f)) continue;
+            int x, y;
+            if (p.convention == 1) {
+                if (density_cell(p, us[j], vs[j], &x, &y))
+                    atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
+                if (density_cell(p, -us[j], -vs[j], &x, &y))
+                    atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
+                continue;
+            }
+            const float tx = __fmul_rn(d2f(us[j]), p.u_scale);
+            const float ty = __fmul_rn(d2f(vs[j]), p.v_scale);
+            if (float_cell(p, tx, ty, &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
+            if (float_cell(p, -tx, -ty, &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
+        }
     }
 }
 
-__global__ void density_sums_kernel(const float* d, int64_t n, double* sums) {
+// sum d and sum d^2 (d > 0) in FP64: one pair of adds a block (a pair a warp,
+// 78,000 adds to two words, took most of 123 us for 2048^2), the conversions
+// from the bits
+__global__ void __launch_bounds__(256) density_sums_kernel(const float* d, int64_t n,
+                                                           double* sums) {
     double s = 0.0, s2 = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        double v = (double)d[i];
+        const float f = d[i];
+        if (f == 0.0f) continue;
+        const double v = f2d(f);
         s += v;
         if (v > 0.0) s2 += v * v;
     }
+    __shared__ double sh[2][8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&sums[0], s);
-        atomicAdd(&sums[1], s2);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        sh[0][warp] = s;
+        sh[1][warp] = s2;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int k = 0; k < 8; ++k) t += sh[threadIdx.x][k];
+        atomicAdd(&sums[threadIdx.x], t);
     }
 }
 
@@ -134,14 +179,14 @@ void apply_weighting(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, int32_t m
         if (b.n > 0) {
             // the density is built at build_u, build_v when given (the row
             // path's VisImagingWeight coordinates), looked up at u, v
-            density_kernel<<<grid_blocks(b.n, 256), 256, 0, ctx->stream>>>(
+            density_kernel<<<grid_blocks(b.n, 256 * kDensityVec), 256, 0, ctx->stream>>>(
                 build_u ? build_u : b.u, build_v ? build_v : b.v, b.weight, b.n, p, density);
             note_launch(ctx, "density_kernel");
         }
         if (mode == CR_WEIGHT_BRIGGS) {
             double* sums = (double*)workspace(ctx, "wt_sums", 16);
             CR_CUDA_CHECK(cudaMemsetAsync(sums, 0, 16, ctx->stream));
-            density_sums_kernel<<<grid_blocks((int64_t)nx * ny, 256), 256, 0, ctx->stream>>>(
+            density_sums_kernel<<<grid_blocks((int64_t)nx * ny, 256, 152 * 8), 256, 0, ctx->stream>>>(
                 density, (int64_t)nx * ny, sums);
             note_launch(ctx, "density_sums_kernel");
             double h[2];
