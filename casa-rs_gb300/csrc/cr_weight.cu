@@ -55,40 +55,97 @@ __device__ __forceinline__ bool density_cell(const DensityCellParams& p, double 
     return float_cell(p, __fmul_rn(d2f(u), p.u_scale), __fmul_rn(d2f(v), p.v_scale), ox, oy);
 }
 
-// Four samples a thread, so that their loads and adds are in flight together;
-// the float32 coordinates come from the bits (the FP64 pipe converted four
-// doubles a sample), and the mirror's are the negated ones.
-constexpr int kDensityVec = 4;
-__global__ void __launch_bounds__(256) density_kernel(const double* u, const double* v,
-                                                      const float* weight, int64_t n,
-                                                      DensityCellParams p, float* density) {
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < n;
-         base += step * kDensityVec) {
+// the cells of (u, v) and of (-u, -v)
+__device__ __forceinline__ void density_cells(const DensityCellParams& p, double u, double v,
+                                              int* x, int* y, bool* ok, int* xm, int* ym,
+                                              bool* okm) {
+    if (p.convention == 1) {
+        *ok = density_cell(p, u, v, x, y);
+        *okm = density_cell(p, -u, -v, xm, ym);
+        return;
+    }
+    const float tx = __fmul_rn(d2f(u), p.u_scale), ty = __fmul_rn(d2f(v), p.v_scale);
+    *ok = float_cell(p, tx, ty, x, y);
+    *okm = float_cell(p, -tx, -ty, xm, ym);
+}
+
+// A block takes contiguous samples, four to a thread at a time (their loads
+// are in flight together; the float32 coordinates come from the bits, since
+// the FP64 pipe converted four doubles a sample).
+//
+// With TABLE the block first collects its samples by cell in a hashed table
+// in shared memory.  Samples are mostly in time order, and successive times
+// of one baseline share a cell: added one by one, the few cells of the
+// shortest baselines take tens of thousands of adds each, which memory works
+// off one after the other.  A cell's mirror is as a rule the cell reflected,
+// so one entry stands for both; a sample for which rounding or the edge makes
+// it another, or whose slot another cell holds, is added directly.
+// With / without the table: 10.1 M samples on 2048^2 62 / 316 us, 1.05 M on
+// 512^2 14.0 / 26.7 us, 250,001 on 2048^2 9.8 / 15.8 us, 60,001 on 256^2
+// 8.6 / 6.8 us.
+constexpr int kDensityVec = 4, kDensityThreads = 512, kDensityBlocks = 2;
+constexpr int kSlotBits = 13, kSlots = 1 << kSlotBits;
+constexpr uint32_t kEmptySlot = ~0u;
+constexpr int64_t kTableSamples = 1 << 17;
+
+template <bool TABLE>
+__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks)
+density_kernel(const double* u, const double* v, const float* weight, int64_t n,
+               DensityCellParams p, float* density) {
+    extern __shared__ uint32_t s_cell[];   // [kSlots], then their sums
+    float* s_sum = reinterpret_cast<float*>(s_cell + kSlots);
+    if (TABLE) {
+        for (int k = threadIdx.x; k < kSlots; k += kDensityThreads) {
+            s_cell[k] = kEmptySlot;
+            s_sum[k] = 0.0f;
+        }
+        __syncthreads();
+    }
+    const int mx = p.convention == 1 ? p.nx : p.nx - 1, my = p.convention == 1 ? p.ny : p.ny - 1;
+    const int64_t share = (n + gridDim.x - 1) / gridDim.x;
+    const int64_t end = min(n, (blockIdx.x + 1) * share);
+    for (int64_t base = blockIdx.x * share + threadIdx.x; base < end;
+         base += kDensityThreads * kDensityVec) {
         float w[kDensityVec];
         double us[kDensityVec], vs[kDensityVec];
 #pragma unroll
         for (int j = 0; j < kDensityVec; ++j) {
-            const int64_t i = base + j * step;
-            w[j] = i < n ? weight[i] : 0.0f;
-            us[j] = i < n ? u[i] : 0.0;
-            vs[j] = i < n ? v[i] : 0.0;
+            const int64_t i = base + kDensityThreads * j;
+            w[j] = i < end ? weight[i] : 0.0f;
+            us[j] = i < end ? u[i] : 0.0;
+            vs[j] = i < end ? v[i] : 0.0;
         }
 #pragma unroll
         for (int j = 0; j < kDensityVec; ++j) {
             if (!(isfinite(w[j]) && w[j] > 0.0f)) continue;
-            int x, y;
-            if (p.convention == 1) {
-                if (density_cell(p, us[j], vs[j], &x, &y))
-                    atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
-                if (density_cell(p, -us[j], -vs[j], &x, &y))
-                    atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
-                continue;
+            int x = 0, y = 0, xm = 0, ym = 0;
+            bool ok, okm;
+            density_cells(p, us[j], vs[j], &x, &y, &ok, &xm, &ym, &okm);
+            const uint32_t cell = (uint32_t)x * (uint32_t)p.ny + (uint32_t)y;
+            if (TABLE && ok && okm && xm == mx - x && ym == my - y) {
+                const uint32_t slot = (cell * 2654435761u) >> (32 - kSlotBits);
+                uint32_t held = *(volatile uint32_t*)&s_cell[slot];
+                if (held == kEmptySlot) {
+                    held = atomicCAS(&s_cell[slot], kEmptySlot, cell);
+                    if (held == kEmptySlot) held = cell;
+                }
+                if (held == cell) {
+                    atomicAdd(&s_sum[slot], w[j]);
+                    continue;
+                }
             }
-            const float tx = __fmul_rn(d2f(us[j]), p.u_scale);
-            const float ty = __fmul_rn(d2f(vs[j]), p.v_scale);
-            if (float_cell(p, tx, ty, &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
-            if (float_cell(p, -tx, -ty, &x, &y)) atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
+            if (ok) atomicAdd(&density[cell], w[j]);
+            if (okm) atomicAdd(&density[(int64_t)xm * p.ny + ym], w[j]);
+        }
+    }
+    if (TABLE) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < kSlots; k += kDensityThreads) {
+            const uint32_t cell = s_cell[k];
+            if (cell == kEmptySlot) continue;
+            const uint32_t x = cell / (uint32_t)p.ny, y = cell % (uint32_t)p.ny;
+            atomicAdd(&density[cell], s_sum[k]);
+            atomicAdd(&density[((uint32_t)mx - x) * (uint32_t)p.ny + ((uint32_t)my - y)], s_sum[k]);
         }
     }
 }
@@ -179,8 +236,15 @@ void apply_weighting(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, int32_t m
         if (b.n > 0) {
             // the density is built at build_u, build_v when given (the row
             // path's VisImagingWeight coordinates), looked up at u, v
-            density_kernel<<<grid_blocks(b.n, 256 * kDensityVec), 256, 0, ctx->stream>>>(
-                build_u ? build_u : b.u, build_v ? build_v : b.v, b.weight, b.n, p, density);
+            const bool table = b.n >= kTableSamples;
+            auto kern = table ? density_kernel<true> : density_kernel<false>;
+            const size_t smem = table ? (size_t)kSlots * 8 : 0;
+            CR_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem));
+            kern<<<grid_blocks(b.n, kDensityThreads * kDensityVec, 152 * kDensityBlocks),
+                   kDensityThreads, smem, ctx->stream>>>(build_u ? build_u : b.u,
+                                                         build_v ? build_v : b.v, b.weight, b.n,
+                                                         p, density);
             note_launch(ctx, "density_kernel");
         }
         if (mode == CR_WEIGHT_BRIGGS) {
