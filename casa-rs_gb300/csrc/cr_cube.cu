@@ -38,6 +38,7 @@
 
 #include "cr_fixed.cuh"
 #include "cr_internal.cuh"
+#include "cr_runs.cuh"
 #include "cr_tma.cuh"
 
 namespace cr {
@@ -874,16 +875,10 @@ struct CubeGridArgs {
 //
 // The kernel is bound by instruction issue (some 18 M records of 49 taps on a
 // 16-channel batch of 1.26 M rows), so records are summed by runs of one start
-// cell.  A warp's four groups of eight lanes take a record each: lane ix of a
-// group holds row ix of the 7 x 7 footprint, its columns as four pairs per
-// component, and a record costs the group one x tap, two 16-byte loads of y
-// taps and twelve paired FMAs.  A vote over the records' cells ends a run:
-// the groups' sums are then exchanged so that each lane holds two columns,
-// and added to the tile.  A float32 add to shared memory is a
-// compare-and-swap loop that the hardware serialises by lane, so re and im
-// share one 64-bit swap.  Records are decoded by a lane each, 32 ahead of
-// their use; warp 0 fetches the next item's ranges before the tile is
-// written; the tile is zeroed as it is read out.
+// cell, four at a time (cr_runs.cuh).  A vote over the records' cells ends a
+// run, whose sums are added to the tile.  Records are decoded by a lane each,
+// 32 ahead of their use; warp 0 fetches the next item's ranges before the tile
+// is written; the tile is zeroed as it is read out.
 //
 // Four warps per block: an item has some 600 records, and every warp more
 // cuts its runs once more (256 threads: 6 % slower; 96 and 64 lose occupancy
@@ -945,24 +940,10 @@ __device__ __forceinline__ void next_item(const CubeGridArgs& a, int lane, GridI
     }
 }
 
-// (re, im) += (x, y) in shared memory, one 64-bit compare-and-swap per try
-__device__ __forceinline__ void shared_add2(float2* p, float x, float y) {
-    unsigned long long* q = reinterpret_cast<unsigned long long*>(p);
-    unsigned long long old = *q, seen;
-    do {
-        seen = old;
-        const float re = __uint_as_float((uint32_t)seen) + x;
-        const float im = __uint_as_float((uint32_t)(seen >> 32)) + y;
-        old = atomicCAS(q, seen,
-                        (unsigned long long)__float_as_uint(im) << 32 | __float_as_uint(re));
-    } while (old != seen);
-}
-
 template <bool RESIDUAL>
 __global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(CubeGridArgs a) {
     constexpr int kPlane = kTile * kRow, kComps = RESIDUAL ? 2 : 3;
     constexpr int kWarps = kGridThreads / 32;
-    constexpr int kAcc = 4 * kComps;   // a lane's sums in pairs: component x 8 columns
     constexpr uint32_t kDone = ~0u;
     __shared__ __align__(16) float s_taps[kTapFloats];
     __shared__ float s_psf[RESIDUAL ? 1 : kPlane];
@@ -997,34 +978,15 @@ __global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(Cu
     float2* w_rb = s_rb + warp * 32;
     const int g = lane >> 3, ix = lane & 7;
     const float* tap_x = s_taps + ix;
-    float2 acc[kAcc];
-    auto clear = [&]() {
-#pragma unroll
-        for (int q = 0; q < kAcc; ++q) acc[q] = make_float2(0.0f, 0.0f);
-    };
+    RunSums<kComps> sums;
     for (int buf = 0;; buf ^= 1) {
         __syncthreads();
         const GridItem& it = s_items[buf];
         if (it.count < 0) break;
-        // the groups' sums of the run at cell (x, y) of the tile, exchanged so
-        // that group q holds columns 2 q and 2 q + 1 of each row, into the tile
+        // the sums of the run at cell (x, y) of the tile into the tile
         auto flush = [&](int x, int y) {
-            const bool hi = lane & 16, hi2 = lane & 8;
             float n[kComps][2];
-#pragma unroll
-            for (int c = 0; c < kComps; ++c) {
-                float m[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float2 p0 = acc[4 * c + (t >> 1)], p1 = acc[4 * c + 2 + (t >> 1)];
-                    const float f0 = (t & 1) ? p0.y : p0.x, f1 = (t & 1) ? p1.y : p1.x;
-                    m[t] = (hi ? f1 : f0) + __shfl_xor_sync(0xffffffffu, hi ? f0 : f1, 16);
-                }
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-                    n[c][t] = (hi2 ? m[t + 2] : m[t]) +
-                              __shfl_xor_sync(0xffffffffu, hi2 ? m[t] : m[t + 2], 8);
-            }
+            sums.exchange(lane, n);
             const bool row = ix < 7 && (unsigned)(x + ix) < kTile;
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
@@ -1043,7 +1005,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(Cu
         const uint32_t w1 = it.first + min(n, (warp + 1) * share);
         int open_x = 0, open_y = 0;
         bool any = false;
-        clear();
+        sums.clear();
 #pragma unroll 1
         for (int s = 0; s < 4; ++s) {
             const uint32_t lo = max(w0, it.off[s]), hi = min(w1, it.off[s + 1]);
@@ -1087,30 +1049,13 @@ __global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(Cu
                     uint32_t cell = (uint32_t)A.x;
                     const float wq = __int_as_float(A.w);
                     const float wx = tap_x[A.y];
-                    const float4* wy = reinterpret_cast<const float4*>(s_taps + A.z);
-                    const float4 y0 = wy[0], y1 = wy[1];
-                    const float2 y[4] = {make_float2(y0.x, y0.y), make_float2(y0.z, y0.w),
-                                         make_float2(y1.x, y1.y), make_float2(y1.z, y1.w)};
+                    float2 y[4];
+                    tap_pairs(s_taps + A.z, y);
                     for (;;) {
                         const bool mine = cell == open;
                         const unsigned match = __ballot_sync(0xffffffffu, mine);
                         if (match) {
-                            int c = 0;
-                            if (!RESIDUAL) {
-                                const float p = mine ? __fmul_rn(wx, wq) : 0.0f;
-#pragma unroll
-                                for (int q = 0; q < 4; ++q)
-                                    acc[q] = __ffma2_rn(make_float2(p, p), y[q], acc[q]);
-                                c = 4;
-                            }
-                            const float p = mine ? __fmul_rn(wx, B.x) : 0.0f;
-                            const float q2 = mine ? __fmul_rn(wx, B.y) : 0.0f;
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                acc[c + q] = __ffma2_rn(make_float2(p, p), y[q], acc[c + q]);
-                                acc[c + 4 + q] =
-                                    __ffma2_rn(make_float2(q2, q2), y[q], acc[c + 4 + q]);
-                            }
+                            sums.add(mine, wx, y, wq, B);
                             if (match == 0xffffffffu) break;
                             if (mine) cell = kDone;
                         }
@@ -1118,7 +1063,7 @@ __global__ void __launch_bounds__(kGridThreads, kGridBlocks) cube_grid_kernel(Cu
                         if (!rest) break;
                         if (any) {
                             flush(open_x, open_y);
-                            clear();
+                            sums.clear();
                         }
                         any = true;
                         open = __shfl_sync(0xffffffffu, cell, __ffs(rest) - 1);

@@ -3,14 +3,15 @@
 //
 // Gridding restates grid_sample_taps_real_complex_pair_planned_f64
 // (gridder.rs:1021-1071): PSF += gw * wx*wy and dirty += vis*gw * wx*wy, the
-// tap product wx*wy rounded in float32.  A warp sums the taps of consecutive
-// records with one start cell in registers and adds them once per run to the
-// home tile's 38 x 38 footprint in shared memory, which is flushed to the grid
-// with FP32 atomics.
+// value times wx rounded in float32 before wy.  A warp sums the taps of
+// consecutive records with one start cell in registers and adds them once per
+// run to the home tile's 38 x 38 footprint in shared memory, which is flushed to
+// the grid with FP32 atomics.
 // Degridding restates degrid_sample_taps_planned_normalized
 // (gridder.rs:1278-1312) with a warp per record.
 #include "cr_fixed.cuh"
 #include "cr_internal.cuh"
+#include "cr_runs.cuh"
 
 namespace cr {
 
@@ -18,11 +19,11 @@ namespace {
 
 constexpr int kStdThreads = 256;
 constexpr int kFoot = kTile + 6;   // 38
-// footprint rows 39 floats apart (= 7 mod 32): the 49 taps of a record hit
-// distinct banks within each warp-wide atomic
+// footprint rows 39 cells apart (= 7 mod 32), so that the seven rows of a
+// footprint fall in different banks
 constexpr int kFootRow = 39;
-constexpr int kStdMaxTaps = 255 * 7;   // oversampling up to 254
-constexpr int kStdBlocksPerSm = 6;
+constexpr int kStdMaxTaps = 255 * 8;   // oversampling up to 254
+constexpr int kStdBlocksPerSm = 4;
 // Work is measured in records, a home tile's flush counting as kStdTileCost
 // of them: tile T's records lie at positions tile_start[T] + kStdTileCost T
 // onwards.  An item is a range of positions, found by a search over the
@@ -50,20 +51,23 @@ struct StdGridArgs {
     int64_t gnx, gny;
 };
 
-// Bound by the issue of the per-record work (two tap slots per lane) and by
-// shared-memory atomics per run.  With one atomic per tap and record, chunks of
-// 2048 records of one tile and a work list: 68 us for 4,001 samples of a 256^2
-// image, 137 for 126,360 (512^2), 511 for 5.0 M (3000^2); now 16, 18 and 265.
+// Bound by the issue of the per-record work and, for small batches, by its
+// latency.  Records are summed by runs of one start cell, four at a time
+// (cr_runs.cuh).  4,001 samples of a 256^2 image, 126,360 (512^2) and 5.0 M
+// (3000^2): 18, 17 and 140 us; with a lane per tap, and a shared-memory add
+// per tap and run, 16, 18 and 261; with one add per tap and record, chunks of
+// 2048 records of one tile and a work list, 68, 137 and 511.
 template <bool RESIDUAL>
-__global__ void __launch_bounds__(kStdThreads) std_grid_kernel(StdGridArgs a) {
+__global__ void __launch_bounds__(kStdThreads, kStdBlocksPerSm) std_grid_kernel(StdGridArgs a) {
     __shared__ float s_psf[RESIDUAL ? 1 : kFoot * kFootRow];
-    __shared__ float s_dr[kFoot * kFootRow];
-    __shared__ float s_di[kFoot * kFootRow];
-    __shared__ float s_taps[kStdMaxTaps];
-    // per warp, 32 decoded records: {start cell, tap row offsets, weight}
-    // and the value
-    __shared__ int4 s_ra[kStdThreads];
+    __shared__ __align__(8) float2 s_ri[kFoot * kFootRow];
+    __shared__ __align__(16) float s_taps[kStdMaxTaps];
+    // per warp, 32 decoded records: {cell of the tile, tap row offsets,
+    // weight} and the value
+    __shared__ __align__(16) int4 s_ra[kStdThreads];
     __shared__ float2 s_rb[kStdThreads];
+    constexpr int kComps = RESIDUAL ? 2 : 3;
+    constexpr uint32_t kDone = ~0u;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t nrec = (int64_t)a.counts[2];
     const int64_t span = nrec + kStdTileCost * a.ntiles;
@@ -74,16 +78,12 @@ __global__ void __launch_bounds__(kStdThreads) std_grid_kernel(StdGridArgs a) {
     for (int k = tid; k < a.tap_floats; k += kStdThreads) s_taps[k] = a.taps[k];
     for (int c = tid; c < kFoot * kFootRow; c += kStdThreads) {
         if (!RESIDUAL) s_psf[c] = 0.0f;
-        s_dr[c] = 0.0f;
-        s_di[c] = 0.0f;
+        s_ri[c] = make_float2(0.0f, 0.0f);
     }
     __syncthreads();
-    // lane t holds taps t (slot 0) and t + 32 (slot 1, lanes 0-16; the other
-    // lanes form a dummy product that is never added)
-    const int ix0 = lane / 7, iy0 = lane % 7;
-    const bool has1 = lane + 32 < 49;
-    const int ix1 = has1 ? (lane + 32) / 7 : 0, iy1 = has1 ? (lane + 32) % 7 : 0;
-    const int off0 = ix0 * kFootRow + iy0, off1 = ix1 * kFootRow + iy1;
+    const int grp = lane >> 3, ix = lane & 7;
+    const float* tap_x = s_taps + ix;
+    RunSums<kComps> sums;
     int4* w_ra = s_ra + warp * 32;
     float2* w_rb = s_rb + warp * 32;
     for (int64_t v0 = blockIdx.x * item; v0 < span; v0 += gridDim.x * item) {
@@ -106,63 +106,78 @@ __global__ void __launch_bounds__(kStdThreads) std_grid_kernel(StdGridArgs a) {
             const int64_t e = min((int64_t)a.tile_start[T + 1], v1 - kStdTileCost * T);
             if (e <= s) break;   // the tile begins past the item's end
             const bool more = e == a.tile_start[T + 1];
-            bool open = false;   // a run is being summed
-            int cx = 0, cy = 0;
-            // (psf slot 0, slot 1), (re, im) slot 0, (re, im) slot 1
-            float2 pp = make_float2(0.f, 0.f), ri0 = pp, ri1 = pp;
+            // each warp takes a contiguous share of the tile's records
+            const uint32_t n = (uint32_t)(e - s), kWarps = kStdThreads / 32;
+            const uint32_t share = max(32u, (n + 4 * kWarps - 1) / (4 * kWarps) * 4u);
+            const uint32_t w0 = (uint32_t)s + min(n, warp * share);
+            const uint32_t w1 = (uint32_t)s + min(n, (warp + 1) * share);
+            uint32_t open = kDone - 1;   // the run's cell; none yet
             auto flush = [&]() {
-                const int b = (cx - x0) * kFootRow + (cy - y0);
-                if (!RESIDUAL) atomicAdd(&s_psf[b + off0], pp.x);
-                atomicAdd(&s_dr[b + off0], ri0.x);
-                atomicAdd(&s_di[b + off0], ri0.y);
-                if (has1) {
-                    if (!RESIDUAL) atomicAdd(&s_psf[b + off1], pp.y);
-                    atomicAdd(&s_dr[b + off1], ri1.x);
-                    atomicAdd(&s_di[b + off1], ri1.y);
+                float v[kComps][2];
+                sums.exchange(lane, v);
+                const int c = ((open >> 5) + ix) * kFootRow + (open & 31u) + 2 * grp;
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (ix < 7 && 2 * grp + t < 7) {
+                        if (!RESIDUAL) atomicAdd(&s_psf[c + t], v[0][t]);
+                        shared_add2(&s_ri[c + t], v[kComps - 2][t], v[kComps - 1][t]);
+                    }
                 }
             };
-            for (int64_t g = s + warp * 32; g < e; g += kStdThreads) {
-                const int64_t r = g + lane;
-                if (r < e) {
+            sums.clear();
+#pragma unroll 1
+            for (uint32_t g = w0; g < w1; g += 32) {
+                const uint32_t r = g + lane;
+                int4 ra = make_int4((int)kDone, 0, 0, 0);
+                float2 val = make_float2(0.0f, 0.0f);
+                if (r < w1) {
                     const int2 q = a.xy[r];
                     const uint32_t m = a.meta[r];
                     const float4 v = a.vsum[r];
                     const float2 w = a.wsum[r];
-                    float2 val = make_float2(v.x, v.z);
+                    val = make_float2(v.x, v.z);
                     if (RESIDUAL) val = residual_value(v, w, a.pred[r]);
-                    w_ra[lane] = make_int4(q.x, q.y, (int)((m & 0xffffu) * 7u | ((m >> 16) * 7u) << 16),
-                                           __float_as_int(w.x));
-                    w_rb[lane] = val;
+                    ra = make_int4((q.x & 31) << 5 | (q.y & 31), (int)(m & 0xffffu) * 8,
+                                   (int)(m >> 16) * 8, __float_as_int(w.x));
                 }
+                __syncwarp();   // the slots' last readers are done
+                w_ra[lane] = ra;
+                w_rb[lane] = val;
                 __syncwarp();
-                const int n = (int)min((int64_t)32, e - g);
-                for (int k = 0; k < n; ++k) {
+                const int nb = (int)min(32u, w1 - g);
+#pragma unroll 1
+                for (int k = grp; k - grp < nb; k += 4) {
                     const int4 A = w_ra[k];
                     const float2 B = w_rb[k];
-                    if (!open || A.x != cx || A.y != cy) {
-                        if (open) flush();
-                        open = true;
-                        cx = A.x;
-                        cy = A.y;
-                        pp = ri0 = ri1 = make_float2(0.f, 0.f);
+                    uint32_t cell = (uint32_t)A.x;
+                    const float wx = tap_x[A.y];
+                    float2 y[4];
+                    tap_pairs(s_taps + A.z, y);
+                    // the groups' records belong to the run, or end it
+                    for (;;) {
+                        const bool mine = cell == open;
+                        const unsigned match = __ballot_sync(0xffffffffu, mine);
+                        if (match) {
+                            sums.add(mine, wx, y, __int_as_float(A.w), B);
+                            if (match == 0xffffffffu) break;
+                            if (mine) cell = kDone;
+                        }
+                        const unsigned rest = __ballot_sync(0xffffffffu, cell != kDone);
+                        if (!rest) break;
+                        if (open != kDone - 1) {
+                            flush();
+                            sums.clear();
+                        }
+                        open = __shfl_sync(0xffffffffu, cell, __ffs(rest) - 1);
                     }
-                    const float* wx = s_taps + (A.z & 0xffff);
-                    const float* wy = s_taps + ((unsigned)A.z >> 16);
-                    const float pw = __int_as_float(A.w);
-                    const float2 w = __fmul2_rn(make_float2(wx[ix0], wx[ix1]),
-                                                make_float2(wy[iy0], wy[iy1]));
-                    if (!RESIDUAL) pp = __ffma2_rn(make_float2(pw, pw), w, pp);
-                    ri0 = __ffma2_rn(B, make_float2(w.x, w.x), ri0);
-                    ri1 = __ffma2_rn(B, make_float2(w.y, w.y), ri1);
                 }
-                __syncwarp();   // the slots are refilled by the next batch
             }
-            if (open) flush();
+            if (open != kDone - 1) flush();
             __syncthreads();
             for (int k = tid; k < kFoot * kFoot; k += kStdThreads) {
                 const int fx = k / kFoot, fy = k - fx * kFoot, c = fx * kFootRow + fy;
                 const int64_t cell = (int64_t)(x0 + fx) * a.gny + (y0 + fy);
-                const float2 d = make_float2(s_dr[c], s_di[c]);
+                const float2 d = s_ri[c];
                 // cells past the grid's edge hold zeros
                 if (!RESIDUAL && s_psf[c] != 0.0f) {
                     atomicAdd(&a.psf[cell * a.psf_step], s_psf[c]);
@@ -170,8 +185,7 @@ __global__ void __launch_bounds__(kStdThreads) std_grid_kernel(StdGridArgs a) {
                 }
                 if (d.x != 0.0f || d.y != 0.0f) {
                     atomicAdd(&a.dirty[cell], d);
-                    s_dr[c] = 0.0f;
-                    s_di[c] = 0.0f;
+                    s_ri[c] = make_float2(0.0f, 0.0f);
                 }
             }
             __syncthreads();
@@ -228,8 +242,8 @@ __global__ void __launch_bounds__(256) std_degrid_kernel(StdDegridArgs a) {
 void std_grid(cr_ctx* ctx, cr_gridder* g, const Records& r, float* psf, int psf_step,
               float2* dirty, int mode) {
     StdGridArgs a{r.rec_xy, r.rec_meta, r.rec_vsum, r.rec_wsum, r.rec_pred, r.tile_start,
-                  r.counts, r.ntx * r.nty, r.nty, g->taps_d, g->tap_rows * 7, psf, psf_step, dirty, g->info.grid_nx,
-                  g->info.grid_ny};
+                  r.counts, r.ntx * r.nty, r.nty, g->taps8_d, g->tap_rows * 8, psf, psf_step, dirty,
+                  g->info.grid_nx, g->info.grid_ny};
     const unsigned blocks = (unsigned)(ctx->sms * kStdBlocksPerSm);
     kernel_mark(ctx, 0, false);
     if (mode == 0) {
