@@ -202,18 +202,19 @@ __device__ __forceinline__ int cube_b(int t, int off, int q, const CubeGeom& c) 
 constexpr int kBandRows = 8;
 constexpr int kBands = kTile / kBandRows;   // 4 bands per tile
 constexpr int kBandWarps = 8;               // warps per block
-// Candidate records per work item.  A warp works them off one after the
-// other, so that a small batch is a matter of the longest chain; long chains
-// flush a band less often.  wp_grid at 256 / 128 / 64 / 32: 1000 samples 96 /
-// 71 / 42 / 30 us, 60,000 133 / 78 / 54 / 34, 250,000 160 / 126 / 118 / 131,
-// 1 M 430 / 411 / 442 / 548, 5 M at supports up to 64 5.90 / 5.99 / 6.28 /
-// 6.99 ms.  (A context with an allocation limit keeps the shortest lists.)
-inline uint32_t band_chunk(int64_t samples) {
-    return samples < (1 << 17)   ? 32u
-           : samples < (1 << 19) ? 64u
-           : samples < (1 << 21) ? 128u
-                                 : 256u;
-}
+constexpr int kBandChunk = 256;             // candidate records per work item
+// A warp works an item's records off one after the other, each a matter of the
+// latency of its kernel values; a small batch, which cannot fill the chip, is
+// one such chain.  Below kDeepSamples samples the loads of kDeep records are in
+// flight together, for which a warp takes the registers of three.  (Smaller
+// items are faster still, but every flush more is a rounding at the size of
+// the grid's sums, in any order: 32 candidates gave ten times the difference
+// between two runs of 5,000 samples, the block's warps on one item twice.)
+// wp_grid one / four / eight deep: 1000 samples (256^2) 73 / 42 / 37 us, 16,000
+// (512^2) 107 / 59 / 50, 60,000 (1024^2) 132 / 86 / 79, 250,000 152 / 152 / 137
+// (supports up to 12) and 232 / 250 / 238 (up to 24), 1 M 414 / 524 / 516.
+constexpr int kDeep = 8;
+constexpr int64_t kDeepSamples = 1 << 17;
 constexpr int kNbr = (2 * kMaxSegRadius + 1) * (2 * kMaxSegRadius + 1);
 
 struct __align__(16) BandEntry {
@@ -269,7 +270,6 @@ struct BandArgs {
     const uint32_t* seg_pre;   // [ntiles][kNbr + 1] exclusive prefix of segment lengths
     const uint8_t* nseg;       // [ntiles]
     const uint2* items;        // (tile * kBands + band, first candidate)
-    uint32_t chunk;            // candidates per item
     const unsigned long long* n_items;
     unsigned int* item_counter;
     float2* psf;
@@ -300,8 +300,8 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <bool RESIDUAL>
-__global__ void __launch_bounds__(kBandWarps * 32, 3) wp_grid_kernel(BandArgs a) {
+template <bool RESIDUAL, bool DEEP>
+__global__ void __launch_bounds__(kBandWarps * 32, DEEP ? 1 : 3) wp_grid_kernel(BandArgs a) {
     __shared__ BandEntry s_ent[kBandWarps][32];
     __shared__ __align__(16) int s_rows[kBandWarps][32][kBandRows];
     __shared__ uint32_t s_lo[kBandWarps][kNbr];
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3) wp_grid_kernel(BandArgs a)
         for (int k = lane; k < ns; k += 32) lo_s[k] = a.seg_lo[T * kNbr + k];
         for (int k = lane; k <= ns; k += 32) pre_s[k] = a.seg_pre[T * (kNbr + 1) + k];
         __syncwarp();
-        const uint32_t cbeg = it.y, cend = min(pre_s[ns], cbeg + a.chunk);
+        const uint32_t cbeg = it.y, cend = min(pre_s[ns], cbeg + (uint32_t)kBandChunk);
         // lane l's candidate c (segment k with pre[k] <= c < pre[k+1]) into
         // candidate buffer b
         auto fetch = [&](uint32_t c, int b) {
@@ -401,7 +401,38 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3) wp_grid_kernel(BandArgs a)
             // kernel values are loaded (zero outside the window) before the
             // paired FMAs
             const int nt = __popc(bal);
-            for (int q = 0; q < nt; ++q) {
+            if (DEEP) {
+                for (int q0 = 0; q0 < nt; q0 += kDeep) {
+                    float2 kv[kDeep][kBandRows];
+#pragma unroll
+                    for (int d = 0; d < kDeep; ++d) {
+                        const int q = min(q0 + d, nt - 1);
+                        const BandEntry& E = ent[q];
+                        const int col = E.cb + lane;
+                        const bool colok = (unsigned)col < (unsigned)E.w;
+                        const int bcol = colok ? cube_b(col - E.s, E.oy, E.q, a.cg) : 0;
+                        const float2* kp = a.cube + E.base + bcol;
+#pragma unroll
+                        for (int k = 0; k < kBandRows; ++k) {
+                            const int av = s_rows[warp][q][k];
+                            kv[d][k] = (colok && av >= 0) ? __ldg(kp + av) : make_float2(0.f, 0.f);
+                        }
+                    }
+#pragma unroll
+                    for (int d = 0; d < kDeep; ++d) {
+                        if (q0 + d >= nt) break;
+                        const float4 vx = ent[q0 + d].vx;
+                        const float2 pw = ent[q0 + d].pw;
+#pragma unroll
+                        for (int k = 0; k < kBandRows; ++k) {
+                            X[k] = __ffma2_rn(kv[d][k], make_float2(vx.x, vx.y), X[k]);
+                            Y[k] = __ffma2_rn(kv[d][k], make_float2(vx.z, vx.w), Y[k]);
+                            if (!RESIDUAL) P[k] = __ffma2_rn(kv[d][k], pw, P[k]);
+                        }
+                    }
+                }
+            }
+            for (int q = DEEP ? nt : 0; q < nt; ++q) {
                 const BandEntry& E = ent[q];
                 const int col = E.cb + lane;
                 const bool colok = (unsigned)col < (unsigned)E.w;
@@ -477,7 +508,7 @@ __global__ void band_work_count(const uint32_t* tile_start, const uint32_t* rmet
                                 const int32_t* first_plane, int32_t max_support, int monotone,
                                 int64_t ntx, int64_t nty, int R, int64_t gnx,
                                 uint32_t* seg_lo, uint32_t* seg_pre, uint8_t* nseg,
-                                uint32_t chunk, uint32_t* nitems) {
+                                uint32_t* nitems) {
     const int64_t ntiles = ntx * nty;
     const int lane = threadIdx.x & 31, D = 2 * R + 1;
     for (int64_t T = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; T < ntiles;
@@ -531,13 +562,13 @@ __global__ void band_work_count(const uint32_t* tile_start, const uint32_t* rmet
             const int64_t rows_left = gnx - tx * kTile;
             const int64_t nb = (rows_left + kBandRows - 1) / kBandRows;
             const int bands = (int)(nb < kBands ? nb : kBands);
-            nitems[T] = total ? (uint32_t)bands * ((total + chunk - 1) / chunk) : 0u;
+            nitems[T] = total ? (uint32_t)bands * ((total + kBandChunk - 1) / kBandChunk) : 0u;
         }
     }
 }
 
 __global__ void band_work_fill(const uint32_t* nitems, const uint32_t* first, int64_t ntx,
-                               int64_t nty, int64_t gnx, uint32_t chunk, uint2* items) {
+                               int64_t nty, int64_t gnx, uint2* items) {
     const int64_t ntiles = ntx * nty;
     const int lane = threadIdx.x & 31;
     for (int64_t T = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; T < ntiles;
@@ -549,7 +580,7 @@ __global__ void band_work_fill(const uint32_t* nitems, const uint32_t* first, in
         const uint32_t bands = (uint32_t)(nb < kBands ? nb : kBands), f = first[T];
         // chunk-major, band-minor: the bands of one chunk are consecutive items
         for (uint32_t k = lane; k < n; k += 32)
-            items[f + k] = make_uint2((uint32_t)T * kBands + k % bands, k / bands * chunk);
+            items[f + k] = make_uint2((uint32_t)T * kBands + k % bands, k / bands * kBandChunk);
     }
 }
 
@@ -960,7 +991,6 @@ static void wproj_grid_band(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2*
     const int R = (31 + wp->info.max_support) / kTile;
     if (R > kMaxSegRadius) fail(CR_INVALID, "W-projection support above 127 is not supported");
     const int64_t gnx = wp->g->info.grid_nx;
-    const uint32_t chunk = ctx->alloc_limit > 0 ? 256u : band_chunk(r.n_samples);
     uint32_t* seg_lo = (uint32_t*)workspace(ctx, "wb_seg_lo", (size_t)ntiles * kNbr * 4);
     uint32_t* seg_pre = (uint32_t*)workspace(ctx, "wb_seg_pre", (size_t)ntiles * (kNbr + 1) * 4);
     uint8_t* nseg = (uint8_t*)workspace(ctx, "wb_nseg", (size_t)ntiles);
@@ -969,17 +999,17 @@ static void wproj_grid_band(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2*
     unsigned long long* total = (unsigned long long*)workspace(ctx, "wb_total", 16);
     band_work_count<<<grid_blocks(ntiles * 32, 256), 256, 0, ctx->stream>>>(
         r.tile_start, r.rec_meta, wp->first_plane_d, wp->info.max_support,
-        wp->support_monotone ? 1 : 0, r.ntx, r.nty, R, gnx, seg_lo, seg_pre, nseg, chunk, nitems);
+        wp->support_monotone ? 1 : 0, r.ntx, r.nty, R, gnx, seg_lo, seg_pre, nseg, nitems);
     note_launch(ctx, "band_work_count");
     exclusive_scan_u32(ctx, nitems, first, ntiles, total);
     // every record is a candidate of at most (2R+1)^2 tiles; each tile has
     // at most kBands items per started chunk
     const size_t max_items = (size_t)kBands * ((size_t)ntiles +
                              (size_t)((2 * R + 1) * (2 * R + 1)) *
-                                 (size_t)(r.n_samples / chunk + 1));
+                                 (size_t)(r.n_samples / kBandChunk + 1));
     uint2* items = (uint2*)workspace(ctx, "wb_items", max_items * 8);
     band_work_fill<<<grid_blocks(ntiles * 32, 256), 256, 0, ctx->stream>>>(nitems, first, r.ntx,
-                                                                       r.nty, gnx, chunk, items);
+                                                                       r.nty, gnx, items);
     note_launch(ctx, "band_work_fill");
     unsigned int* counter = (unsigned int*)(total + 1);
     CR_CUDA_CHECK(cudaMemsetAsync(counter, 0, 4, ctx->stream));
@@ -996,9 +1026,11 @@ static void wproj_grid_band(cr_ctx* ctx, cr_wproj* wp, const Records& r, float2*
             wp->support_d, wp->axis, r.counts, packed, weight);
     note_launch(ctx, "band_pack_kernel");
     BandArgs a{packed, weight, wp->cube_off_d, wp->cube_q_d, wp->cube_d, cube_geom(wp),
-               wp->radius, r.nty, seg_lo, seg_pre, nseg, items, chunk, total, counter, psf, dirty, gnx,
+               wp->radius, r.nty, seg_lo, seg_pre, nseg, items, total, counter, psf, dirty, gnx,
                wp->g->info.grid_ny};
-    auto kern = mode == 0 ? wp_grid_kernel<false> : wp_grid_kernel<true>;
+    const bool deep = r.n_samples < kDeepSamples;
+    auto kern = deep ? (mode == 0 ? wp_grid_kernel<false, true> : wp_grid_kernel<true, true>)
+                     : (mode == 0 ? wp_grid_kernel<false, false> : wp_grid_kernel<true, false>);
     // shared memory for three blocks, the rest to L1: the kernel is bound by
     // what it reads of the kernel cubes through L2 (8 TB/s; with the largest
     // carve-out 6.02 ms against 5.90 at supports up to 64)
