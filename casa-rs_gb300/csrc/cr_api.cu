@@ -1385,6 +1385,7 @@ int cr_cube_plan_create(cr_ctx* ctx, cr_gridder* g, const cr_cube_batch* batch,
             tm.mark();
             p->sums.resize((size_t)in.C);
             cube_read_sums(ctx, p->rec, p->sums.data());
+            check_device_status(ctx);
         } catch (...) {
             cr_cube_plan_destroy(p);
             throw;
