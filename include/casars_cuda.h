@@ -179,8 +179,8 @@ int64_t cr_ctx_workspace_bytes(cr_ctx* ctx);
 /* Bounds of the device-side waits, for tests of the timeout paths.  The
  * reference has no device waits; its counterpart is the error taxonomy of
  * ImagingError (crates/casa-imaging/src/error.rs:7-24).  barrier_polls bounds
- * each wait of the Hogbom grid barrier (polls ~64 ns apart; default 2^24,
- * about a second), mbar_polls the first wait on each bulk copy of the cube
+ * each wait of the Hogbom blocks for one another (default 2^24 polls, about
+ * a second), mbar_polls the first wait on each bulk copy of the cube
  * kernels (default 2^22 polls).  0 gives up at once: a call whose wait gives
  * up returns CR_TIMEOUT and leaves its outputs undefined; the context stays
  * usable.  A negative value restores the default.  Waits that let a block's
@@ -298,7 +298,7 @@ int cr_plan_residual_image(cr_ctx* ctx, cr_plan* plan, const float* model,
  * Centred inverse FFT (fft.rs:600-630) of a grid then crop x correction:
  * corrected_image_from_grid_f64 (gridder.rs:1646-1657), or the W-projection
  * correction (gridder.rs:1685-1715) when wp is given; the result is scaled
- * by `scale` (float32 multiply).  cuFFT performs the bare transform only. */
+ * by `scale` (float32 multiply). */
 int cr_grid_to_image(cr_ctx* ctx, cr_gridder* g, cr_wproj* wp, const float* grid,
                      int32_t grid_location, float scale, float* image, int32_t out_location,
                      char** err);
@@ -424,9 +424,8 @@ int cr_cube_plan_create(cr_ctx* ctx, cr_gridder* g, const cr_cube_batch* batch,
                         char** err);
 void cr_cube_plan_destroy(cr_cube_plan* plan);
 int32_t cr_cube_plan_channels(const cr_cube_plan* plan);
-/* Transforms of the image calls: 32 = float32 C2C (the default; FP64 runs
- * at a small fraction of the float32 rate on this GPU), 64 = FP64 Z2Z as in
- * the single-plane calls.  Returns CR_INVALID for other values. */
+/* Transforms of the image calls: 32 = float32 (the default), 64 = FP64-grade
+ * as in the single-plane calls.  Returns CR_INVALID for other values. */
 int cr_cube_plan_set_fft_precision(cr_cube_plan* plan, int32_t bits);
 int cr_cube_plan_grid_dirty(cr_ctx* ctx, cr_cube_plan* plan, float* psf_grids,
                             float* dirty_grids, int32_t out_location, char** err);
