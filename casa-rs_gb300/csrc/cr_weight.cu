@@ -134,7 +134,7 @@ density_kernel(const double* u, const double* v, const float* weight, int64_t n,
                     continue;
                 }
             }
-            if (ok) atomicAdd(&density[cell], w[j]);
+            if (ok) atomicAdd(&density[(int64_t)x * p.ny + y], w[j]);
             if (okm) atomicAdd(&density[(int64_t)xm * p.ny + ym], w[j]);
         }
     }
@@ -236,7 +236,8 @@ void apply_weighting(cr_ctx* ctx, cr_gridder* g, const DeviceBatch& b, int32_t m
         if (b.n > 0) {
             // the density is built at build_u, build_v when given (the row
             // path's VisImagingWeight coordinates), looked up at u, v
-            const bool table = b.n >= kTableSamples;
+            // (the table's keys are 32-bit cells)
+            const bool table = b.n >= kTableSamples && (int64_t)nx * ny < kEmptySlot;
             auto kern = table ? density_kernel<true> : density_kernel<false>;
             const size_t smem = table ? (size_t)kSlots * 8 : 0;
             CR_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
