@@ -6,8 +6,8 @@ values in flight.  The same samples followed by samples of zero weight, up to
 the rounding of float32 sums in another order (1e-5 of the peak, the bound of
 the other W-projection tests) and the counts are equal.  The sizes leave one,
 eight, nine and many records in a warp's batch; the largest is the last below
-the change.  (The residual form is held to the oracle by the adjoint and
-residual tests of test_gpu_wproj.py, test_gpu_dfft.py and test_gpu_autograd.py.)
+the change.  (test_residual_refresh_matches_oracle of test_gpu_wproj.py holds
+the residual form to the oracle.)
 """
 import numpy as np
 import pytest
